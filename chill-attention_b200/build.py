@@ -2,8 +2,8 @@
 
     python chill-attention_b200/build.py            # -> chill_attention/_lib/libchill_b200.so
 
-Each mask functor's tensor-core kernels are a translation unit of their own
-(csrc/tc_inst.cu with -DCHILL_INST_MASK=<functor>), compiled in parallel.
+Each mask functor's tensor-core kernels and its CUDA-core kernels are translation units of their own
+(csrc/tc_inst.cu, csrc/simt_inst.cu with -DCHILL_INST_MASK=<functor>), compiled in parallel.
 ``build_library`` is also what ``chill_attention.custom`` calls to produce a private
 library for a user-defined mask functor.
 """
@@ -44,7 +44,7 @@ def _sources_digest(extra=()):
     for name in names:
         path = name if os.path.isabs(name) else os.path.join(CSRC, name)
         if os.path.isfile(path):
-            h.update(name.encode())
+            h.update(os.path.basename(name).encode())  # not the full path: a built tree may be moved
             with open(path, "rb") as f:
                 h.update(f.read())
     for e in extra:
@@ -82,8 +82,9 @@ def build_library(out_path=None, custom_header=None, custom_functor=None, verbos
     jobs = [([nvcc] + NVCC_FLAGS + defines + ["-c", os.path.join(CSRC, src + ".cu"), "-o",
                                                os.path.join(obj_dir, src + ".o")]) for src in ("chill_abi", "host_pipeline")]
     for fn in functors:
-        jobs.append([nvcc] + NVCC_FLAGS + defines + [f"-DCHILL_INST_MASK={fn}", "-c", os.path.join(CSRC, "tc_inst.cu"),
-                                                      "-o", os.path.join(obj_dir, f"tc_{fn}.o")])
+        for unit in ("tc", "simt"):
+            jobs.append([nvcc] + NVCC_FLAGS + defines + [f"-DCHILL_INST_MASK={fn}", "-c", os.path.join(CSRC, f"{unit}_inst.cu"),
+                                                          "-o", os.path.join(obj_dir, f"{unit}_{fn}.o")])
     if verbose:
         jobs = [j[:1] + ["-Xptxas", "-v"] + j[1:] for j in jobs]
     with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:

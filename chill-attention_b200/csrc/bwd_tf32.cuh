@@ -18,7 +18,7 @@
 //     then decides the size TO of the streamed tiles: 128 positions at head dim 64 (64 KB resident + 128 KB
 //     streamed), 32 at head dim 128 (128 KB resident + 64 KB streamed).
 // The kernels are deliberately plain: one ring stage, the tensor cores and the compute warps alternate.  They run
-// at a few hundred TFLOP/s where the IEEE kernels (generic.cuh) that otherwise serve fp32 reach about one.
+// at a few hundred TFLOP/s where the IEEE kernels (simt.cuh) that otherwise serve fp32 reach about thirty.
 // Inputs are used as they are (the tensor core drops all but 10 mantissa bits); gradients match the fp64 oracle
 // to about 1e-3 relative on N(0,1) inputs (the tests state 5e-3).
 #pragma once

@@ -12,6 +12,7 @@
 #include "chill_b200.h"
 #include "fwd_tc.cuh"
 #include "generic.cuh"
+#include "simt.cuh"
 #include "tc_launch.h"
 
 namespace chill {
@@ -213,19 +214,28 @@ static int check_fwd(const chill_fwd_args* a) {
   return CHILL_OK;
 }
 
+// Rows of this tensor can be moved in 16-byte vectors (fp32 only; see simt.cuh).
+static uint32_t vec_bit(uint32_t bit, const void* p, const int64_t* st, int dtype, int D) {
+  if (dtype != CHILL_F32 || st[3] != 1 || D % 4 != 0 || ((uintptr_t)p) % 16 != 0) return 0;
+  return (st[0] % 4 == 0 && st[1] % 4 == 0 && st[2] % 4 == 0) ? bit : 0;
+}
+
 static int fwd_generic(const chill_fwd_args& a, cudaStream_t st) {
-  FwdP p;
+  simt::FwdParams pp;
+  FwdP& p = pp.f;
   p.g = to_geo(a.s);
   p.q = to_ref(a.q, a.q_strides); p.k = to_ref(a.k, a.k_strides);
   p.v = to_ref(a.v, a.v_strides); p.o = to_ref(a.o, a.o_strides);
   p.lse = a.lse;
   p.lse_sb = a.lse_strides[0]; p.lse_sh = a.lse_strides[1]; p.lse_sl = a.lse_strides[2];
-  dim3 grid((a.s.Lq + kGenericWarps - 1) / kGenericWarps, a.s.H, a.s.B);
-  CHILL_MASK_SWITCH(a.s.mask.id,
-                    CHILL_DTYPE_SWITCH(a.s.dtype, (fwd_generic_kernel<ElemT, MaskT><<<grid, kGenericWarps * 32, 0, st>>>(p))))
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) g_launches += 1;
-  return e == cudaSuccess ? CHILL_OK : cuda_fail(e, "fwd_generic launch");
+  const int dt = a.s.dtype, D = a.s.D;
+  pp.dtype = dt;
+  pp.vec = vec_bit(simt::kVecQ, a.q, a.q_strides, dt, D) | vec_bit(simt::kVecK, a.k, a.k_strides, dt, D) |
+           vec_bit(simt::kVecV, a.v, a.v_strides, dt, D) | vec_bit(simt::kVecO, a.o, a.o_strides, dt, D);
+  int e = 0;
+  CHILL_MASK_SWITCH(a.s.mask.id, (e = simt_launch_fwd<MaskT>(pp, st)))
+  if (e == 0) g_launches += 1;
+  return e == 0 ? CHILL_OK : cuda_fail((cudaError_t)e, "fwd_generic launch");
 }
 
 static int fwd_tc(const chill_fwd_args& a, cudaStream_t st) {
@@ -376,18 +386,18 @@ static int bwd_which(uint32_t flags) {
 }
 
 static int bwd_generic(const chill_bwd_args& a, cudaStream_t st) {
-  BwdP p = to_bwdp(a);
-  const chill_shape& s = a.s;
-  const int which = bwd_which(s.flags);
-  dim3 gq((s.Lq + kGenericWarps - 1) / kGenericWarps, s.H, s.B);
-  dim3 gk((s.Lk + kGenericWarps - 1) / kGenericWarps, s.H_kv, s.B);
-  CHILL_MASK_SWITCH(s.mask.id, CHILL_DTYPE_SWITCH(s.dtype, {
-                      if (which & 2) (bwd_dq_generic_kernel<ElemT, MaskT><<<gq, kGenericWarps * 32, 0, st>>>(p));
-                      if (which & 1) (bwd_dkdv_generic_kernel<ElemT, MaskT><<<gk, kGenericWarps * 32, 0, st>>>(p));
-                    }))
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) g_launches += (which == 3 ? 2 : 1);
-  return e == cudaSuccess ? CHILL_OK : cuda_fail(e, "bwd_generic launch");
+  simt::BwdParams pp;
+  pp.b = to_bwdp(a);
+  const int dt = a.s.dtype, D = a.s.D;
+  pp.dtype = dt;
+  pp.vec = vec_bit(simt::kVecQ, a.q, a.q_strides, dt, D) | vec_bit(simt::kVecK, a.k, a.k_strides, dt, D) |
+           vec_bit(simt::kVecV, a.v, a.v_strides, dt, D) | vec_bit(simt::kVecDo, a.d_o, a.do_strides, dt, D) |
+           vec_bit(simt::kVecDq, a.dq, a.dq_strides, dt, D) | vec_bit(simt::kVecDk, a.dk, a.dk_strides, dt, D) |
+           vec_bit(simt::kVecDv, a.dv, a.dv_strides, dt, D);
+  int e = 0;
+  CHILL_MASK_SWITCH(a.s.mask.id, (e = simt_launch_bwd<MaskT>(pp, bwd_which(a.s.flags), st)))
+  if (e == 0) g_launches += 1;
+  return e == 0 ? CHILL_OK : cuda_fail((cudaError_t)e, "bwd_generic launch");
 }
 
 // Side stream + fork/join events per device, created on first use: the dK/dV and the dQ kernel are

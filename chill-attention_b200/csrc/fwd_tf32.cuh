@@ -12,7 +12,7 @@
 //   * O is stored as fp32.
 // Q, K and V are used as they are: the tensor core drops all but 10 mantissa bits (truncation); P is rounded to
 // nearest by the softmax warps.  Against the fp64 oracle the output error on N(0,1) inputs is 2e-3 .. 4e-3 (the
-// tests state 5e-3), three orders above the generic IEEE kernels that serve precision="ieee".
+// tests state 5e-3), well above the IEEE kernels (simt.cuh) that serve precision="ieee".
 // Reference: chill_attention/chill_fwd.py:13-359 with input_precision="tf32".
 #pragma once
 #include <type_traits>

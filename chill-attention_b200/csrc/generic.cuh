@@ -1,14 +1,5 @@
-// Generic (CUDA-core, fp32 arithmetic) kernels: any dtype, any head dim <= 256, any strides.
-//
-// They serve every call the tensor-core kernels cannot take (fp32 inputs with IEEE
-// precision, head dims other than 64/128, channel stride != 1, misaligned strides) so the
-// operator has no host fallback.  One warp owns one output row; the other axis is walked in
-// chunks of 32 positions, one per lane, clipped by the mask functor's range function.
-//
-//   fwd_generic_kernel     O, LSE          (reference math: chill_attention/chill_fwd.py:188-359)
-//   delta_kernel           delta           (chill_attention/utils.py:93-217)
-//   bwd_dq_generic_kernel  dQ              (chill_attention/chill_bwd_dq.py:15-229)
-//   bwd_dkdv_generic_kernel dK, dV         (chill_attention/chill_bwd_dkdv.py:15-277)
+// What every kernel shares: tensor references, call geometry, scalar conversions; and the kernels that are not attention
+// itself: delta (chill_attention/utils.py:93-217) and the tabulation of a mask functor.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -84,16 +75,6 @@ template <typename T>
 __device__ __forceinline__ const T* row_ptr(const TRef& t, int b, int h, int l) {
   return reinterpret_cast<const T*>(t.p) + b * t.sb + h * t.sh + l * t.sl;
 }
-template <typename T>
-__device__ __forceinline__ T* row_ptr_w(const TRef& t, int b, int h, int l) {
-  return reinterpret_cast<T*>(t.p) + b * t.sb + h * t.sh + l * t.sl;
-}
-
-__device__ __forceinline__ float warp_max(float x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
-  return x;
-}
 __device__ __forceinline__ float warp_sum(float x) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -104,83 +85,6 @@ __device__ __forceinline__ int valid_len(const Geo& g, int b) {
   int n = g.seq_len;
   if (g.lens != nullptr) n = imin(n, g.lens[b]);
   return n;
-}
-
-template <typename T>
-__device__ __forceinline__ float dot_row(const float* s, const T* x, long long sd, int D) {
-  float acc = 0.f;
-  for (int d = 0; d < D; ++d) acc = fmaf(s[d], to_f(x[d * sd]), acc);
-  return acc;
-}
-
-// ------------------------------------------------------------------------------- forward
-template <typename T, class M>
-__global__ void __launch_bounds__(kGenericWarps * 32) fwd_generic_kernel(FwdP p) {
-  __shared__ float qs[kGenericWarps][kMaxD];
-  const Geo& g = p.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * kGenericWarps + warp;
-  const int h = blockIdx.y, b = blockIdx.z;
-  if (row >= g.Lq) return;
-  const int hk = h / (g.H / g.Hkv);
-  const int n = valid_len(g, b);
-  const int qg = row + g.q_off;
-  const int D = g.D;
-  T* orow = row_ptr_w<T>(p.o, b, h, row);
-  if (qg >= n) {  // padded query row
-    for (int d = lane; d < D; d += 32) orow[d * p.o.sd] = from_f<T>(0.f);
-    if (p.lse != nullptr && lane == 0) p.lse[b * p.lse_sb + h * p.lse_sh + row * p.lse_sl] = 0.f;
-    return;
-  }
-  const T* qrow = row_ptr<T>(p.q, b, h, row);
-  for (int d = lane; d < D; d += 32) qs[warp][d] = to_f(qrow[d * p.q.sd]);
-  __syncwarp();
-
-  int lo, hi;
-  M::k_range_for_q(qg, n, g.margs, lo, hi);
-  const int jlo = imax(lo - g.k_off, 0);
-  const int jhi = imin(imin(hi, n - 1) - g.k_off, g.Lk - 1);
-  const float c = g.scale * kLog2e;
-
-  float m = -CUDART_INF_F, l = 0.f;
-  float acc[kMaxD / 32];
-#pragma unroll
-  for (int t = 0; t < kMaxD / 32; ++t) acc[t] = 0.f;
-
-  for (int j0 = jlo; j0 <= jhi; j0 += 32) {
-    const int j = j0 + lane;
-    const bool ok = (j <= jhi) && M::mask(qg, j + g.k_off, n, g.margs);
-    float s = -CUDART_INF_F;
-    if (ok) s = dot_row<T>(qs[warp], row_ptr<T>(p.k, b, hk, j), p.k.sd, D) * c;
-    const float m_new = fmaxf(m, warp_max(s));
-    const float m_safe = (m_new == -CUDART_INF_F) ? 0.f : m_new;
-    const float alpha = exp2f(m - m_safe);
-    const float pj = ok ? exp2f(s - m_safe) : 0.f;
-    l = l * alpha + warp_sum(pj);
-#pragma unroll
-    for (int t = 0; t < kMaxD / 32; ++t) acc[t] *= alpha;
-    const int cnt = imin(32, jhi - j0 + 1);
-    for (int jj = 0; jj < cnt; ++jj) {
-      const float pb = __shfl_sync(0xffffffffu, pj, jj);
-      if (pb != 0.f) {
-        const T* vrow = row_ptr<T>(p.v, b, hk, j0 + jj);
-#pragma unroll
-        for (int t = 0; t < kMaxD / 32; ++t) {
-          const int d = lane + 32 * t;
-          if (d < D) acc[t] = fmaf(pb, to_f(vrow[d * p.v.sd]), acc[t]);
-        }
-      }
-    }
-    m = m_new;
-  }
-  const float l_safe = (l == 0.f) ? 1.f : l;
-  const float inv = 1.f / l_safe;
-#pragma unroll
-  for (int t = 0; t < kMaxD / 32; ++t) {
-    const int d = lane + 32 * t;
-    if (d < D) orow[d * p.o.sd] = from_f<T>(acc[t] * inv);
-  }
-  if (p.lse != nullptr && lane == 0) p.lse[b * p.lse_sb + h * p.lse_sh + row * p.lse_sl] = m + log2f(l_safe);
 }
 
 // --------------------------------------------------------------------------------- delta
@@ -229,163 +133,6 @@ __global__ void __launch_bounds__(256) delta_rows16_kernel(const T* __restrict__
   if (row < Lq && li == 0) {
     if (dlse != nullptr) acc -= kLog2e * dlse[b * dl_sb + h * dl_sh + row * dl_sl];  // gradient through the returned LSE
     delta[((long long)b * H + h) * Lq + row] = acc;
-  }
-}
-
-// ------------------------------------------------------------------------------ backward
-template <typename T, class M>
-__global__ void __launch_bounds__(kGenericWarps * 32) bwd_dq_generic_kernel(BwdP p) {
-  __shared__ float qs[kGenericWarps][kMaxD];
-  __shared__ float ds_[kGenericWarps][kMaxD];
-  const Geo& g = p.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row = blockIdx.x * kGenericWarps + warp;
-  const int h = blockIdx.y, b = blockIdx.z;
-  if (row >= g.Lq) return;
-  const int hk = h / (g.H / g.Hkv);
-  const int n = valid_len(g, b);
-  const int qg = row + g.q_off;
-  const int D = g.D;
-  T* dqrow = row_ptr_w<T>(p.dq, b, h, row);
-  if (qg >= n) {
-    for (int d = lane; d < D; d += 32) dqrow[d * p.dq.sd] = from_f<T>(0.f);
-    return;
-  }
-  const T* qrow = row_ptr<T>(p.q, b, h, row);
-  const T* dorow = row_ptr<T>(p.d_o, b, h, row);
-  for (int d = lane; d < D; d += 32) {
-    qs[warp][d] = to_f(qrow[d * p.q.sd]);
-    ds_[warp][d] = to_f(dorow[d * p.d_o.sd]);
-  }
-  __syncwarp();
-  float lse = p.lse[b * p.lse_sb + h * p.lse_sh + row * p.lse_sl];
-  if (lse == -CUDART_INF_F) lse = 0.f;
-  const float delta = p.delta[((long long)b * g.H + h) * g.Lq + row];
-
-  int lo, hi;
-  M::k_range_for_q(qg, n, g.margs, lo, hi);
-  const int jlo = imax(lo - g.k_off, 0);
-  const int jhi = imin(imin(hi, n - 1) - g.k_off, g.Lk - 1);
-  const float c = g.scale * kLog2e;
-  float acc[kMaxD / 32];
-#pragma unroll
-  for (int t = 0; t < kMaxD / 32; ++t) acc[t] = 0.f;
-
-  for (int j0 = jlo; j0 <= jhi; j0 += 32) {
-    const int j = j0 + lane;
-    const bool ok = (j <= jhi) && M::mask(qg, j + g.k_off, n, g.margs);
-    float ds = 0.f;
-    if (ok) {
-      const float s = dot_row<T>(qs[warp], row_ptr<T>(p.k, b, hk, j), p.k.sd, D) * c;
-      const float pj = exp2f(s - lse);
-      const float dp = dot_row<T>(ds_[warp], row_ptr<T>(p.v, b, hk, j), p.v.sd, D);
-      ds = pj * (dp - delta);
-    }
-    const int cnt = imin(32, jhi - j0 + 1);
-    for (int jj = 0; jj < cnt; ++jj) {
-      const float dsb = __shfl_sync(0xffffffffu, ds, jj);
-      if (dsb != 0.f) {
-        const T* krow = row_ptr<T>(p.k, b, hk, j0 + jj);
-#pragma unroll
-        for (int t = 0; t < kMaxD / 32; ++t) {
-          const int d = lane + 32 * t;
-          if (d < D) acc[t] = fmaf(dsb, to_f(krow[d * p.k.sd]), acc[t]);
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < kMaxD / 32; ++t) {
-    const int d = lane + 32 * t;
-    if (d < D) dqrow[d * p.dq.sd] = from_f<T>(acc[t] * g.scale);
-  }
-}
-
-template <typename T, class M>
-__global__ void __launch_bounds__(kGenericWarps * 32) bwd_dkdv_generic_kernel(BwdP p) {
-  __shared__ float ks[kGenericWarps][kMaxD];
-  __shared__ float vs[kGenericWarps][kMaxD];
-  const Geo& g = p.g;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x * kGenericWarps + warp;
-  const int hk = blockIdx.y, b = blockIdx.z;
-  if (j >= g.Lk) return;
-  const int G = g.H / g.Hkv;
-  const int n = valid_len(g, b);
-  const int kg = j + g.k_off;
-  const int D = g.D;
-  T* dkrow = row_ptr_w<T>(p.dk, b, hk, j);
-  T* dvrow = row_ptr_w<T>(p.dv, b, hk, j);
-  float* dkpart = p.part.row(p.part.dk, b, hk, j, g.Lk);
-  float* dvpart = p.part.row(p.part.dv, b, hk, j, g.Lk);
-  if (kg >= n) {
-    for (int d = lane; d < D; d += 32) {
-      dkrow[d * p.dk.sd] = from_f<T>(0.f);
-      dvrow[d * p.dv.sd] = from_f<T>(0.f);
-      if (dkpart != nullptr) dkpart[d] = dvpart[d] = 0.f;
-    }
-    return;
-  }
-  const T* krow = row_ptr<T>(p.k, b, hk, j);
-  const T* vrow = row_ptr<T>(p.v, b, hk, j);
-  for (int d = lane; d < D; d += 32) {
-    ks[warp][d] = to_f(krow[d * p.k.sd]);
-    vs[warp][d] = to_f(vrow[d * p.v.sd]);
-  }
-  __syncwarp();
-  int lo, hi;
-  M::q_range_for_k(kg, n, g.margs, lo, hi);
-  const int ilo = imax(lo - g.q_off, 0);
-  const int ihi = imin(imin(hi, n - 1) - g.q_off, g.Lq - 1);
-  const float c = g.scale * kLog2e;
-  float acck[kMaxD / 32], accv[kMaxD / 32];
-#pragma unroll
-  for (int t = 0; t < kMaxD / 32; ++t) acck[t] = accv[t] = 0.f;
-
-  for (int gi = 0; gi < G; ++gi) {
-    const int h = hk * G + gi;
-    for (int i0 = ilo; i0 <= ihi; i0 += 32) {
-      const int i = i0 + lane;
-      const bool ok = (i <= ihi) && M::mask(i + g.q_off, kg, n, g.margs);
-      float pi = 0.f, ds = 0.f;
-      if (ok) {
-        float lse = p.lse[b * p.lse_sb + h * p.lse_sh + i * p.lse_sl];
-        if (lse == -CUDART_INF_F) lse = 0.f;
-        const float s = dot_row<T>(ks[warp], row_ptr<T>(p.q, b, h, i), p.q.sd, D) * c;
-        pi = exp2f(s - lse);
-        const float dp = dot_row<T>(vs[warp], row_ptr<T>(p.d_o, b, h, i), p.d_o.sd, D);
-        ds = pi * (dp - p.delta[((long long)b * g.H + h) * g.Lq + i]);
-      }
-      const int cnt = imin(32, ihi - i0 + 1);
-      for (int ii = 0; ii < cnt; ++ii) {
-        const float pb = __shfl_sync(0xffffffffu, pi, ii);
-        const float dsb = __shfl_sync(0xffffffffu, ds, ii);
-        if (pb != 0.f || dsb != 0.f) {
-          const T* qrow = row_ptr<T>(p.q, b, h, i0 + ii);
-          const T* dorow = row_ptr<T>(p.d_o, b, h, i0 + ii);
-#pragma unroll
-          for (int t = 0; t < kMaxD / 32; ++t) {
-            const int d = lane + 32 * t;
-            if (d < D) {
-              accv[t] = fmaf(pb, to_f(dorow[d * p.d_o.sd]), accv[t]);
-              acck[t] = fmaf(dsb, to_f(qrow[d * p.q.sd]), acck[t]);
-            }
-          }
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int t = 0; t < kMaxD / 32; ++t) {
-    const int d = lane + 32 * t;
-    if (d < D) {
-      dkrow[d * p.dk.sd] = from_f<T>(acck[t] * g.scale);
-      dvrow[d * p.dv.sd] = from_f<T>(accv[t]);
-      if (dkpart != nullptr) {
-        dkpart[d] = acck[t] * g.scale;
-        dvpart[d] = accv[t];
-      }
-    }
   }
 }
 

@@ -14,6 +14,10 @@ namespace tc {
 struct FwdTcParams;
 struct BwdTcParams;
 }  // namespace tc
+namespace simt {
+struct FwdParams;
+struct BwdParams;
+}  // namespace simt
 
 // Raises a kernel's dynamic shared-memory limit the first time the kernel is launched on a device.  The attribute
 // is per (kernel, device); the record of where it has been set is per call site (pass a distinct `Tag` per kernel)
@@ -39,6 +43,19 @@ static cudaError_t ensure_dynamic_smem(Kern kern, int smem_bytes, bool prefer_ma
   done[dev] = true;
   return cudaSuccess;
 }
+
+// SMs of the current device.
+static inline int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  return n;
+}
+
+// CUDA-core kernels (simt.cuh).  `which`: bit 0 dK / dV, bit 1 dQ.
+template <class M>
+int simt_launch_fwd(const simt::FwdParams& p, cudaStream_t st);
+template <class M>
+int simt_launch_bwd(const simt::BwdParams& p, int which, cudaStream_t st);
 
 // maps: Q, K, V, O.  Returns a cudaError_t cast to int.
 template <class M>
