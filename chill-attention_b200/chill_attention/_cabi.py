@@ -34,6 +34,7 @@ _DTYPES = {torch.float32: CHILL_F32, torch.float16: CHILL_F16, torch.bfloat16: C
 
 ABI_VERSION = 5
 FLAG_BWD_DETERMINISTIC = 32
+FLAG_NARROW_HEAD = 64
 SELFTEST_STATUS = 901
 
 EXPORTS = (

@@ -47,24 +47,22 @@ def _backward_operand(do: torch.Tensor) -> torch.Tensor:
     return do if _cabi.tma_compatible(do) else do.contiguous()
 
 
-#: 16-bit head dims that chill_attention() zero-pads to _PADDED_TO channels (tensor-core kernels instead of generic)
-_PADDED_HEAD_DIMS = (16, 32)
-_PADDED_TO = 64
-
-
 def _tensor_core_operands(q, k, v):
     """16-bit q, k, v with a head dimension the tensor-core kernels serve, but in a memory layout TMA cannot describe
     (channel stride != 1, a broadcast dimension, rows not 16-byte aligned): one packing copy each puts them on the
     tensor-core path, ~1000x faster than the generic kernels that would otherwise take the call.  The reference reads
     such tensors through block pointers at full speed (chill_fwd.py:74-98); results are identical either way."""
-    if q.dtype == torch.float32 or q.shape[-1] not in (64, 128, 256):
+    if q.dtype == torch.float32:
         return q, k, v
     return tuple(t if _cabi.tma_compatible(t) else t.contiguous() for t in (q, k, v))
 
 
-def _precision_flags(precision, dtype) -> int:
-    """precision="tf32" (the reference's tl.dot input_precision) lets fp32 tensors use the TF32 tensor cores."""
-    return _cabi.FLAG_ALLOW_TF32 if (precision == "tf32" and dtype == torch.float32) else 0
+def _call_flags(precision, dtype) -> int:
+    """precision="tf32" (the reference's tl.dot input_precision) lets fp32 tensors use the TF32 tensor cores; 16-bit
+    tensors use the tensor cores for narrow heads (16 / 32 channels) too."""
+    if dtype == torch.float32:
+        return _cabi.FLAG_ALLOW_TF32 if precision == "tf32" else 0
+    return _cabi.FLAG_NARROW_HEAD
 
 
 def _run_backward(lib, functor_id, q, k, v, lens, o, lse, do, mask_args, sm_scale, d_lse=None, flags=0):
@@ -150,7 +148,7 @@ def register_chill_mask(mask: ChillMask):
             O = torch.empty_like(q, memory_format=torch.contiguous_format)
             LSE = torch.empty(q.shape[:3], dtype=torch.float32, device=q.device) if return_lse else None
             lens_c = lens.contiguous() if lens is not None else None
-            flags = _precision_flags(precision, q.dtype)
+            flags = _call_flags(precision, q.dtype)
             shape = _cabi.make_shape(q, k, functor_id, mask_args, lens_c, sm_scale, flags=flags)
             _cabi.forward(lib, q, k, v, O, LSE, shape)
         if LSE is None:
@@ -181,7 +179,7 @@ def register_chill_mask(mask: ChillMask):
         autotune: bool,
     ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
         return _run_backward(lib, functor_id, q, k, v, lens, o, lse, do, mask_args, sm_scale,
-                             flags=_precision_flags(precision, q.dtype))
+                             flags=_call_flags(precision, q.dtype))
 
     @torch.library.register_fake(f"chill_attention::backward{mask_name}")
     def attention_backward_adapter_abstract(q, k, v, lens, o, lse, do, mask_args, sm_scale, prescale_qk, precision,
@@ -209,7 +207,8 @@ def register_chill_mask(mask: ChillMask):
         mask_args: typing.List[typing.Union[int, float, bool]],
         sm_scale: float,
     ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
-        return _run_backward(lib, functor_id, q, k, v, lens, o, lse, do, mask_args, sm_scale, d_lse=dlse.float())
+        return _run_backward(lib, functor_id, q, k, v, lens, o, lse, do, mask_args, sm_scale, d_lse=dlse.float(),
+                             flags=_call_flags("ieee", q.dtype))
 
     @torch.library.register_fake(f"chill_attention::backward_with_dlse{mask_name}")
     def attention_backward_dlse_adapter_abstract(q, k, v, lens, o, lse, do, dlse, mask_args, sm_scale):
@@ -308,9 +307,8 @@ def chill_attention(
         precision: "ieee" or "tf32"; for fp32 inputs "tf32" runs forward and backward (head dim 64 / 128) on the
             tensor cores in TF32 (~1e-3 error instead of ~1e-6), everything else is IEEE fp32.
 
-    fp16 / bf16 tensors with head dim 16 or 32 are zero-padded to 64 channels here, so that they run the tensor-core
-    kernels (zero channels change neither Q K^T nor the first head_dim columns of P V; autograd slices the gradients
-    back).  The reference serves these head dims with tl.dot directly (chill.py:81-92).
+    fp16 / bf16 tensors with head dim 16 or 32 run the 64-channel tensor-core kernels on tiles that TMA fills up with
+    zeros.  The reference serves these head dims with tl.dot directly (chill.py:81-92).
 
     Returns: O, or (O, LSE) when ``return_lse``.
     """
@@ -320,22 +318,10 @@ def chill_attention(
         entry = _REGISTRY.get(mask.name)
     if sm_scale is None:
         sm_scale = 1.0 / (q.shape[-1] ** 0.5)
-    head_dim = q.shape[-1]
-    if head_dim in _PADDED_HEAD_DIMS and q.dtype in (torch.float16, torch.bfloat16) and q.is_cuda \
-            and k.shape[-1] == head_dim and v.shape[-1] == head_dim and k.dtype == q.dtype and v.dtype == q.dtype:
-        pad = (0, _PADDED_TO - head_dim)
-        out = chill_attention(
-            torch.nn.functional.pad(q, pad), torch.nn.functional.pad(k, pad), torch.nn.functional.pad(v, pad), mask,
-            lens=lens, sm_scale=sm_scale, return_lse=return_lse, prescale_qk=prescale_qk, precision=precision,
-            autotune=autotune,
-        )
-        if return_lse:
-            return out[0][..., :head_dim].contiguous(), out[1]
-        return out[..., :head_dim].contiguous()
     compiling = torch.compiler.is_compiling()
     if not compiling and entry is not None and _eager.usable(q, k, v, lens):
         # plain eager call: same kernels through the short host path (see _eager.py), which validates the arguments
-        flags = _precision_flags(precision, q.dtype)
+        flags = _call_flags(precision, q.dtype)
         return _eager.attention(entry, q, k, v, lens, mask.constargs, float(sm_scale), bool(return_lse), flags)
     if not compiling:
         for i in (q, k, v):

@@ -115,8 +115,8 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (n_it == 0) {
     // nobody attends these keys (padding, or outside every query's range on this shard)
     const int rows = imin(kTile, g.Lk - kb);
-    zero_rows<T, D>(reinterpret_cast<T*>(p.dk) + b * p.dk_sb + hk * p.dk_sh + kb * p.dk_sl, p.dk_sl, rows, kFusedThreads);
-    zero_rows<T, D>(reinterpret_cast<T*>(p.dv) + b * p.dv_sb + hk * p.dv_sh + kb * p.dv_sl, p.dv_sl, rows, kFusedThreads);
+    zero_rows<T>(reinterpret_cast<T*>(p.dk) + b * p.dk_sb + hk * p.dk_sh + kb * p.dk_sl, p.dk_sl, rows, g.D, kFusedThreads);
+    zero_rows<T>(reinterpret_cast<T*>(p.dv) + b * p.dv_sb + hk * p.dv_sh + kb * p.dv_sl, p.dv_sl, rows, g.D, kFusedThreads);
     zero_part_rows<D>(p.part, b, hk, kb, rows, g.Lk, kFusedThreads);
     return;
   }
@@ -502,7 +502,7 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 template <typename T, int D>
 __global__ void __launch_bounds__(256)
 dq_convert_kernel(const float* __restrict__ accum, T* __restrict__ dq, long long sb, long long sh, long long sl, int H,
-                  int Lq, float scale) {
+                  int Lq, int width, float scale) {
   const int qi = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   const int n_qt_total = gridDim.x;
   const float* src = accum + (((size_t)b * H + h) * n_qt_total + qi) * (size_t)(kTile * D);
@@ -510,6 +510,7 @@ dq_convert_kernel(const float* __restrict__ accum, T* __restrict__ dq, long long
   const int rows = imin(kTile, Lq - qi * kTile);
   for (int idx = threadIdx.x; idx < (kTile / 2) * (D / 4); idx += 256) {
     const int c4 = idx % (D / 4), r0 = (idx / (D / 4)) * 2;
+    if (D == 64 && 4 * c4 >= width) continue;  // channels of the tile that a narrow head does not have
     const float4* s4 = reinterpret_cast<const float4*>(src + (size_t)(r0 / 32) * (32 * D) + c4 * 128 + (r0 % 32) * 4);
     const float4 a = s4[0], bb = s4[1];
     if (r0 < rows)
@@ -540,7 +541,7 @@ int launch_bwd_fused_one(const CUtensorMap* maps, const BwdTcParams& p, cudaStre
   if (e != cudaSuccess) return (int)e;
   dim3 gc((unsigned)((g.Lq + kTile - 1) / kTile), (unsigned)g.H, (unsigned)g.B);
   dq_convert_kernel<T, D><<<gc, 256, 0, st>>>(p.dq_accum, reinterpret_cast<T*>(p.dq), p.dq_sb, p.dq_sh, p.dq_sl, g.H,
-                                               g.Lq, g.scale);
+                                               g.Lq, g.D, g.scale);
   return (int)cudaGetLastError();
 }
 

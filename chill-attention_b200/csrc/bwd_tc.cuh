@@ -77,11 +77,12 @@ enum : int {
   kStDqProducer = 301, kStDqMma = 302, kStDqCompute = 303, kStDqEpilogue = 304
 };
 
-// Zero `rows` rows of D 16-bit channels starting at `base` (row stride `sl` elements).
-template <typename T, int D>
-__device__ __forceinline__ void zero_rows(T* base, long long sl, int rows, int nthreads) {
-  for (int idx = threadIdx.x; idx < rows * (D / 8); idx += nthreads) {
-    const int r = idx / (D / 8), c = idx % (D / 8);
+// Zero `rows` rows of `width` 16-bit channels starting at `base` (row stride `sl` elements).
+template <typename T>
+__device__ __forceinline__ void zero_rows(T* base, long long sl, int rows, int width, int nthreads) {
+  const int units = width / 8;
+  for (int idx = threadIdx.x; idx < rows * units; idx += nthreads) {
+    const int r = idx / units, c = idx % units;
     *reinterpret_cast<uint4*>(base + r * sl + c * 8) = make_uint4(0, 0, 0, 0);
   }
 }
@@ -180,8 +181,8 @@ bwd_dkdv_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   if (n_it == 0) {
     // nobody attends these keys (padding, or outside every query's range on this shard)
     const int rows = imin(kTile, g.Lk - kb);
-    zero_rows<T, D>(reinterpret_cast<T*>(p.dk) + b * p.dk_sb + hk * p.dk_sh + kb * p.dk_sl, p.dk_sl, rows, kBwdThreads);
-    zero_rows<T, D>(reinterpret_cast<T*>(p.dv) + b * p.dv_sb + hk * p.dv_sh + kb * p.dv_sl, p.dv_sl, rows, kBwdThreads);
+    zero_rows<T>(reinterpret_cast<T*>(p.dk) + b * p.dk_sb + hk * p.dk_sh + kb * p.dk_sl, p.dk_sl, rows, g.D, kBwdThreads);
+    zero_rows<T>(reinterpret_cast<T*>(p.dv) + b * p.dv_sb + hk * p.dv_sh + kb * p.dv_sl, p.dv_sl, rows, g.D, kBwdThreads);
     zero_part_rows<D>(p.part, b, hk, kb, rows, g.Lk, kBwdThreads);
     return;
   }
@@ -531,8 +532,8 @@ bwd_dq_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
   const int n_it = kt_hi - kt_lo;
   if (n_it == 0) {
-    zero_rows<T, D>(reinterpret_cast<T*>(p.dq) + b * p.dq_sb + h * p.dq_sh + qb * p.dq_sl, p.dq_sl,
-                    imin(kTile, g.Lq - qb), kBwdThreads);
+    zero_rows<T>(reinterpret_cast<T*>(p.dq) + b * p.dq_sb + h * p.dq_sh + qb * p.dq_sl, p.dq_sl,
+                    imin(kTile, g.Lq - qb), g.D, kBwdThreads);
     return;
   }
 

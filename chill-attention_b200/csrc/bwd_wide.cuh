@@ -96,7 +96,7 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
   const long long o_sh = MODE == kWideDV ? p.dv_sh : (MODE == kWideDK ? p.dk_sh : p.dq_sh);
   const long long o_sl = MODE == kWideDV ? p.dv_sl : (MODE == kWideDK ? p.dk_sl : p.dq_sl);
   if (n_it == 0) {  // padding rows, or rows nothing on this shard can see: zero gradient
-    zero_rows<T, D>(out_base + b * o_sb + hr * o_sh + rb * o_sl, o_sl, rows_here, kWideThreads);
+    zero_rows<T>(out_base + b * o_sb + hr * o_sh + rb * o_sl, o_sl, rows_here, D, kWideThreads);
     if (MODE == kWideDV) zero_part_rows<D>(p.part, b, hr, rb, rows_here, g.Lk, kWideThreads);  // dK and dV partials
     return;
   }

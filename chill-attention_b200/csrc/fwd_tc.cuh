@@ -16,6 +16,8 @@
 //
 // TMEM columns: kSBufs buffers of KT fp32 columns for S, each overlaid by its P (16-bit, first KT / 2
 // columns); then D columns of O.
+// Head dims 16 and 32 run the head-dim-64 kernels (here and in the backward): the tensor maps have the true width, so TMA
+// fills the missing channels of a 64-channel box with zeros on load and drops them on store.
 // Reference math: chill_attention/chill_fwd.py:188-359 (three-segment key loop, base-2
 // online softmax, LSE = m + log2 l); the segment split is replaced by a per-tile "full tile"
 // test derived from the functor's k_full_range_for_q.
@@ -275,8 +277,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     // its zero-initialised outputs, chill_fwd.py:70-71).
     T* obase = reinterpret_cast<T*>(p.o) + b * p.o_sb + h * p.o_sh;
     const int rows = imin(kTile, g.Lq - qb);
-    for (int idx = threadIdx.x; idx < rows * (D / 8); idx += kFwdThreads) {
-      const int r = idx / (D / 8), c = idx % (D / 8);
+    const int units = g.D / 8;
+    for (int idx = threadIdx.x; idx < rows * units; idx += kFwdThreads) {
+      const int r = idx / units, c = idx % units;
       *reinterpret_cast<uint4*>(obase + (qb + r) * p.o_sl + c * 8) = make_uint4(0, 0, 0, 0);
     }
     if (p.lse != nullptr)

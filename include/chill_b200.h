@@ -85,6 +85,8 @@ extern "C" {
                                      * (chill_fwd.py:13-359, chill_bwd_dq.py:312, chill_bwd_dkdv.py:347:
                                      * input_precision).  Without the flag, and for other head dims, fp32 is
                                      * computed in IEEE fp32 by the generic kernels. */
+#define CHILL_FLAG_NARROW_HEAD 64u  /* 16-bit head dim 16 / 32 may run the tensor-core kernels (P and dS rounded to 16 bits
+                                     * like every tensor-core call); without it they take the fp32 CUDA-core kernels */
 
 /* The mask constants a ChillMask instance was built with (ChillMask.constargs,
  * mask.py:31-49).  Each is passed both ways: `i[n]` = the value truncated to an
