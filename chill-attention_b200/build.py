@@ -40,7 +40,7 @@ def _nvcc():
 
 def _sources_digest(extra=()):
     h = hashlib.sha256()
-    names = sorted(os.listdir(CSRC)) + [os.path.join(INCLUDE, "chill_b200.h")]
+    names = sorted(n for n in os.listdir(CSRC) if n != "torch_ext.cpp") + [os.path.join(INCLUDE, "chill_b200.h")]
     for name in names:
         path = name if os.path.isabs(name) else os.path.join(CSRC, name)
         if os.path.isfile(path):
@@ -99,6 +99,34 @@ def build_library(out_path=None, custom_header=None, custom_functor=None, verbos
     return out_path
 
 
+def build_extension(force=False):
+    """Compile the native eager-mode call path (csrc/torch_ext.cpp) against the installed torch; returns its path."""
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    out = os.path.join(LIB_DIR, "_chill_torch.so")
+    src = os.path.join(CSRC, "torch_ext.cpp")
+    h = hashlib.sha256((torch.__version__ + sys.version).encode())
+    for path in (src, os.path.join(INCLUDE, "chill_b200.h")):
+        with open(path, "rb") as f:
+            h.update(f.read())
+    stamp = out + ".stamp"
+    if not force and os.path.exists(out) and os.path.exists(stamp) and open(stamp).read() == h.hexdigest():
+        return out
+    os.makedirs(LIB_DIR, exist_ok=True)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    includes = include_paths() + [os.path.join(cuda, "include"), sysconfig.get_paths()["include"], INCLUDE]
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+          "-DTORCH_EXTENSION_NAME=_chill_torch"] + [x for i in includes for x in ("-isystem", i)] + [src, "-o", out]
+         + [f"-L{p}" for p in library_paths()] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+    with open(stamp, "w") as f:
+        f.write(h.hexdigest())
+    return out
+
+
 if __name__ == "__main__":
     path = build_library(verbose="-v" in sys.argv, force="-f" in sys.argv)
     print(path)
+    print(build_extension(force="-f" in sys.argv))

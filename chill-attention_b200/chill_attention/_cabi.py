@@ -229,6 +229,10 @@ def set_deterministic(flag: bool) -> None:
     ``torch.use_deterministic_algorithms(True)`` is set or CHILL_ATTENTION_DETERMINISTIC=1."""
     global _deterministic
     _deterministic = bool(flag)
+    from . import _eager
+
+    if _eager._extension is not None:  # otherwise handed over when the extension is loaded
+        _eager._extension.set_deterministic(_deterministic)
 
 
 def is_deterministic() -> bool:

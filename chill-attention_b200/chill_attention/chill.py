@@ -31,12 +31,17 @@ logger = logging.getLogger(__name__)
 
 _HEAD_DIMS = {16, 32, 64, 128, 256}
 #: how many backward calls each kernel family served (read by tests; see backward_path_counts)
-_BWD_PATHS = {"tensor_core": 0, "generic": 0}
+_BWD_PATHS = {"tensor_core": 0, "generic": 0}  # calls through the dispatcher ops; the eager path counts its own
 
 
 def backward_path_counts() -> dict:
     """Copy of the per-process counters of backward calls served by the tensor-core and by the generic kernels."""
-    return dict(_BWD_PATHS)
+    counts = dict(_BWD_PATHS)
+    if _eager._extension is not None:
+        tc, generic = _eager._extension.backward_counts()
+        counts["tensor_core"] += tc
+        counts["generic"] += generic
+    return counts
 
 
 def _backward_operand(do: torch.Tensor) -> torch.Tensor:
@@ -86,8 +91,12 @@ def _run_backward(lib, functor_id, q, k, v, lens, o, lse, do, mask_args, sm_scal
         _cabi.check(lib, lib.chill_bwd_delta(C.byref(a), st), "chill_bwd_delta")
         _cabi.check(lib, lib.chill_bwd(C.byref(a), st), "chill_bwd")
     return DQ, DK, DV
+
+
 #: mask class name -> (library, functor id); filled by register_chill_mask
 _REGISTRY: dict[str, tuple] = {}
+#: mask class name -> native call object of the eager path (_eager.py), made on its first eager call
+_NATIVE: dict[str, object] = {}
 
 
 def _resolve_functor(mask: ChillMask):
@@ -127,7 +136,7 @@ def register_chill_mask(mask: ChillMask):
     if hasattr(torch.ops.chill_attention, f"forward{mask_name}"):
         return
     lib, functor_id = _resolve_functor(mask)
-    _REGISTRY[mask_name] = (lib, functor_id)  # also what the eager call path (_eager.py) looks up
+    _REGISTRY[mask_name] = (lib, functor_id)
 
     @torch.library.custom_op(f"chill_attention::forward{mask_name}", mutates_args=(), device_types=("cuda",))
     def attention_forward_adapter(
@@ -312,17 +321,22 @@ def chill_attention(
 
     Returns: O, or (O, LSE) when ``return_lse``.
     """
-    entry = _REGISTRY.get(mask.name)
-    if entry is None:
+    if mask.name not in _REGISTRY:
         register_chill_mask(mask)
-        entry = _REGISTRY.get(mask.name)
     if sm_scale is None:
         sm_scale = 1.0 / (q.shape[-1] ** 0.5)
     compiling = torch.compiler.is_compiling()
-    if not compiling and entry is not None and _eager.usable(q, k, v, lens):
-        # plain eager call: same kernels through the short host path (see _eager.py), which validates the arguments
-        flags = _call_flags(precision, q.dtype)
-        return _eager.attention(entry, q, k, v, lens, mask.constargs, float(sm_scale), bool(return_lse), flags)
+    if not compiling and _eager.usable(q, k, v, lens):
+        # plain eager call: same kernels through the short host path (see _eager.py)
+        native = _NATIVE.get(mask.name)
+        if native is None and mask.name in _REGISTRY:
+            native = _NATIVE[mask.name] = _eager.native_library(*_REGISTRY[mask.name])
+        if native is not None:
+            out = _eager.attention(native, q, k, v, lens, mask.constargs, sm_scale, bool(return_lse), _call_flags(precision, q.dtype))
+            if out is not None:
+                return out
+            _check_inputs(q, k, v, lens, sm_scale)  # says which argument is wrong
+            raise AssertionError("q, k, v and lens must be on one device")
     if not compiling:
         for i in (q, k, v):
             if getattr(i, "_dynamo_static_indices", None) != {1, 3}:
