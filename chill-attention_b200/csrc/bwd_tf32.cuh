@@ -15,10 +15,16 @@
 //   * an fp32 operand read MN-major (dO and Q as B of the dV / dK GEMMs, K as B of the dQ GEMM) needs the
 //     "128-byte swizzle with 32-byte atoms" layout, a K-major one the plain 128-byte swizzle (a K-major descriptor
 //     does not take the 32-byte-atom layout), so those tiles are loaded twice, once per layout.  Shared memory
-//     then decides the size TO of the streamed tiles: 128 positions at head dim 64 (64 KB resident + 128 KB
-//     streamed), 32 at head dim 128 (128 KB resident + 64 KB streamed).
-// The kernels are deliberately plain: one ring stage, the tensor cores and the compute warps alternate.  They run
-// at a few hundred TFLOP/s where the IEEE kernels (simt.cuh) that otherwise serve fp32 reach about thirty.
+//     then decides the size TO of the streamed tiles: 64 positions at head dim 64, 32 at head dim 128.
+//
+// Pipeline: the score GEMMs of step it + 1 are issued before the accumulate GEMMs of step it, into the other of two
+// S / dP column pairs, so they run while the compute warps work on step it, and the accumulate GEMMs of step it run
+// while those work on step it + 1.  That needs two stages of the tiles the score GEMMs read; the MN-major copies, which
+// only the accumulate GEMMs read, get what shared memory is left (one stage each at head dim 128, with barriers of
+// their own so that dO is refilled as soon as dV has used it).  With a single stage and one S / dP pair the tensor
+// cores and the compute warps alternated (5300 clocks per 32-query step against about 2000 of MMA issue).  Causal fp32
+// (B, H, L, D) = (2, 16, 4096, 128): dK/dV 1305 -> 801 us, dQ 1210 -> 639 us (354 and 333 TFLOP/s executed).  What bounds
+// them now is the issue of the score MMAs, 16 per GEMM at N = 32, which read a 4 KB A slice from shared memory for each.
 // Inputs are used as they are (the tensor core drops all but 10 mantissa bits); gradients match the fp64 oracle
 // to about 1e-3 relative on N(0,1) inputs (the tests state 5e-3).
 #pragma once
@@ -35,23 +41,25 @@ enum : int { kStTfProducer = 501, kStTfMma = 502, kStTfCompute = 503, kStTfEpilo
 // D: head dim; TO: positions per streamed tile (queries in the dK/dV kernel, keys in the dQ kernel).
 template <int D>
 struct Tf32Shape {
-  static constexpr int TO = (D == 64) ? 128 : 32;
-  static constexpr int kChunks = D / 32;                       // 128-byte column blocks per row
+  static constexpr int TO = (D == 64) ? 64 : 32;
+  static constexpr int kStages = 2;                            // stages of the score operands, S / dP column pairs
+  static constexpr int kAccStages = (D == 64) ? 2 : 1;         // dK/dV kernel: stages of the MN-major dO and Q tiles
   static constexpr int kFixBytes = kTile * D * 4;              // a resident tile: 128 positions
-  static constexpr int kFixChunkBytes = kTile * 128;
+  static constexpr int kFixChunkBytes = kTile * 128;           // 128-byte column blocks, D / 32 per tile
   static constexpr int kRingBytes = TO * D * 4;                // a streamed tile: TO positions
   static constexpr int kRingChunkBytes = TO * 128;
   static constexpr int kFixA = 0;                              // K (dkdv) or Q (dq), K-major
   static constexpr int kFixB = kFixA + kFixBytes;              // V (dkdv) or dO (dq), K-major
-  static constexpr int kRing = kFixB + kFixBytes;              // up to four streamed tiles
-  static constexpr int kRows = kRing + 4 * kRingBytes;         // per compute warp: -lse[TO/2], -delta[TO/2] (dkdv)
-  static constexpr int kBars = kRows + 8 * 2 * 64 * 4;
-  static constexpr int kNumBars = 6;
+  static constexpr int kRing = kFixB + kFixBytes;              // kStages x [Q | dO] (dkdv) or [K | V] (dq), K-major
+  static constexpr int kAcc = kRing + 2 * kStages * kRingBytes;  // kAccStages x [dO | Q] (dkdv) or two stages of K (dq), MN-major
+  static constexpr int kRows = kAcc + 2 * kAccStages * kRingBytes;  // per compute warp: -lse[TO/2], -delta[TO/2] (dkdv)
+  static constexpr int kBars = kRows + 8 * 2 * (TO / 2) * 4;
+  static constexpr int kNumBars = 16;
   static constexpr int kMisc = kBars + 8 * kNumBars;
   static constexpr int kTotal = kMisc + 16;
   static constexpr int kDynamic = kTotal + 1024;
   static_assert(kDynamic <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
-  static_assert(256 + 2 * D <= 512, "TMEM columns");
+  static_assert(kStages * TO <= 128 && 256 + 2 * D <= 512, "TMEM columns");
   // 16-byte units to add to a K-major descriptor for MMA step kk (8 channels = 32 bytes) of a tile whose column
   // blocks are `chunk_bytes` apart
   __host__ __device__ static constexpr uint32_t kstep(int kk, int chunk_bytes) {
@@ -87,7 +95,7 @@ __device__ __forceinline__ void tmem_st_cols(uint32_t taddr, const uint32_t* r) 
 }
 
 // ============================================================================ dK / dV
-// TMEM: S^T / P^T at column 0 (TO columns), dP^T / dS^T at 128 (TO), dV at 256 (D), dK at 256 + D (D).
+// TMEM: two buffers of S^T / P^T at column 0 (TO columns each), of dP^T / dS^T at 128, dV at 256 (D), dK at 256 + D (D).
 template <int D, class M>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_constant__ CUtensorMap tmQm,
@@ -96,7 +104,6 @@ bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_cons
   using L = Tf32Shape<D>;
   constexpr int TO = L::TO;     // queries per streamed tile
   constexpr int CW = TO / 2;    // query columns per compute warp
-  constexpr int CC = CW < 32 ? CW : 32;  // columns per TMEM access
   const Geo& g = p.g;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int hb, kt;
@@ -135,11 +142,14 @@ bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_cons
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t sK = base + L::kFixA, sV = base + L::kFixB;
-  const uint32_t sQk = base + L::kRing, sQm = sQk + L::kRingBytes, sdOk = sQm + L::kRingBytes, sdOm = sdOk + L::kRingBytes;
+  const uint32_t sRing = base + L::kRing, sAcc = base + L::kAcc;
   float* rows_s = reinterpret_cast<float*>(gen_base + L::kRows);
   const uint32_t bars = base + L::kBars;
-  const uint32_t bar_kv_full = bars, bar_ring_full = bars + 8, bar_ring_empty = bars + 16, bar_sdp_full = bars + 24,
-                 bar_ds_full = bars + 32, bar_acc_full = bars + 40;
+  // One barrier per buffer throughout: nobody can run a whole round of a ring ahead of a waiter, so parities cannot alias.
+  // sdp_full[s] (scores of a step complete) is also what frees stage s of the ring.
+  const uint32_t bar_kv_full = bars, bar_acc_full = bars + 8, bar_ring_full = bars + 16, bar_sdp_full = bars + 32,
+                 bar_ds_full = bars + 48, bar_do_full = bars + 64, bar_do_empty = bars + 80, bar_q_full = bars + 96,
+                 bar_q_empty = bars + 112;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen_base + L::kMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_base + L::kMisc + 4);
   const Guard guard{p.status, abort_flag};
@@ -148,11 +158,16 @@ bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_cons
     if (lane == 0) {
       *abort_flag = 0;
       mbar_init(bar_kv_full, 1);
-      mbar_init(bar_ring_full, 1);
-      mbar_init(bar_ring_empty, 1);
-      mbar_init(bar_sdp_full, 1);
-      mbar_init(bar_ds_full, kBwdComputeThreads / 32);
       mbar_init(bar_acc_full, 1);
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(bar_ring_full + 8 * s, 1);
+        mbar_init(bar_sdp_full + 8 * s, 1);
+        mbar_init(bar_ds_full + 8 * s, kBwdComputeThreads / 32);
+        mbar_init(bar_do_full + 8 * s, 1);
+        mbar_init(bar_do_empty + 8 * s, 1);
+        mbar_init(bar_q_full + 8 * s, 1);
+        mbar_init(bar_q_empty + 8 * s, 1);
+      }
       fence_barrier_init();
       fence_proxy_async_smem();
       mbar_arrive_expect_tx(bar_kv_full, 2 * L::kFixBytes);
@@ -170,19 +185,36 @@ bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_cons
   const uint32_t tSt = tmem, tdPt = tmem + 128, tdV = tmem + 256, tdK = tmem + 256 + D;
 
   if (warp == 8) {
-    // --------------------------------------------------------------------- TMA producer (one ring stage)
+    // --------------------------------------------------------------------- TMA producer
     if (lane == 0) {
       bool ok = true;
+      auto load_scores = [&](int it) -> bool {  // K-major Q and dO of step `it`
+        const int s = it % L::kStages, h = hk * G + it / n_qt, qrow = (qt_lo + it % n_qt) * TO;
+        if (it >= L::kStages && !mbar_wait(bar_sdp_full + 8 * s, (uint32_t)(it / L::kStages - 1) & 1u, guard, kStTfProducer)) return false;
+        const uint32_t dst = sRing + s * 2 * L::kRingBytes;
+        mbar_arrive_expect_tx(bar_ring_full + 8 * s, 2 * L::kRingBytes);
+        tma_tile_f32<D, TO>(dst, &tmQk, bar_ring_full + 8 * s, qrow, h, b);
+        tma_tile_f32<D, TO>(dst + L::kRingBytes, &tmdOk, bar_ring_full + 8 * s, qrow, h, b);
+        return true;
+      };
+      auto load_acc = [&](int it) -> bool {  // MN-major dO and Q of step `it`
+        const int s = it % L::kAccStages, h = hk * G + it / n_qt, qrow = (qt_lo + it % n_qt) * TO;
+        const uint32_t dst = sAcc + s * 2 * L::kRingBytes, par = ((uint32_t)(it / L::kAccStages) & 1u) ^ 1u;
+        if (!mbar_wait(bar_do_empty + 8 * s, par, guard, kStTfProducer)) return false;
+        mbar_arrive_expect_tx(bar_do_full + 8 * s, L::kRingBytes);
+        tma_tile_f32<D, TO>(dst, &tmdOm, bar_do_full + 8 * s, qrow, h, b);
+        if (!mbar_wait(bar_q_empty + 8 * s, par, guard, kStTfProducer)) return false;
+        mbar_arrive_expect_tx(bar_q_full + 8 * s, L::kRingBytes);
+        tma_tile_f32<D, TO>(dst + L::kRingBytes, &tmQm, bar_q_full + 8 * s, qrow, h, b);
+        return true;
+      };
+      // in the order in which the tensor cores free the buffers: scores(it + 1), accumulate(it), scores(it + 2), ...
+      for (int it = 0; it < imin(n_it, 2); ++it) load_scores(it);  // the first round waits for nothing
+      for (int it = 0; it < imin(n_it, L::kAccStages); ++it) load_acc(it);
+      if (n_it > 2) ok = load_scores(2);
       for (int it = 0; it < n_it && ok; ++it) {
-        const int h = hk * G + it / n_qt;
-        const int qrow = (qt_lo + it % n_qt) * TO;
-        ok = mbar_wait(bar_ring_empty, ((uint32_t)it & 1u) ^ 1u, guard, kStTfProducer);
-        if (!ok) break;
-        mbar_arrive_expect_tx(bar_ring_full, 4 * L::kRingBytes);
-        tma_tile_f32<D, TO>(sQk, &tmQk, bar_ring_full, qrow, h, b);
-        tma_tile_f32<D, TO>(sQm, &tmQm, bar_ring_full, qrow, h, b);
-        tma_tile_f32<D, TO>(sdOk, &tmdOk, bar_ring_full, qrow, h, b);
-        tma_tile_f32<D, TO>(sdOm, &tmdOm, bar_ring_full, qrow, h, b);
+        if (it + 3 < n_it) ok = load_scores(it + 3);
+        if (ok && it + L::kAccStages < n_it) ok = load_acc(it + L::kAccStages);
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
@@ -197,36 +229,49 @@ bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_cons
       constexpr uint32_t hi_k = desc_hi_sw128(1024);         // K-major tiles: 8-row groups 1 KB apart
       constexpr uint32_t hi_m = desc_hi_sw128_base32(512);   // MN-major fp32 tiles: 4-row groups 512 B apart
       const uint32_t k_lo = desc_lo_sw128(sK, 16), v_lo = desc_lo_sw128(sV, 16);
-      const uint32_t qk_lo = desc_lo_sw128(sQk, 16), dok_lo = desc_lo_sw128(sdOk, 16);
-      const uint32_t qm_lo = desc_lo_sw128(sQm, L::kRingChunkBytes), dom_lo = desc_lo_sw128(sdOm, L::kRingChunkBytes);
       bool ok = mbar_wait(bar_kv_full, 0, guard, kStTfMma);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const uint32_t par = (uint32_t)it & 1u;
-        ok = mbar_wait(bar_ring_full, par, guard, kStTfMma);
-        if (!ok) break;
+      // S^T = K Q^T and dP^T = V dO^T: 8 channels (32 bytes) per instruction.  They overwrite P^T / dS^T of step it - 2,
+      // which the accumulate GEMMs issued before them have consumed (issue order).
+      auto issue_scores = [&](int it) -> bool {
+        const int s = it % L::kStages;
+        if (!mbar_wait(bar_ring_full + 8 * s, (uint32_t)(it / L::kStages) & 1u, guard, kStTfMma)) return false;
         tc_fence_after();
-        // S^T = K Q^T and dP^T = V dO^T: 8 channels (32 bytes) per instruction.  They overwrite P^T / dS^T of the
-        // previous query tile, which the accumulate GEMMs issued before them have consumed (issue order).
+        const uint32_t q_lo = desc_lo_sw128(sRing + s * 2 * L::kRingBytes, 16);
+        const uint32_t do_lo = desc_lo_sw128(sRing + s * 2 * L::kRingBytes + L::kRingBytes, 16);
 #pragma unroll
         for (int kk = 0; kk < D / 8; ++kk)
-          mma_ss_tf32(tSt, k_lo + L::kstep(kk, L::kFixChunkBytes), qk_lo + L::kstep(kk, L::kRingChunkBytes), hi_k, idesc_s,
-                      kk > 0 ? 1u : 0u);
+          mma_ss_tf32(tSt + s * TO, k_lo + L::kstep(kk, L::kFixChunkBytes), q_lo + L::kstep(kk, L::kRingChunkBytes), hi_k,
+                      idesc_s, kk > 0 ? 1u : 0u);
 #pragma unroll
         for (int kk = 0; kk < D / 8; ++kk)
-          mma_ss_tf32(tdPt, v_lo + L::kstep(kk, L::kFixChunkBytes), dok_lo + L::kstep(kk, L::kRingChunkBytes), hi_k, idesc_s,
-                      kk > 0 ? 1u : 0u);
-        mma_commit(bar_sdp_full);
-        ok = mbar_wait(bar_ds_full, par, guard, kStTfMma);
+          mma_ss_tf32(tdPt + s * TO, v_lo + L::kstep(kk, L::kFixChunkBytes), do_lo + L::kstep(kk, L::kRingChunkBytes), hi_k,
+                      idesc_s, kk > 0 ? 1u : 0u);
+        mma_commit(bar_sdp_full + 8 * s);
+        return true;
+      };
+      if (ok) ok = issue_scores(0);
+      for (int it = 0; it < n_it && ok; ++it) {
+        const int s = it % L::kStages, sa = it % L::kAccStages;
+        const uint32_t acc_par = (uint32_t)(it / L::kAccStages) & 1u;
+        if (it + 1 < n_it) ok = issue_scores(it + 1);
+        if (ok) ok = mbar_wait(bar_do_full + 8 * sa, acc_par, guard, kStTfMma);
+        if (ok) ok = mbar_wait(bar_ds_full + 8 * s, (uint32_t)(it / L::kStages) & 1u, guard, kStTfMma);
         if (!ok) break;
         tc_fence_after();
         // dV += P^T dO, dK += dS^T Q: A from TMEM (8 queries = 8 columns per step), B = 8 rows (1 KB) of dO / Q
+        const uint32_t dom_lo = desc_lo_sw128(sAcc + sa * 2 * L::kRingBytes, L::kRingChunkBytes);
+        const uint32_t qm_lo = desc_lo_sw128(sAcc + sa * 2 * L::kRingBytes + L::kRingBytes, L::kRingChunkBytes);
 #pragma unroll
         for (int kk = 0; kk < TO / 8; ++kk)
-          mma_ts_tf32(tdV, tSt + kk * 8, dom_lo + kk * 64, hi_m, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
+          mma_ts_tf32(tdV, tSt + s * TO + kk * 8, dom_lo + kk * 64, hi_m, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(bar_do_empty + 8 * sa);
+        ok = mbar_wait(bar_q_full + 8 * sa, acc_par, guard, kStTfMma);
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < TO / 8; ++kk)
-          mma_ts_tf32(tdK, tdPt + kk * 8, qm_lo + kk * 64, hi_m, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(bar_ring_empty);
+          mma_ts_tf32(tdK, tdPt + s * TO + kk * 8, qm_lo + kk * 64, hi_m, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(bar_q_empty + 8 * sa);
       }
       if (ok) mma_commit(bar_acc_full);
     }
@@ -239,60 +284,70 @@ bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_cons
     const int kg = kg0 + r;
     const bool key_ok = kg < n && kb + r < g.Lk;
     const float c = g.scale * kLog2e;
-    float* slot = rows_s + warp * 128;  // warp-private: [0, CW) -LSE, [64, 64 + CW) -delta of this warp's columns
+    static_assert(CW <= 32, "one query column per lane");
+    float* slot = rows_s + warp * 2 * CW;  // warp-private: [0, CW) -LSE, [CW, 2 CW) -delta of this warp's columns
+    // LSE / delta of this lane's query column, fetched a step ahead and not touched until then
+    auto fetch_rows = [&](int it, float& lv, float& dl) {
+      const int h = hk * G + it / n_qt;
+      const int qrow = (qt_lo + it % n_qt) * TO + c0 + (CW < 32 ? lane % CW : lane);
+      const bool in = qrow < g.Lq;  // row 0 stands in for rows beyond Lq: those columns are masked out anyway
+      lv = __ldg(p.lse + b * p.lse_sb + h * p.lse_sh + (in ? qrow : 0) * p.lse_sl);
+      dl = __ldg(p.delta + ((long long)b * g.H + h) * g.Lq + (in ? qrow : 0));
+    };
+    float lse_next, delta_next;
+    fetch_rows(0, lse_next, delta_next);
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
-      const uint32_t par = (uint32_t)it & 1u;
-      const int h = hk * G + it / n_qt;
+      const int sb = it % L::kStages;
       const int qi = qt_lo + it % n_qt;
       const int qg0 = qi * TO + g.q_off;
       __syncwarp();
-      for (int e = lane; e < CW; e += 32) {
-        const int qrow = qi * TO + c0 + e;
-        const bool in = qrow < g.Lq;
-        const float lv = p.lse[b * p.lse_sb + h * p.lse_sh + (in ? qrow : 0) * p.lse_sl];
-        const float dl = p.delta[((long long)b * g.H + h) * g.Lq + (in ? qrow : 0)];
-        slot[e] = (lv == -CUDART_INF_F) ? 0.f : -lv;
-        slot[64 + e] = -dl;
+      if (lane < CW) {
+        slot[lane] = (lse_next == -CUDART_INF_F) ? 0.f : -lse_next;
+        slot[CW + lane] = -delta_next;
       }
       __syncwarp();
+      if (it + 1 < n_it) fetch_rows(it + 1, lse_next, delta_next);
       const bool full = M::kHasQFullRange && qg0 >= full_lo && qg0 + TO <= full_hi && qg0 + TO <= n &&
                         qi * TO + TO <= g.Lq && kg0 + kTile <= n && kb + kTile <= g.Lk;
       const int qlim = imin(n - qg0, g.Lq - qi * TO);
       int w_lo = 0, w_hi = -1;  // visible query columns of this key row inside the tile (interval functors)
       if (interval_rows<M>::value && !full && key_ok) row_window<M, false>(kg, qg0, qlim, n, g.margs, w_lo, w_hi);
-      ok = mbar_wait(bar_sdp_full, par, guard, kStTfCompute);
+      ok = mbar_wait(bar_sdp_full + 8 * sb, (uint32_t)(it / L::kStages) & 1u, guard, kStTfCompute);
       ok = __all_sync(0xffffffffu, ok);  // keep the warp converged for the .sync.aligned TMEM accesses
       if (!ok) break;
       tc_fence_after();
-#pragma unroll
-      for (int part = 0; part < CW / CC; ++part) {
-        const int cb = c0 + part * CC;
-        uint32_t sreg[CC], dpreg[CC];
-        tmem_ld_cols<CC>(tSt + lane_sel + cb, sreg);
-        tmem_ld_cols<CC>(tdPt + lane_sel + cb, dpreg);
+      {
+        const uint32_t tSb = tSt + sb * TO + lane_sel + c0, tdPb = tdPt + sb * TO + lane_sel + c0;
+        uint32_t sreg[CW], dpreg[CW];
+        tmem_ld_cols<CW>(tSb, sreg);
+        tmem_ld_cols<CW>(tdPb, dpreg);
         tmem_wait_ld();
+        auto body = [&](auto masked_tag) {  // two copies: full tiles run without any mask arithmetic
+          constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
-        for (int j = 0; j < CC; ++j) {
-          const int cq = cb + j;
-          float pv = ex2(fmaf(__uint_as_float(sreg[j]), c, slot[part * CC + j]));
-          bool vis = full;
-          if (!full) {
-            if (interval_rows<M>::value) vis = cq >= w_lo && cq <= w_hi;
-            else vis = key_ok && cq < qlim && M::mask(qg0 + cq, kg, n, g.margs);
+          for (int j = 0; j < CW; ++j) {
+            const int cq = c0 + j;
+            float pv = ex2(fmaf(__uint_as_float(sreg[j]), c, slot[j]));
+            if (kMasked) {
+              const bool vis = interval_rows<M>::value ? (cq >= w_lo && cq <= w_hi)
+                                                       : (key_ok && cq < qlim && M::mask(qg0 + cq, kg, n, g.margs));
+              pv = vis ? pv : 0.f;
+            }
+            const float ds = pv * (__uint_as_float(dpreg[j]) + slot[CW + j]);
+            sreg[j] = to_tf32(pv);
+            dpreg[j] = to_tf32(ds);
           }
-          pv = vis ? pv : 0.f;
-          const float ds = pv * (__uint_as_float(dpreg[j]) + slot[64 + part * CC + j]);
-          sreg[j] = to_tf32(pv);
-          dpreg[j] = to_tf32(ds);
-        }
-        tmem_st_cols<CC>(tSt + lane_sel + cb, sreg);    // P^T over the scores it came from
-        tmem_st_cols<CC>(tdPt + lane_sel + cb, dpreg);  // dS^T over dP^T
+        };
+        if (full) body(std::false_type{});
+        else body(std::true_type{});
+        tmem_st_cols<CW>(tSb, sreg);    // P^T over the scores it came from
+        tmem_st_cols<CW>(tdPb, dpreg);  // dS^T over dP^T
       }
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_ds_full);
+      if (lane == 0) mbar_arrive(bar_ds_full + 8 * sb);
     }
 
     // ---- epilogue: warps 0-3 store dV, warps 4-7 store dK * sm_scale, one fp32 row per thread
@@ -328,7 +383,7 @@ bwd_dkdv_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_cons
 }
 
 // ================================================================================ dQ
-// TMEM: S at column 0 (TO columns), dP / dS at 128 (TO), dQ at 256 (D).
+// TMEM: two buffers of S at column 0 (TO columns each), of dP / dS at 128, dQ at 256 (D).
 template <int D, class M>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_constant__ CUtensorMap tmKk,
@@ -337,7 +392,6 @@ bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_consta
   using L = Tf32Shape<D>;
   constexpr int TO = L::TO;     // keys per streamed tile
   constexpr int CW = TO / 2;
-  constexpr int CC = CW < 32 ? CW : 32;
   const Geo& g = p.g;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qt_total = (g.Lq + kTile - 1) / kTile;
@@ -374,10 +428,10 @@ bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_consta
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
   const uint32_t sQ = base + L::kFixA, sdO = base + L::kFixB;
-  const uint32_t sKk = base + L::kRing, sKm = sKk + L::kRingBytes, sVk = sKm + L::kRingBytes;
+  const uint32_t sRing = base + L::kRing, sKm = base + L::kAcc;
   const uint32_t bars = base + L::kBars;
-  const uint32_t bar_q_full = bars, bar_ring_full = bars + 8, bar_ring_empty = bars + 16, bar_sdp_full = bars + 24,
-                 bar_ds_full = bars + 32, bar_acc_full = bars + 40;
+  const uint32_t bar_q_full = bars, bar_acc_full = bars + 8, bar_ring_full = bars + 16, bar_sdp_full = bars + 32,
+                 bar_ds_full = bars + 48, bar_km_full = bars + 64, bar_km_empty = bars + 80;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen_base + L::kMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_base + L::kMisc + 4);
   const Guard guard{p.status, abort_flag};
@@ -386,11 +440,14 @@ bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_consta
     if (lane == 0) {
       *abort_flag = 0;
       mbar_init(bar_q_full, 1);
-      mbar_init(bar_ring_full, 1);
-      mbar_init(bar_ring_empty, 1);
-      mbar_init(bar_sdp_full, 1);
-      mbar_init(bar_ds_full, kBwdComputeThreads / 32);
       mbar_init(bar_acc_full, 1);
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(bar_ring_full + 8 * s, 1);
+        mbar_init(bar_sdp_full + 8 * s, 1);
+        mbar_init(bar_ds_full + 8 * s, kBwdComputeThreads / 32);
+        mbar_init(bar_km_full + 8 * s, 1);
+        mbar_init(bar_km_empty + 8 * s, 1);
+      }
       fence_barrier_init();
       fence_proxy_async_smem();
       mbar_arrive_expect_tx(bar_q_full, 2 * L::kFixBytes);
@@ -410,14 +467,28 @@ bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_consta
   if (warp == 8) {
     if (lane == 0) {
       bool ok = true;
+      auto load_scores = [&](int it) -> bool {  // K-major K and V of step `it`
+        const int s = it % L::kStages, krow = (kt_lo + it) * TO;
+        if (it >= L::kStages && !mbar_wait(bar_sdp_full + 8 * s, (uint32_t)(it / L::kStages - 1) & 1u, guard, kStTfProducer)) return false;
+        const uint32_t dst = sRing + s * 2 * L::kRingBytes;
+        mbar_arrive_expect_tx(bar_ring_full + 8 * s, 2 * L::kRingBytes);
+        tma_tile_f32<D, TO>(dst, &tmKk, bar_ring_full + 8 * s, krow, hk, b);
+        tma_tile_f32<D, TO>(dst + L::kRingBytes, &tmV, bar_ring_full + 8 * s, krow, hk, b);
+        return true;
+      };
+      auto load_acc = [&](int it) -> bool {  // MN-major K of step `it`
+        const int s = it & 1;
+        if (!mbar_wait(bar_km_empty + 8 * s, ((uint32_t)(it / 2) & 1u) ^ 1u, guard, kStTfProducer)) return false;
+        mbar_arrive_expect_tx(bar_km_full + 8 * s, L::kRingBytes);
+        tma_tile_f32<D, TO>(sKm + s * L::kRingBytes, &tmKm, bar_km_full + 8 * s, (kt_lo + it) * TO, hk, b);
+        return true;
+      };
+      for (int it = 0; it < imin(n_it, 2); ++it) load_scores(it);
+      for (int it = 0; it < imin(n_it, 2); ++it) load_acc(it);
+      if (n_it > 2) ok = load_scores(2);
       for (int it = 0; it < n_it && ok; ++it) {
-        const int krow = (kt_lo + it) * TO;
-        ok = mbar_wait(bar_ring_empty, ((uint32_t)it & 1u) ^ 1u, guard, kStTfProducer);
-        if (!ok) break;
-        mbar_arrive_expect_tx(bar_ring_full, 3 * L::kRingBytes);
-        tma_tile_f32<D, TO>(sKk, &tmKk, bar_ring_full, krow, hk, b);
-        tma_tile_f32<D, TO>(sKm, &tmKm, bar_ring_full, krow, hk, b);
-        tma_tile_f32<D, TO>(sVk, &tmV, bar_ring_full, krow, hk, b);
+        if (it + 3 < n_it) ok = load_scores(it + 3);
+        if (ok && it + 2 < n_it) ok = load_acc(it + 2);
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
@@ -431,30 +502,38 @@ bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_consta
       constexpr uint32_t hi_k = desc_hi_sw128(1024);
       constexpr uint32_t hi_m = desc_hi_sw128_base32(512);
       const uint32_t q_lo = desc_lo_sw128(sQ, 16), do_lo = desc_lo_sw128(sdO, 16);
-      const uint32_t kk_lo = desc_lo_sw128(sKk, 16), vk_lo = desc_lo_sw128(sVk, 16);
-      const uint32_t km_lo = desc_lo_sw128(sKm, L::kRingChunkBytes);
       bool ok = mbar_wait(bar_q_full, 0, guard, kStTfMma);
-      for (int it = 0; it < n_it && ok; ++it) {
-        const uint32_t par = (uint32_t)it & 1u;
-        ok = mbar_wait(bar_ring_full, par, guard, kStTfMma);
-        if (!ok) break;
+      auto issue_scores = [&](int it) -> bool {
+        const int s = it % L::kStages;
+        if (!mbar_wait(bar_ring_full + 8 * s, (uint32_t)(it / L::kStages) & 1u, guard, kStTfMma)) return false;
         tc_fence_after();
+        const uint32_t kk_lo = desc_lo_sw128(sRing + s * 2 * L::kRingBytes, 16);
+        const uint32_t vk_lo = desc_lo_sw128(sRing + s * 2 * L::kRingBytes + L::kRingBytes, 16);
 #pragma unroll
         for (int kk = 0; kk < D / 8; ++kk)  // S = Q K^T
-          mma_ss_tf32(tS, q_lo + L::kstep(kk, L::kFixChunkBytes), kk_lo + L::kstep(kk, L::kRingChunkBytes), hi_k, idesc_s,
-                      kk > 0 ? 1u : 0u);
+          mma_ss_tf32(tS + s * TO, q_lo + L::kstep(kk, L::kFixChunkBytes), kk_lo + L::kstep(kk, L::kRingChunkBytes), hi_k,
+                      idesc_s, kk > 0 ? 1u : 0u);
 #pragma unroll
         for (int kk = 0; kk < D / 8; ++kk)  // dP = dO V^T
-          mma_ss_tf32(tdP, do_lo + L::kstep(kk, L::kFixChunkBytes), vk_lo + L::kstep(kk, L::kRingChunkBytes), hi_k, idesc_s,
-                      kk > 0 ? 1u : 0u);
-        mma_commit(bar_sdp_full);
-        ok = mbar_wait(bar_ds_full, par, guard, kStTfMma);
+          mma_ss_tf32(tdP + s * TO, do_lo + L::kstep(kk, L::kFixChunkBytes), vk_lo + L::kstep(kk, L::kRingChunkBytes), hi_k,
+                      idesc_s, kk > 0 ? 1u : 0u);
+        mma_commit(bar_sdp_full + 8 * s);
+        return true;
+      };
+      if (ok) ok = issue_scores(0);
+      for (int it = 0; it < n_it && ok; ++it) {
+        const int s = it & 1;
+        const uint32_t par = (uint32_t)(it / 2) & 1u;
+        if (it + 1 < n_it) ok = issue_scores(it + 1);
+        if (ok) ok = mbar_wait(bar_km_full + 8 * s, par, guard, kStTfMma);
+        if (ok) ok = mbar_wait(bar_ds_full + 8 * s, par, guard, kStTfMma);
         if (!ok) break;
         tc_fence_after();
+        const uint32_t km_lo = desc_lo_sw128(sKm + s * L::kRingBytes, L::kRingChunkBytes);
 #pragma unroll
         for (int kk = 0; kk < TO / 8; ++kk)  // dQ += dS K: 8 keys = 8 columns of dS, 8 rows of K per step
-          mma_ts_tf32(tdQ, tdP + kk * 8, km_lo + kk * 64, hi_m, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(bar_ring_empty);
+          mma_ts_tf32(tdQ, tdP + s * TO + kk * 8, km_lo + kk * 64, hi_m, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(bar_km_empty + 8 * s);
       }
       if (ok) mma_commit(bar_acc_full);
     }
@@ -474,7 +553,7 @@ bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_consta
     }
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
-      const uint32_t par = (uint32_t)it & 1u;
+      const int sb = it % L::kStages;
       const int kt = kt_lo + it;
       const int kg0 = kt * TO + g.k_off;
       const bool full = M::kHasKFullRange && kg0 >= full_lo && kg0 + TO <= full_hi && kg0 + TO <= n &&
@@ -482,35 +561,38 @@ bwd_dq_tf32_kernel(const __grid_constant__ CUtensorMap tmQk, const __grid_consta
       const int klim = imin(n - kg0, g.Lk - kt * TO);
       int w_lo = 0, w_hi = -1;
       if (interval_rows<M>::value && !full && row_ok) row_window<M, true>(qg, kg0, klim, n, g.margs, w_lo, w_hi);
-      ok = mbar_wait(bar_sdp_full, par, guard, kStTfCompute);
+      ok = mbar_wait(bar_sdp_full + 8 * sb, (uint32_t)(it / L::kStages) & 1u, guard, kStTfCompute);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after();
-#pragma unroll
-      for (int part = 0; part < CW / CC; ++part) {
-        const int cb = c0 + part * CC;
-        uint32_t sreg[CC], dpreg[CC];
-        tmem_ld_cols<CC>(tS + lane_sel + cb, sreg);
-        tmem_ld_cols<CC>(tdP + lane_sel + cb, dpreg);
+      {
+        const uint32_t tSb = tS + sb * TO + lane_sel + c0, tdPb = tdP + sb * TO + lane_sel + c0;
+        uint32_t sreg[CW], dpreg[CW];
+        tmem_ld_cols<CW>(tSb, sreg);
+        tmem_ld_cols<CW>(tdPb, dpreg);
         tmem_wait_ld();
+        auto body = [&](auto masked_tag) {
+          constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
-        for (int j = 0; j < CC; ++j) {
-          const int col = cb + j;
-          float pv = ex2(fmaf(__uint_as_float(sreg[j]), c, nlse));
-          bool vis = full;
-          if (!full) {
-            if (interval_rows<M>::value) vis = col >= w_lo && col <= w_hi;
-            else vis = row_ok && col < klim && M::mask(qg, kg0 + col, n, g.margs);
+          for (int j = 0; j < CW; ++j) {
+            const int col = c0 + j;
+            float pv = ex2(fmaf(__uint_as_float(sreg[j]), c, nlse));
+            if (kMasked) {
+              const bool vis = interval_rows<M>::value ? (col >= w_lo && col <= w_hi)
+                                                       : (row_ok && col < klim && M::mask(qg, kg0 + col, n, g.margs));
+              pv = vis ? pv : 0.f;
+            }
+            dpreg[j] = to_tf32(pv * (__uint_as_float(dpreg[j]) + ndelta));
           }
-          pv = vis ? pv : 0.f;
-          dpreg[j] = to_tf32(pv * (__uint_as_float(dpreg[j]) + ndelta));
-        }
-        tmem_st_cols<CC>(tdP + lane_sel + cb, dpreg);  // dS over dP
+        };
+        if (full) body(std::false_type{});
+        else body(std::true_type{});
+        tmem_st_cols<CW>(tdPb, dpreg);  // dS over dP
       }
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_ds_full);
+      if (lane == 0) mbar_arrive(bar_ds_full + 8 * sb);
     }
 
     // ---- epilogue: dQ * sm_scale; warps 0-3 take channels [0, D/2), warps 4-7 the rest

@@ -457,9 +457,9 @@ static void fill_bwd_tc_params(const chill_bwd_args& a, tc::BwdTcParams& p) {
 
 static int bwd_tf32(const chill_bwd_args& a, cudaStream_t st) {
   const chill_shape& s = a.s;
-  // streamed tiles have TO rows (128 at head dim 64, 32 at head dim 128), resident ones 128; "mn" copies (read
+  // streamed tiles have TO rows (64 at head dim 64, 32 at head dim 128: Tf32Shape), resident ones 128; "mn" copies (read
   // MN-major by the tensor core) take the 128-byte swizzle with 32-byte atoms
-  const int to = s.D == 64 ? 128 : 32;
+  const int to = s.D == 64 ? 64 : 32;
   struct MapSpec { const void* p; const int64_t* st; bool kv; int rows; bool mn; };
   const MapSpec spec[11] = {
       {a.q, a.q_strides, false, to, false},   {a.q, a.q_strides, false, to, true},

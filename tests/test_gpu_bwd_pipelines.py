@@ -1,0 +1,48 @@
+"""Pipelined backward kernels at the sizes where a ring, a step or a half tile can go wrong: one to a few steps (so that the
+first round of every ring, the wrap-around and the last step are each reached), ragged ends, several heads per key tile."""
+import pytest
+import torch
+
+from helpers import big_masks, ensure_built, make_inputs, oracle_all
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _lib():
+    ensure_built()
+    from chill_attention import _cabi
+
+    lib = _cabi.load_library()
+    yield lib
+    assert lib.chill_read_device_status() == 0
+
+
+def _gradients(mask, lens, q, k, v, do, precision):
+    import chill_attention as ca
+
+    qd, kd, vd = (t.cuda().requires_grad_(True) for t in (q, k, v))
+    o = ca.chill_attention(qd, kd, vd, mask=mask, lens=lens.cuda(), precision=precision)
+    return torch.autograd.grad(o, (qd, kd, vd), do.cuda())
+
+
+def _check(grads, refs, lens, rtol):
+    for name, g, r in zip(("dq", "dk", "dv"), grads, refs):
+        g = g.cpu().double()
+        assert torch.isfinite(g).all(), name
+        rel = ((g - r).norm() / r.norm()).item()
+        assert rel <= rtol, f"{name} relative error {rel}"
+        for b, n in enumerate(lens.tolist()):
+            assert (g[b, :, n:] == 0).all(), f"{name}: padded rows must be exactly zero"
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("L", [32, 33, 64, 65, 96, 97, 129, 191, 260])
+def test_tf32_steps(D, L):
+    """Steps of 64 (head dim 64) or 32 positions, two stages; tolerance as stated for TF32 (operands lose all but 10 mantissa
+    bits, i.e. 2^-10 relative each, through two GEMMs in a row)."""
+    for mask in (big_masks()[L % 7], big_masks()[(L + 3) % 7]):
+        q, k, v, do = make_inputs(2, 4, 2, L, D, torch.float32, seed=L + D)
+        lens = torch.tensor([L, max(20, L // 3)], dtype=torch.int32)
+        _, _, *refs = oracle_all(mask, q, k, v, do, lens)
+        _check(_gradients(mask, lens, q, k, v, do, "tf32"), refs, lens, 5e-3)
