@@ -13,16 +13,22 @@
 //     P^T = 2^(S^T c - LSE)             -> 16-bit over S^T in TMEM, A operand of  dV += P^T dO
 //     dS^T = P^T (dP^T - delta)         -> 16-bit tile in shared memory [key][query]; read K-major it is the
 //                                          A operand of dK += dS^T Q, read MN-major the A operand of dQ = dS K
-// TMEM (512 columns): S^T | dP^T (re-used for the dQ tile once the compute warps have read dP^T) | dV | dK.
+// TMEM (512 columns): S^T | dP^T (D = 128: re-used for the dQ tile once the compute warps have read dP^T) | dV | dK | D = 64: dQ.
 // Shared memory (D = 128): K, V, two stages of [Q | dO]; the dS^T tile overlays the dO slot of its own stage
-// once dV(u) has consumed dO(u) (no 32 KB are left for a buffer of its own; D = 64 has one).
+// once dV(u) has consumed dO(u) (no 32 KB are left for a buffer of its own; D = 64 has two, and three stages).
 //
 // Tensor-core order in steady state, chosen so that every wait of the issuing thread has been satisfied long
-// before it is reached:
+// before it is reached (D = 128):
 //     dQ(u), dK(u)        need dS^T(u)           | compute warps: exponentials of S^T(u+1)
 //     dP^T(u+1)           needs dQ(u) drained    | drain warps read dQ(u) while dK(u) runs
 //     dV(u+1)             needs P^T(u+1)         | compute warps: dS^T(u+1)
 //     S^T(u+2)
+// At D = 64 the dQ tile has columns of its own, so dP^T(u+1) does not wait for dQ(u) and its drain: it is issued first,
+// and the compute warps go from dS^T(u) to the exponentials of S^T(u+1) to dS^T(u+1) without a pause.
+// Q and dO of a stage complete on barriers of their own, and the compute warps walk heads and tiles without divisions (these
+// took about 500 of the 4400 clocks of a tile).  Together, fp16 (4,16,4096,64) full 905 -> 845 us, bf16 (8,16,4096,128) causal
+// 1281 -> 1266 us.  At D = 128 the period is set by the issuing thread: dQ, dK, the drain of dQ (about 1000 clocks from the
+// commit until the columns are free), dP^T, dV, S^T.
 //
 // Roles (512 threads, register budgets re-balanced per warpgroup with setmaxnreg): warps 0-7 compute (thread
 // (w % 4) * 32 + lane owns key row = TMEM lane; warps 0-3 / 4-7 split the query columns), warps 8-11 drain the
@@ -59,19 +65,20 @@ __device__ __forceinline__ void bulk_wait_read() {
 template <int D>
 struct FusedSmem {
   static constexpr int kTileBytes = kTile * D * 2;
-  static constexpr int kStages = 2;
+  static constexpr bool kOwnDq = (D == 64);  // TMEM columns for the dQ tile and room for two dS^T tiles
+  static constexpr int kStages = kOwnDq ? 3 : 2;
   static constexpr int kDsBytes = kTile * kTile * 2;
-  static constexpr bool kDsOverlay = (kTileBytes >= kDsBytes);  // dS^T lives in the dO slot of its stage
+  static_assert(kOwnDq || kTileBytes >= kDsBytes, "dS^T lives in the dO slot of its stage");
   static constexpr int kK = 0;
   static constexpr int kV = kK + kTileBytes;
   static constexpr int kRing = kV + kTileBytes;  // per stage: [Q | dO]
   static constexpr int kDs = kRing + kStages * 2 * kTileBytes;
-  static constexpr int kRows = kDs + (kDsOverlay ? 0 : kDsBytes);  // per compute warp: -lse[64], -delta[64]
+  static constexpr int kRows = kDs + (kOwnDq ? 2 * kDsBytes : 0);  // per compute warp: -lse[64], -delta[64]
   static constexpr int kDrainChunkBytes = 16 * 32 * 4;  // 16 channels of a drain warp's 32 rows, fp32
   static constexpr int kDrainBufs = 3;
   static constexpr int kDrain = kRows + 8 * 2 * 64 * 4;  // per drain warp: kDrainBufs staging chunks
   static constexpr int kBars = kDrain + 4 * kDrainBufs * kDrainChunkBytes;
-  static constexpr int kNumBars = 9 + 2 * kStages;
+  static constexpr int kNumBars = 8 + 3 * kStages;
   static constexpr int kMisc = kBars + 8 * kNumBars;
   static constexpr int kTotal = kMisc + 16;
   static constexpr int kDynamic = kTotal + 1024;
@@ -127,16 +134,16 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t sK = base + L::kK, sV = base + L::kV, sRing = base + L::kRing;
   float* rows_s = reinterpret_cast<float*>(gen_base + L::kRows);  // [warp][0: -lse, 1: -delta][64]
   const uint32_t bars = base + L::kBars;
-  const uint32_t bar_kv_full = bars, bar_acc_full = bars + 8, bar_s_full = bars + 16, bar_dp_full = bars + 24,
-                 bar_p_full = bars + 32, bar_ds_full = bars + 40, bar_dv_done = bars + 48, bar_dq_full = bars + 56,
-                 bar_dq_drained = bars + 64;
-  const uint32_t bar_ring_full = bars + 72, bar_ring_empty = bar_ring_full + 8 * L::kStages;
+  const uint32_t bar_acc_full = bars, bar_s_full = bars + 8, bar_dp_full = bars + 16, bar_p_full = bars + 24,
+                 bar_ds_full = bars + 32, bar_dv_done = bars + 40, bar_dq_full = bars + 48, bar_dq_drained = bars + 56;
+  // Q and dO of a stage complete separately (K with the first Q, V with the first dO): S^T does not wait for dO
+  const uint32_t bar_q_full = bars + 64, bar_do_full = bar_q_full + 8 * L::kStages, bar_ring_empty = bar_do_full + 8 * L::kStages;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen_base + L::kMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_base + L::kMisc + 4);
   const Guard guard{p.status, abort_flag};
   // byte offset (from the aligned base) of the dS^T tile that belongs to iteration `it`
   auto ds_offset = [&](int it) -> int {
-    return L::kDsOverlay ? L::kRing + (it % L::kStages) * 2 * L::kTileBytes + L::kTileBytes : L::kDs;
+    return L::kOwnDq ? L::kDs + (it & 1) * L::kDsBytes : L::kRing + (it % L::kStages) * 2 * L::kTileBytes + L::kTileBytes;
   };
 
   if (warp == 12) {
@@ -144,7 +151,6 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // before the CTA-wide set-up (TMEM allocation, __syncthreads) completes.
     if (lane == 0) {
       *abort_flag = 0;
-      mbar_init(bar_kv_full, 1);
       mbar_init(bar_acc_full, 1);
       mbar_init(bar_s_full, 1);
       mbar_init(bar_dp_full, 1);
@@ -154,20 +160,21 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(bar_dq_full, 1);
       mbar_init(bar_dq_drained, 4);
       for (int s = 0; s < L::kStages; ++s) {
-        mbar_init(bar_ring_full + 8 * s, 1);
+        mbar_init(bar_q_full + 8 * s, 1);
+        mbar_init(bar_do_full + 8 * s, 1);
         mbar_init(bar_ring_empty + 8 * s, 1);
       }
       fence_barrier_init();
       fence_proxy_async_smem();
-      mbar_arrive_expect_tx(bar_kv_full, 2 * L::kTileBytes);
+      mbar_arrive_expect_tx(bar_q_full, 2 * L::kTileBytes);
       for (int c = 0; c < kChunks; ++c) {
-        tma_load_4d(sK + c * kChunkBytes, &tmK, bar_kv_full, c * 64, kb, hk, b);
-        tma_load_4d(sV + c * kChunkBytes, &tmV, bar_kv_full, c * 64, kb, hk, b);
+        tma_load_4d(sK + c * kChunkBytes, &tmK, bar_q_full, c * 64, kb, hk, b);
+        tma_load_4d(sRing + c * kChunkBytes, &tmQ, bar_q_full, c * 64, qt_lo * kTile, hk * G, b);
       }
-      mbar_arrive_expect_tx(bar_ring_full, 2 * L::kTileBytes);
+      mbar_arrive_expect_tx(bar_do_full, 2 * L::kTileBytes);
       for (int c = 0; c < kChunks; ++c) {
-        tma_load_4d(sRing + c * kChunkBytes, &tmQ, bar_ring_full, c * 64, qt_lo * kTile, hk * G, b);
-        tma_load_4d(sRing + L::kTileBytes + c * kChunkBytes, &tmdO, bar_ring_full, c * 64, qt_lo * kTile, hk * G, b);
+        tma_load_4d(sV + c * kChunkBytes, &tmV, bar_do_full, c * 64, kb, hk, b);
+        tma_load_4d(sRing + L::kTileBytes + c * kChunkBytes, &tmdO, bar_do_full, c * 64, qt_lo * kTile, hk * G, b);
       }
     }
     __syncwarp();
@@ -178,7 +185,7 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tSt = tmem, tdPt = tmem + 128, tdQ = tmem + 128, tdV = tmem + 256, tdK = tmem + 384;
+  const uint32_t tSt = tmem, tdPt = tmem + 128, tdQ = tmem + (L::kOwnDq ? 256 + 2 * D : 128), tdV = tmem + 256, tdK = tmem + 256 + D;
 
   if (warp >= 12) {
     reg_dealloc<kFusedOtherRegs>();
@@ -193,12 +200,12 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int qrow = (qt_lo + it % n_qt) * kTile;
           ok = mbar_wait(bar_ring_empty + 8 * s, ph ^ 1u, guard, kStFusProducer);
           if (!ok) break;
-          mbar_arrive_expect_tx(bar_ring_full + 8 * s, 2 * L::kTileBytes);
           const uint32_t dst = sRing + s * 2 * L::kTileBytes;
-          for (int c = 0; c < kChunks; ++c) {
-            tma_load_4d(dst + c * kChunkBytes, &tmQ, bar_ring_full + 8 * s, c * 64, qrow, h, b);
-            tma_load_4d(dst + L::kTileBytes + c * kChunkBytes, &tmdO, bar_ring_full + 8 * s, c * 64, qrow, h, b);
-          }
+          mbar_arrive_expect_tx(bar_q_full + 8 * s, L::kTileBytes);
+          for (int c = 0; c < kChunks; ++c) tma_load_4d(dst + c * kChunkBytes, &tmQ, bar_q_full + 8 * s, c * 64, qrow, h, b);
+          mbar_arrive_expect_tx(bar_do_full + 8 * s, L::kTileBytes);
+          for (int c = 0; c < kChunks; ++c)
+            tma_load_4d(dst + L::kTileBytes + c * kChunkBytes, &tmdO, bar_do_full + 8 * s, c * 64, qrow, h, b);
         }
         if (!ok) {
           const uint64_t t0 = globaltimer_ns();
@@ -214,11 +221,11 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         constexpr uint32_t hi_k = desc_hi_sw128(1024);
         const uint32_t k_lo = desc_lo_sw128(sK, 16), v_lo = desc_lo_sw128(sV, 16);
         const uint32_t kmn_lo = desc_lo_sw128(sK, kChunkBytes);
-        bool ok = mbar_wait(bar_kv_full, 0, guard, kStFusMma);
+        bool ok = true;
         auto stage_q = [&](int it) { return sRing + (it % L::kStages) * 2 * L::kTileBytes; };
         auto issue_s = [&](int it) -> bool {  // S^T(it) = K Q^T; first user of ring stage `it`
           const int s = it % L::kStages;
-          if (!mbar_wait(bar_ring_full + 8 * s, (uint32_t)(it / L::kStages) & 1u, guard, kStFusMma)) return false;
+          if (!mbar_wait(bar_q_full + 8 * s, (uint32_t)(it / L::kStages) & 1u, guard, kStFusMma)) return false;
           tc_fence_after();
           const uint32_t q_lo = desc_lo_sw128(stage_q(it), 16);
 #pragma unroll
@@ -227,12 +234,15 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           mma_commit(bar_s_full);
           return true;
         };
-        auto issue_dp = [&](int it) {  // dP^T(it) = V dO^T
+        auto issue_dp = [&](int it) -> bool {  // dP^T(it) = V dO^T
+          if (!mbar_wait(bar_do_full + 8 * (it % L::kStages), (uint32_t)(it / L::kStages) & 1u, guard, kStFusMma)) return false;
+          tc_fence_after();
           const uint32_t do_lo = desc_lo_sw128(stage_q(it) + L::kTileBytes, 16);
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk)
             mma_ss_lh(tdPt, v_lo + kmajor_step(kk), do_lo + kmajor_step(kk), hi_k, idesc_s, kk > 0);
           mma_commit(bar_dp_full);
+          return true;
         };
         auto issue_dv = [&](int it) -> bool {  // dV += P^T(it) dO(it)   (16 queries per step)
           if (!mbar_wait(bar_p_full, (uint32_t)it & 1u, guard, kStFusMma)) return false;
@@ -245,7 +255,7 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           return true;
         };
         if (ok) ok = issue_s(0);
-        if (ok) issue_dp(0);
+        if (ok) ok = issue_dp(0);
         if (ok) ok = issue_dv(0);
         if (ok && n_it > 1) ok = issue_s(1);  // overwrites P^T(0) only after dV(0) has read it (MMAs complete in order)
         for (int it = 0; it < n_it && ok; ++it) {
@@ -256,8 +266,15 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           ok = mbar_wait(bar_ds_full, par, guard, kStFusMma);
           if (!ok) break;
           tc_fence_after();
+          if (L::kOwnDq) {
+            // dS^T(it + 1) goes to the tile that dQ and dK(it - 1) read: they were issued before this dP^T
+            if (it + 1 < n_it) ok = issue_dp(it + 1);
+            if (ok && it > 0) ok = mbar_wait(bar_dq_drained, par ^ 1u, guard, kStFusMma);  // the drain warps hold dQ(it - 1) in registers
+            if (!ok) break;
+            tc_fence_after();
+          }
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk)  // dQ tile = dS K   (16 keys per step; overwrites dP^T(it))
+          for (int kk = 0; kk < kTile / 16; ++kk)  // dQ tile = dS K   (16 keys per step; D = 128: overwrites dP^T(it))
             mma_ss_lh(tdQ, dsmn_lo + kk * 128, kmn_lo + kk * 128, hi_k, idesc_dq, kk > 0);
           mma_commit(bar_dq_full);
 #pragma unroll
@@ -265,10 +282,13 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             mma_ss_lh(tdK, dsk_lo + kmajor_step(kk), qmn_lo + kk * 128, hi_k, idesc_acc, (it > 0 || kk > 0));
           mma_commit(bar_ring_empty + 8 * (it % L::kStages));
           if (it + 1 < n_it) {
-            ok = mbar_wait(bar_dq_drained, par, guard, kStFusMma);  // the drain warps hold dQ(it) in registers
-            if (!ok) break;
-            tc_fence_after();
-            issue_dp(it + 1);
+            if (!L::kOwnDq) {
+              ok = mbar_wait(bar_dq_drained, par, guard, kStFusMma);  // the drain warps hold dQ(it) in registers
+              if (!ok) break;
+              tc_fence_after();
+              ok = issue_dp(it + 1);
+              if (!ok) break;
+            }
             ok = issue_dv(it + 1);
             if (ok && it + 2 < n_it) ok = issue_s(it + 2);
           }
@@ -339,26 +359,31 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int t = threadIdx.x;  // 0..255
     float* slot = rows_s + warp * 128;  // warp-private: [0,64) -LSE, [64,128) -delta of this warp's columns
     bool ok = true;
-    // LSE / delta of this lane's two query columns of tile `it`, fetched one tile ahead.  The loaded values are
-    // not touched until the next iteration (any dependent instruction here would stall on the global load).
-    auto fetch_rows = [&](int it, float* lv, float* dl) {
-      const int h = hk * G + it / n_qt;
+    // LSE / delta of this lane's two query columns, fetched one tile ahead (tile qi_next of head h_next).  The loaded
+    // values are not touched until the next iteration (any dependent instruction here would stall on the global load).
+    // The walk over heads and tiles is incremental: the divisions it replaces took 500 of a tile's ~4400 clocks.
+    int h_next = hk * G, qi_next = qt_lo;
+    float nl_next[2], nd_next[2];
+    auto fetch_rows = [&]() {
+      const float* lse_h = p.lse + b * p.lse_sb + h_next * p.lse_sh;
+      const float* delta_h = p.delta + ((long long)b * g.H + h_next) * g.Lq;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int qrow = (qt_lo + it % n_qt) * kTile + c0 + e * 32 + lane;
-        const bool in = qrow < g.Lq;
-        const float* pl = p.lse + b * p.lse_sb + h * p.lse_sh + (in ? qrow : 0) * p.lse_sl;
-        const float* pd = p.delta + ((long long)b * g.H + h) * g.Lq + (in ? qrow : 0);
-        lv[e] = __ldg(pl);  // row 0 stands in for rows beyond Lq: those columns are masked out anyway
-        dl[e] = __ldg(pd);
+        const int qrow = qi_next * kTile + c0 + e * 32 + lane;
+        const int row = qrow < g.Lq ? qrow : 0;  // row 0 stands in for rows beyond Lq: those columns are masked out anyway
+        nl_next[e] = __ldg(lse_h + row * p.lse_sl);
+        nd_next[e] = __ldg(delta_h + row);
       }
     };
-    float nl_next[2], nd_next[2];
-    fetch_rows(0, nl_next, nd_next);
+    fetch_rows();
     for (int it = 0; it < n_it; ++it) {
       const uint32_t par = (uint32_t)it & 1u;
-      const int qi = qt_lo + it % n_qt;
+      const int qi = qi_next;
       const int qg0 = qi * kTile + g.q_off;
+      if (++qi_next == qt_hi) {
+        qi_next = qt_lo;
+        ++h_next;
+      }
       __syncwarp();
 #pragma unroll
       for (int e = 0; e < 2; ++e) {  // negated: they enter the packed FMA / ADD as addends
@@ -366,7 +391,7 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         slot[64 + e * 32 + lane] = -nd_next[e];
       }
       __syncwarp();
-      if (it + 1 < n_it) fetch_rows(it + 1, nl_next, nd_next);
+      if (it + 1 < n_it) fetch_rows();
       const bool full = M::kHasQFullRange && qg0 >= full_lo && qg0 + kTile <= full_hi && qg0 + kTile <= n &&
                         qi * kTile + kTile <= g.Lq && kg0 + kTile <= n && kb + kTile <= g.Lk;
       const int qlim = imin(n - qg0, g.Lq - qi * kTile);
@@ -444,7 +469,7 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
       }
       tc_fence_before();  // orders this warp's dP^T reads before the dQ GEMM that re-uses the columns
-      if (L::kDsOverlay) {
+      if (!L::kOwnDq) {
         // dS^T goes where dO(it) sits: wait until the dV GEMM has read it
         ok = mbar_wait(bar_dv_done, par, guard, kStFusCompute);
         ok = __all_sync(0xffffffffu, ok);

@@ -3,7 +3,7 @@ first round of every ring, the wrap-around and the last step are each reached), 
 import pytest
 import torch
 
-from helpers import big_masks, ensure_built, make_inputs, oracle_all
+from helpers import G_RTOL, big_masks, ensure_built, make_inputs, oracle_all
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +46,14 @@ def test_tf32_steps(D, L):
         lens = torch.tensor([L, max(20, L // 3)], dtype=torch.int32)
         _, _, *refs = oracle_all(mask, q, k, v, do, lens)
         _check(_gradients(mask, lens, q, k, v, do, "tf32"), refs, lens, 5e-3)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=str)
+@pytest.mark.parametrize("L", [2, 127, 128, 129, 257, 385, 513])
+def test_head_dim_64_tiles(L, dtype):
+    """1 to 10 query tiles per key tile (a ring of three stages, two dS tiles, dQ columns of their own), ragged ends."""
+    for mask in (big_masks()[L % 7], big_masks()[(L + 2) % 7]):
+        q, k, v, do = make_inputs(2, 4, 2, L, 64, dtype, seed=L)
+        lens = torch.tensor([L, max(2, L // 3)], dtype=torch.int32)
+        _, _, *refs = oracle_all(mask, q, k, v, do, lens)
+        _check(_gradients(mask, lens, q, k, v, do, "ieee"), refs, lens, G_RTOL[dtype])
