@@ -1,5 +1,5 @@
 // Backward attention in ONE kernel with five GEMMs per (query tile, key tile) pair (sm_100a, 16-bit inputs,
-// head dim 64 or 128).  The two-kernel backward in bwd_tc.cuh computes S and dP twice (seven GEMMs) so that
+// head dim 64 or 128; bwd_fused64.cuh is a form for head dim 64 and few query tiles per key tile).  The two-kernel backward in bwd_tc.cuh computes S and dP twice (seven GEMMs) so that
 // no accumulation crosses CTAs; here a CTA owns a tile of 128 keys, keeps dK and dV in TMEM as that kernel
 // does, and additionally forms the partial product dQ_tile = dS K for every query tile it visits.  The partial
 // products of the CTAs that share a query tile are summed in an fp32 accumulator in global memory with bulk
@@ -545,41 +545,6 @@ dq_convert_kernel(const float* __restrict__ accum, T* __restrict__ dq, long long
       *reinterpret_cast<uint2*>(dst + (r0 + 1) * sl + c4 * 4) =
           make_uint2(pack2<T>(bb.x * scale, bb.y * scale), pack2<T>(bb.z * scale, bb.w * scale));
   }
-}
-
-// ---------------------------------------------------------------------------- launcher
-template <typename T, int D, class M>
-int launch_bwd_fused_one(const CUtensorMap* maps, const BwdTcParams& p, cudaStream_t st) {
-  auto kern = bwd_fused_tc_kernel<T, D, M>;
-  constexpr int smem = FusedSmem<D>::kDynamic;
-  static_assert(smem <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
-  struct Tag {};
-  cudaError_t e = ensure_dynamic_smem<Tag>(kern, smem);
-  if (e != cudaSuccess) return (int)e;
-  const Geo& g = p.g;
-  e = cudaMemsetAsync(p.dq_accum, 0, dq_accum_bytes(g.B, g.H, g.Lq, D), st);
-  if (e != cudaSuccess) return (int)e;
-  // maps: 0 Q, 1 K, 2 V, 3 dO, 4 dQ, 5 dK, 6 dV
-  dim3 gk((unsigned)(((g.Lk + kTile - 1) / kTile) * g.Hkv * g.B), 1, 1);
-  kern<<<gk, kFusedThreads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], maps[5], maps[6], p);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return (int)e;
-  dim3 gc((unsigned)((g.Lq + kTile - 1) / kTile), (unsigned)g.H, (unsigned)g.B);
-  dq_convert_kernel<T, D><<<gc, 256, 0, st>>>(p.dq_accum, reinterpret_cast<T*>(p.dq), p.dq_sb, p.dq_sh, p.dq_sl, g.H,
-                                               g.Lq, g.D, g.scale);
-  return (int)cudaGetLastError();
-}
-
-template <class M>
-int launch_bwd_fused_all(int dtype, int D, const CUtensorMap* maps, const BwdTcParams& p, cudaStream_t st) {
-  if (dtype == 2) {
-    if (D == 128) return launch_bwd_fused_one<__nv_bfloat16, 128, M>(maps, p, st);
-    if (D == 64) return launch_bwd_fused_one<__nv_bfloat16, 64, M>(maps, p, st);
-  } else if (dtype == 1) {
-    if (D == 128) return launch_bwd_fused_one<__half, 128, M>(maps, p, st);
-    if (D == 64) return launch_bwd_fused_one<__half, 64, M>(maps, p, st);
-  }
-  return (int)cudaErrorInvalidValue;
 }
 
 }  // namespace tc

@@ -35,6 +35,7 @@ constexpr int kBwdThreads = 320;
 constexpr int kBwdComputeThreads = 256;
 constexpr int kTmemColsBwd = 512;
 constexpr bool kHaveBwdTc = true;
+constexpr int kF64Step = 64;   // head dim 64, short loops (bwd_fused64.cuh): queries per step = rows of its Q / dO boxes
 constexpr int kWideCols = 64;  // head dim 256 (bwd_wide.cuh): positions of the streamed axis per step = rows of its TMA boxes
 
 struct BwdTcParams {
@@ -47,6 +48,7 @@ struct BwdTcParams {
   int* status;
   int which;  // bit0: launch the dK/dV kernel, bit1: launch the dQ kernel
   float* dq_accum;  // fp32 accumulator of the single-kernel backward (bwd_fused.cuh), else nullptr
+  bool short_loops;  // bwd_fused64.cuh instead of bwd_fused.cuh
   PartOut part;     // optional un-rounded fp32 copies of dK / dV rows
 };
 

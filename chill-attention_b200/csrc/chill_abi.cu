@@ -452,6 +452,7 @@ static void fill_bwd_tc_params(const chill_bwd_args& a, tc::BwdTcParams& p) {
   p.dv_sb = a.dv_strides[0]; p.dv_sh = a.dv_strides[1]; p.dv_sl = a.dv_strides[2];
   p.which = bwd_which(s.flags);
   p.dq_accum = nullptr;
+  p.short_loops = false;
   p.part = to_part(a);
 }
 
@@ -490,17 +491,21 @@ static int bwd_tc(const chill_bwd_args& a, cudaStream_t st, bool concurrent = tr
   const void* ptrs[7] = {a.q, a.k, a.v, a.d_o, a.dq, a.dk, a.dv};
   const int64_t* strs[7] = {a.q_strides, a.k_strides, a.v_strides, a.do_strides, a.dq_strides, a.dk_strides, a.dv_strides};
   const bool is_kv[7] = {false, true, true, false, false, true, true};
-  for (int i = 0; i < 7; ++i) {
-    int rc = make_map(&maps[i], ptrs[i], strs[i], s.B, is_kv[i] ? s.H_kv : s.H, is_kv[i] ? s.Lk : s.Lq, s.D, s.dtype,
-                      tc::kTile);
-    if (rc != CHILL_OK) return rc;
-  }
   tc::BwdTcParams p;
   fill_bwd_tc_params(a, p);
+  const bool single = fused && p.which == 3 && a.dq_accum != nullptr;
+  if (single) {
+    CHILL_MASK_SWITCH(s.mask.id, (p.short_loops = tc_bwd_short_loops<MaskT>(p.g, s.D)))
+  }
+  for (int i = 0; i < 7; ++i) {
+    const int rows = p.short_loops && (i == 0 || i == 3) ? tc::kF64Step : tc::kTile;
+    int rc = make_map(&maps[i], ptrs[i], strs[i], s.B, is_kv[i] ? s.H_kv : s.H, is_kv[i] ? s.Lk : s.Lq, s.D, s.dtype, rows);
+    if (rc != CHILL_OK) return rc;
+  }
   p.status = device_status_ptr();
   if (p.status == nullptr) return cuda_fail(cudaGetLastError(), "status symbol");
   int e = 0;
-  if (fused && p.which == 3 && a.dq_accum != nullptr) {
+  if (single) {
     if ((reinterpret_cast<uintptr_t>(a.dq_accum) & 15u) != 0) return CHILL_E_INVALID;
     p.dq_accum = a.dq_accum;  // single-kernel backward + conversion of the fp32 dQ sums
     CHILL_MASK_SWITCH(s.mask.id, (e = tc_launch_bwd<MaskT>(s.dtype, tc_width(s), maps, p, st)))

@@ -1,6 +1,6 @@
 // Instantiates the tensor-core kernels for ONE mask functor: compile with
 //   -DCHILL_INST_MASK=<functor struct>   (e.g. CausalMask)
-#include "bwd_fused.cuh"
+#include "bwd_fused64.cuh"
 #include "bwd_tc.cuh"
 #include "bwd_tf32.cuh"
 #include "bwd_wide.cuh"
@@ -72,6 +72,11 @@ template <>
 int tc_launch_bwd<InstMask>(int dtype, int D, const CUtensorMap* maps, const tc::BwdTcParams& p, cudaStream_t st) {
   if (p.dq_accum != nullptr) return tc::launch_bwd_fused_all<InstMask>(dtype, D, maps, p, st);
   return tc::launch_bwd_all<InstMask>(dtype, D, maps, p, st);
+}
+
+template <>
+bool tc_bwd_short_loops<InstMask>(const Geo& g, int D) {
+  return tc::bwd_short_loops<InstMask>(g, D);
 }
 
 template <>

@@ -69,6 +69,10 @@ int tc_launch_fwd_tf32(int D, const CUtensorMap* maps, const tc::FwdTcParams& p,
 template <class M>
 int tc_launch_bwd(int dtype, int D, const CUtensorMap* maps, const tc::BwdTcParams& p, cudaStream_t st);
 
+// Which form of the single-kernel backward serves a call of head dim <= 64: bwd_fused64.cuh (true) or bwd_fused.cuh.
+template <class M>
+bool tc_bwd_short_loops(const Geo& g, int D);
+
 // 16-bit head dim 256 (bwd_wide.cuh, three launches); maps: Q, K, V, dO with 128-row boxes, the same four with 64-row
 // boxes, dQ, dK, dV.
 template <class M>

@@ -57,3 +57,19 @@ def test_head_dim_64_tiles(L, dtype):
         lens = torch.tensor([L, max(2, L // 3)], dtype=torch.int32)
         _, _, *refs = oracle_all(mask, q, k, v, do, lens)
         _check(_gradients(mask, lens, q, k, v, do, "ieee"), refs, lens, G_RTOL[dtype])
+
+
+@pytest.mark.parametrize("kind", ["window", "one_sided", "chunkwise", "off_grid_chunks", "full", "causal"])
+def test_head_dim_64_short_loops(kind):
+    """Enough key tiles and few enough query tiles for the form with two CTAs per SM (steps of 64 queries, two to a dQ tile):
+    first or last half of a query tile missing, ragged last step, rows of padding only, one or two heads per key head."""
+    import chill_attention as ca
+
+    mask = {"window": ca.SlidingWindowChillMask(40, 5), "one_sided": ca.SlidingWindowChillMask(0, 70), "chunkwise": ca.ChunkwiseChillMask(64, 1),
+            "off_grid_chunks": ca.ChunkwiseChillMask(48, 0), "full": ca.FullChillMask(), "causal": ca.CausalChillMask()}[kind]
+    L, dtype = (200, torch.bfloat16) if kind in ("full", "causal") else (330, torch.float16)
+    heads = 30 if kind in ("window", "off_grid_chunks") else 60  # these see three query tiles per key tile, the others two
+    q, k, v, do = make_inputs(5, heads, 30, L, 64, dtype, seed=7)
+    lens = torch.tensor([L, L - 1, 129, 64, 2], dtype=torch.int32)
+    _, _, *refs = oracle_all(mask, q, k, v, do, lens)
+    _check(_gradients(mask, lens, q, k, v, do, "ieee"), refs, lens, G_RTOL[dtype])
