@@ -73,3 +73,39 @@ def test_head_dim_64_short_loops(kind):
     lens = torch.tensor([L, L - 1, 129, 64, 2], dtype=torch.int32)
     _, _, *refs = oracle_all(mask, q, k, v, do, lens)
     _check(_gradients(mask, lens, q, k, v, do, "ieee"), refs, lens, G_RTOL[dtype])
+
+
+def test_head_dim_64_short_loops_of_a_shard(_lib):
+    """The same form for a shard: queries [q0, L) against keys [k0, L) (neither on a tile boundary), with the un-rounded fp32
+    copies of the first and last dK / dV rows, which must round to the 16-bit outputs."""
+    import ctypes as C
+
+    import chill_attention as ca
+    from chill_attention import _cabi
+
+    L, q0, k0, H, D, dtype, head, tail = 330, 100, 20, 100, 64, torch.float16, 40, 30
+    mask = ca.SlidingWindowChillMask(40, 5)
+    q, k, v, do = make_inputs(1, H, H, L, D, dtype, seed=9)
+    _, _, dq_ref, dk_ref, dv_ref = oracle_all(mask, q, k, v, do)
+    qs, dos = (t[:, :, q0:].contiguous().cuda() for t in (q, do))
+    ks, vs = (t[:, :, k0:].contiguous().cuda() for t in (k, v))
+    shape = _cabi.make_shape(qs, ks, _cabi.BUILTIN_FUNCTOR_IDS[mask.cuda_functor], mask.constargs, None, D ** -0.5,
+                             q_offset=q0, k_offset=k0, seq_len=L)
+    o, lse = torch.empty_like(qs), torch.empty(1, H, L - q0, dtype=torch.float32, device="cuda")
+    _cabi.forward(_lib, qs, ks, vs, o, lse, shape)
+    delta = torch.empty_like(lse)
+    accum = torch.empty(_lib.chill_bwd_dq_accum_bytes(C.byref(shape)) // 4, dtype=torch.float32, device="cuda")
+    part = [torch.full((1, H, head + tail, D), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2)]
+    g = [torch.full_like(t, float("nan")) for t in (qs, ks, vs)]
+    a = _cabi.backward_args(qs, ks, vs, o, dos, lse, delta, *g, shape, accum, part=(part[0], part[1], head, tail))
+    _cabi.check(_lib, _lib.chill_bwd_delta(C.byref(a), _cabi._stream()), "chill_bwd_delta")
+    _cabi.check(_lib, _lib.chill_bwd(C.byref(a), _cabi._stream()), "chill_bwd")
+    torch.cuda.synchronize()
+    own = q0 + 5 - k0  # keys from here on are seen by queries of this shard only
+    for name, got, ref in (("dq", g[0], dq_ref[:, :, q0:]), ("dk", g[1][:, :, own:], dk_ref[:, :, own + k0:]),
+                           ("dv", g[2][:, :, own:], dv_ref[:, :, own + k0:])):
+        got = got.cpu().double()
+        assert torch.isfinite(got).all(), name
+        assert ((got - ref).norm() / ref.norm()).item() <= G_RTOL[dtype], name
+    for p, out in zip(part, g[1:]):
+        assert torch.equal(p.to(dtype), torch.cat([out[:, :, :head], out[:, :, out.shape[2] - tail:]], dim=2))
