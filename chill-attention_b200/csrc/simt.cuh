@@ -63,13 +63,15 @@ __device__ __forceinline__ void store_elem(void* p, long long i, int dtype, floa
 __device__ __forceinline__ int swz(int row) { return (row >> 2) & 7; }
 
 // One tile of ROWS x DP elements, starting at row `row0` of head h of batch row b, to shared memory as fp32; rows beyond
-// rows_in and channels beyond D become zeros.
+// rows_in (what does not exist or is padding: it may hold anything) and channels beyond D become zeros.  Returns whether
+// one of the elements this thread loaded is NaN or infinite (see accumulate).
 template <int DP, int ROWS>
-__device__ __forceinline__ void load_tile(float* s, const TRef& t, int b, int h, int row0, int rows_in, int D, int dtype, bool vec) {
+__device__ __forceinline__ bool load_tile(float* s, const TRef& t, int b, int h, int row0, int rows_in, int D, int dtype, bool vec) {
   constexpr int kChunks = DP / 4, kPerThread = ROWS * kChunks / kThreads;
   static_assert(ROWS * kChunks % kThreads == 0, "every thread moves the same number of chunks");
   constexpr int kBatch = kPerThread < 8 ? kPerThread : 8;  // loads in flight per thread
   const long long origin = b * t.sb + h * t.sh + row0 * t.sl;
+  uint64_t probe = 0ull;  // both halves stay zero while everything is finite: x * 0 is NaN otherwise
 #pragma unroll 1
   for (int i0 = 0; i0 < kPerThread; i0 += kBatch) {
     float4 v[kBatch];
@@ -89,6 +91,7 @@ __device__ __forceinline__ void load_tile(float* s, const TRef& t, int b, int h,
         float e[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) e[k] = (row < rows_in && c * 4 + k < D) ? load_elem(t.p, origin + row * t.sl + (c * 4 + k) * t.sd, dtype) : 0.f;
+        probe = tc::ffma2(tc::pk2(e[0], e[1]), 0ull, tc::ffma2(tc::pk2(e[2], e[3]), 0ull, probe));
         *reinterpret_cast<float4*>(s + row * DP + 4 * (c ^ swz(row))) = make_float4(e[0], e[1], e[2], e[3]);
       }
       continue;
@@ -97,9 +100,13 @@ __device__ __forceinline__ void load_tile(float* s, const TRef& t, int b, int h,
     for (int i = 0; i < kBatch; ++i) {
       const int idx = (i0 + i) * kThreads + threadIdx.x;
       const int row = idx / kChunks, c = idx % kChunks;
+      probe = tc::ffma2(tc::pk2(v[i].x, v[i].y), 0ull, tc::ffma2(tc::pk2(v[i].z, v[i].w), 0ull, probe));
       *reinterpret_cast<float4*>(s + row * DP + 4 * (c ^ swz(row))) = v[i];
     }
   }
+  float lo, hi;
+  tc::upk2(probe, lo, hi);
+  return !(lo == 0.f && hi == 0.f);
 }
 
 // s[i][j] = sum over channels of A[row0 + i][.] * B[4 * l16 + j][.]
@@ -145,10 +152,48 @@ struct Lane {
   static constexpr int kPairs = DP / 32;
 };
 
+// The channels of one lane in row `row` of the streamed tile X (fx = swz(row)).
+template <int DP>
+__device__ __forceinline__ void lane_channels(const float* X, int row, int fx, int l16, uint64_t (&x)[Lane<DP>::kPairs]) {
+  const float* xr = X + row * DP;
+  if constexpr (DP == 32) {
+    x[0] = *reinterpret_cast<const uint64_t*>(xr + 4 * ((l16 >> 1) ^ fx) + 2 * (l16 & 1));
+  } else {
+#pragma unroll
+    for (int c = 0; c < DP / 64; ++c) {
+      const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(xr + 4 * ((l16 + 16 * c) ^ fx));
+      x[2 * c] = v.x;
+      x[2 * c + 1] = v.y;
+    }
+  }
+}
+
+// Weight of a pair that the row may not see, where that has to be told apart from a probability that has underflowed.
+constexpr uint32_t kHidden = 0x80000000u;  // -0.0f: adds nothing, and 2^x is never it
+
 // acc[i][.] += sum over the 64 streamed positions of W[row0 + i][.] * X[.][channels of this lane]
-template <int DP, int RT>
-__device__ __forceinline__ void accumulate(const float* W, const float* X, int row0, int l16, uint64_t (&acc)[RT][Lane<DP>::kPairs]) {
+//
+// A hidden pair must add nothing, but 0 * NaN and 0 * Inf are NaN.  So tiles of X with such an element (`finite` false, the
+// same for the whole CTA) take a loop that leaves pairs out: every zero weight, or with kKeepZeros only the kHidden ones.
+template <int DP, int RT, bool kKeepZeros = false>
+__device__ __forceinline__ void accumulate(const float* W, const float* X, int row0, int l16, uint64_t (&acc)[RT][Lane<DP>::kPairs], bool finite) {
   const int fa = swz(row0);
+  if (!finite) {
+#pragma unroll 1
+    for (int kx = 0; kx < kCols; ++kx) {
+      uint64_t x[Lane<DP>::kPairs];
+      lane_channels<DP>(X, kx, swz(kx), l16, x);
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        const float wk = W[(row0 + i) * kCols + 4 * ((kx >> 2) ^ (fa + (i >> 2))) + (kx & 3)];
+        if (kKeepZeros ? __float_as_uint(wk) == kHidden : wk == 0.f) continue;
+        const uint64_t w2 = tc::pk2(wk, wk);
+#pragma unroll
+        for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) acc[i][pidx] = tc::ffma2(w2, x[pidx], acc[i][pidx]);
+      }
+    }
+    return;
+  }
 #pragma unroll 2
   for (int k4 = 0; k4 < kCols / 4; ++k4) {
     float4 w[RT];
@@ -157,18 +202,8 @@ __device__ __forceinline__ void accumulate(const float* W, const float* X, int r
     const int fx = k4 & 7;  // swz of positions 4 * k4 .. 4 * k4 + 3
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) {
-      const float* xr = X + (4 * k4 + kk) * DP;
       uint64_t x[Lane<DP>::kPairs];
-      if constexpr (DP == 32) {
-        x[0] = *reinterpret_cast<const uint64_t*>(xr + 4 * ((l16 >> 1) ^ fx) + 2 * (l16 & 1));
-      } else {
-#pragma unroll
-        for (int c = 0; c < DP / 64; ++c) {
-          const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(xr + 4 * ((l16 + 16 * c) ^ fx));
-          x[2 * c] = v.x;
-          x[2 * c + 1] = v.y;
-        }
-      }
+      lane_channels<DP>(X, 4 * k4 + kk, fx, l16, x);
 #pragma unroll
       for (int i = 0; i < RT; ++i) {
         const float wk = kk == 0 ? w[i].x : (kk == 1 ? w[i].y : (kk == 2 ? w[i].z : w[i].w));
@@ -185,15 +220,15 @@ __device__ __forceinline__ int pair_channel(int l16, int pidx) {
   return DP == 32 ? 2 * l16 : 4 * (l16 + 16 * (pidx >> 1)) + 2 * (pidx & 1);
 }
 
-// One row of accumulators, times `mul`, to element offset `off` of tensor p.
+// One row of accumulators, times `mul`, to element offset `off` of tensor p; a row of padding (`valid` false) is zero.
 template <int DP>
-__device__ __forceinline__ void store_row(void* p, long long off, long long sd, int D, int dtype, bool vec, int l16, const uint64_t* acc, float mul) {
+__device__ __forceinline__ void store_row(void* p, long long off, long long sd, int D, int dtype, bool vec, int l16, const uint64_t* acc, float mul, bool valid) {
 #pragma unroll
   for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) {
     float a, b;
     tc::upk2(acc[pidx], a, b);
-    a *= mul;
-    b *= mul;
+    a = valid ? a * mul : 0.f;
+    b = valid ? b * mul : 0.f;
     const int ch = pair_channel<DP>(l16, pidx);
     if (vec) {
       if (ch < D) *reinterpret_cast<float2*>(static_cast<float*>(p) + off + ch) = make_float2(a, b);
@@ -260,7 +295,7 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
     }
     if (M::kHasKFullRange) M::k_full_range_for_q(qg0, kRows, n, g.margs, full_lo, full_hi);
   }
-  load_tile<DP, kRows>(sQ, p.q, b, h, qb, rows_in, D, pp.dtype, pp.vec & kVecQ);
+  load_tile<DP, kRows>(sQ, p.q, b, h, qb, imin(rows_in, n - qg0), D, pp.dtype, pp.vec & kVecQ);
   const float c = g.scale * kLog2e;
   float m[RT], l[RT];
   uint64_t acc[RT][Lane<DP>::kPairs];
@@ -273,14 +308,14 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
   }
   for (int kt = kt_lo; kt < kt_hi; ++kt) {
     const int kb = kt * kCols, kg0 = kb + g.k_off;
+    const int ncols = imin(n - kg0, g.Lk - kb);
     __syncthreads();  // the previous step has read K and V
-    load_tile<DP, kCols>(sK, p.k, b, hk, kb, g.Lk - kb, D, pp.dtype, pp.vec & kVecK);
-    load_tile<DP, kCols>(sV, p.v, b, hk, kb, g.Lk - kb, D, pp.dtype, pp.vec & kVecV);
-    __syncthreads();
+    load_tile<DP, kCols>(sK, p.k, b, hk, kb, ncols, D, pp.dtype, pp.vec & kVecK);
+    const bool odd = load_tile<DP, kCols>(sV, p.v, b, hk, kb, ncols, D, pp.dtype, pp.vec & kVecV);
+    const bool finite = !__syncthreads_or(odd);
     float s[RT][4];
     scores<DP, RT>(sQ, sK, row0, l16, s);
-    const bool full = M::kHasKFullRange && kg0 >= full_lo && kg0 + kCols <= full_hi && kg0 + kCols <= n && kb + kCols <= g.Lk;
-    const int ncols = imin(n - kg0, g.Lk - kb);
+    const bool full = M::kHasKFullRange && kg0 >= full_lo && kg0 + kCols <= full_hi && ncols >= kCols;
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       const uint32_t vis = full ? 15u : visible4<M, true>(qg0 + row0 + i, kg0, ncols, l16, n, g.margs);
@@ -305,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
       *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = w;
     }
     __syncwarp();  // a row of W is written and read by one half-warp
-    accumulate<DP, RT>(sW, sV, row0, l16, acc);
+    accumulate<DP, RT>(sW, sV, row0, l16, acc, finite);
     __syncwarp();
   }
 #pragma unroll
@@ -316,8 +351,8 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
     const int row = qb + row0 + i;
     if (row >= g.Lq) continue;
     const bool valid = row + g.q_off < n;  // padded query rows: O = 0, LSE = 0
-    const float inv = (valid && sum != 0.f) ? 1.f / sum : 0.f;
-    store_row<DP>(p.o.p, b * p.o.sb + h * p.o.sh + row * p.o.sl, p.o.sd, D, pp.dtype, pp.vec & kVecO, l16, acc[i], inv);
+    const float inv = sum != 0.f ? 1.f / sum : 0.f;
+    store_row<DP>(p.o.p, b * p.o.sb + h * p.o.sh + row * p.o.sl, p.o.sd, D, pp.dtype, pp.vec & kVecO, l16, acc[i], inv, valid);
     if (p.lse != nullptr && l16 == 0)
       p.lse[b * p.lse_sb + h * p.lse_sh + row * p.lse_sl] = valid ? (sum == 0.f ? -CUDART_INF_F : m[i] + log2f(sum)) : 0.f;
   }
@@ -369,8 +404,9 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
   const TRef& r2 = kKeyRows ? p.v : p.d_o;
   const TRef& c1 = kKeyRows ? p.q : p.k;
   const TRef& c2 = kKeyRows ? p.d_o : p.v;
-  load_tile<DP, kRows>(sR1, r1, b, hr, rb, rows_in, D, pp.dtype, pp.vec & (kKeyRows ? kVecK : kVecQ));
-  load_tile<DP, kRows>(sR2, r2, b, hr, rb, rows_in, D, pp.dtype, pp.vec & (kKeyRows ? kVecV : kVecDo));
+  const int rows_valid = imin(rows_in, n - rg0);
+  load_tile<DP, kRows>(sR1, r1, b, hr, rb, rows_valid, D, pp.dtype, pp.vec & (kKeyRows ? kVecK : kVecQ));
+  load_tile<DP, kRows>(sR2, r2, b, hr, rb, rows_valid, D, pp.dtype, pp.vec & (kKeyRows ? kVecV : kVecDo));
   const float c = g.scale * kLog2e;
   float lse_r[RT], delta_r[RT];  // dQ part: of this half-warp's rows
   uint64_t acc1[RT][Lane<DP>::kPairs];                    // dK or dQ
@@ -393,9 +429,11 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
     const int hc = kKeyRows ? hr * G + gi : hr / G;
     for (int ct = ct_lo; ct < ct_hi; ++ct) {
       const int cb = ct * kCols, cg0 = cb + c_off;
+      const int ncols = imin(n - cg0, c_len - cb);
       __syncthreads();  // the previous step has read the streamed tiles
-      load_tile<DP, kCols>(sC1, c1, b, hc, cb, c_len - cb, D, pp.dtype, pp.vec & (kKeyRows ? kVecQ : kVecK));
-      load_tile<DP, kCols>(sC2, c2, b, hc, cb, c_len - cb, D, pp.dtype, pp.vec & (kKeyRows ? kVecDo : kVecV));
+      bool odd = load_tile<DP, kCols>(sC1, c1, b, hc, cb, ncols, D, pp.dtype, pp.vec & (kKeyRows ? kVecQ : kVecK));
+      const bool odd2 = load_tile<DP, kCols>(sC2, c2, b, hc, cb, ncols, D, pp.dtype, pp.vec & (kKeyRows ? kVecDo : kVecV));
+      if (kKeyRows) odd = odd || odd2;  // dV accumulates C2 as well
       float lse_c[4], delta_c[4];  // dK / dV part: of this lane's columns
       if (kKeyRows) {
 #pragma unroll
@@ -406,11 +444,9 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
           delta_c[j] = p.delta[((long long)b * g.H + hc) * g.Lq + q];
         }
       }
-      __syncthreads();
+      const bool finite = !__syncthreads_or(odd);
       const bool has_full = kKeyRows ? M::kHasQFullRange : M::kHasKFullRange;
-      const bool full = has_full && cg0 >= full_lo && cg0 + kCols <= full_hi && cg0 + kCols <= n && cb + kCols <= c_len &&
-                        rg0 + kRows <= n && rows_in == kRows;
-      const int ncols = imin(n - cg0, c_len - cb);
+      const bool full = has_full && cg0 >= full_lo && cg0 + kCols <= full_hi && ncols >= kCols && rows_valid == kRows;
       float w[RT][4];
       scores<DP, RT>(sR1, sC1, row0, l16, w);
 #pragma unroll
@@ -420,14 +456,14 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const float pe = exp2f(fmaf(w[i][j], c, -(kKeyRows ? lse_c[j] : lse_r[i])));
-          w[i][j] = ((vis >> j) & 1u) ? pe : 0.f;
+          w[i][j] = ((vis >> j) & 1u) ? pe : __uint_as_float(kHidden);
         }
         if (kKeyRows)
           *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = make_float4(w[i][0], w[i][1], w[i][2], w[i][3]);
       }
       if constexpr (kKeyRows) {
         __syncwarp();
-        accumulate<DP, RT>(sW, sC2, row0, l16, acc2);
+        accumulate<DP, RT, true>(sW, sC2, row0, l16, acc2, finite);
         __syncwarp();
       }
       {
@@ -436,12 +472,15 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
 #pragma unroll
         for (int i = 0; i < RT; ++i) {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) w[i][j] *= dp[i][j] - (kKeyRows ? delta_c[j] : delta_r[i]);
+          for (int j = 0; j < 4; ++j) {  // a select, not the product with zero: dP and delta of a hidden pair may be anything
+            const float ds = w[i][j] * (dp[i][j] - (kKeyRows ? delta_c[j] : delta_r[i]));
+            w[i][j] = __float_as_uint(w[i][j]) == kHidden ? 0.f : ds;
+          }
           *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = make_float4(w[i][0], w[i][1], w[i][2], w[i][3]);
         }
       }
       __syncwarp();
-      accumulate<DP, RT>(sW, sC1, row0, l16, acc1);
+      accumulate<DP, RT>(sW, sC1, row0, l16, acc1, finite);
       __syncwarp();
     }
   }
@@ -450,12 +489,13 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
     for (int i = 0; i < RT; ++i) {
       const int j = rb + row0 + i;
       if (j >= g.Lk) continue;
-      store_row<DP>(p.dk.p, b * p.dk.sb + hr * p.dk.sh + j * p.dk.sl, p.dk.sd, D, pp.dtype, pp.vec & kVecDk, l16, acc1[i], g.scale);
-      store_row<DP>(p.dv.p, b * p.dv.sb + hr * p.dv.sh + j * p.dv.sl, p.dv.sd, D, pp.dtype, pp.vec & kVecDv, l16, acc2[i], 1.f);
+      const bool valid = row0 + i < rows_valid;
+      store_row<DP>(p.dk.p, b * p.dk.sb + hr * p.dk.sh + j * p.dk.sl, p.dk.sd, D, pp.dtype, pp.vec & kVecDk, l16, acc1[i], g.scale, valid);
+      store_row<DP>(p.dv.p, b * p.dv.sb + hr * p.dv.sh + j * p.dv.sl, p.dv.sd, D, pp.dtype, pp.vec & kVecDv, l16, acc2[i], 1.f, valid);
       float* dkpart = p.part.row(p.part.dk, b, hr, j, g.Lk);
       if (dkpart != nullptr) {
-        store_row<DP>(dkpart, 0, 1, D, 0, true, l16, acc1[i], g.scale);
-        store_row<DP>(p.part.row(p.part.dv, b, hr, j, g.Lk), 0, 1, D, 0, true, l16, acc2[i], 1.f);
+        store_row<DP>(dkpart, 0, 1, D, 0, true, l16, acc1[i], g.scale, valid);
+        store_row<DP>(p.part.row(p.part.dv, b, hr, j, g.Lk), 0, 1, D, 0, true, l16, acc2[i], 1.f, valid);
       }
     }
   } else {
@@ -463,7 +503,8 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
     for (int i = 0; i < RT; ++i) {
       const int row = rb + row0 + i;
       if (row < g.Lq)
-        store_row<DP>(p.dq.p, b * p.dq.sb + hr * p.dq.sh + row * p.dq.sl, p.dq.sd, D, pp.dtype, pp.vec & kVecDq, l16, acc1[i], g.scale);
+        store_row<DP>(p.dq.p, b * p.dq.sb + hr * p.dq.sh + row * p.dq.sl, p.dq.sd, D, pp.dtype, pp.vec & kVecDq, l16, acc1[i], g.scale,
+                      row0 + i < rows_valid);
     }
   }
 }
