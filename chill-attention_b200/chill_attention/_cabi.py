@@ -150,6 +150,8 @@ def check(lib, status: int, what: str):
 
 
 def mask_desc(mask_id: int, args) -> MaskDesc:
+    """Mask constants in both members of the descriptor; whole numbers beyond 64 bits are saturated (ctypes would wrap
+    them around), NaN and infinity raise as in int()."""
     d = MaskDesc()
     d.id = mask_id
     args = tuple(args)
@@ -157,7 +159,7 @@ def mask_desc(mask_id: int, args) -> MaskDesc:
         raise ValueError(f"a mask takes at most {MAX_MASK_ARGS} constants")
     d.n_args = len(args)
     for n, a in enumerate(args):
-        d.i[n] = int(a)
+        d.i[n] = max(-2**63, min(2**63 - 1, int(a)))
         d.f[n] = float(a)
     return d
 

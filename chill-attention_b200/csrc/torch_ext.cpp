@@ -18,6 +18,8 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <utility>
+#include <vector>
 
 #include "chill_b200.h"
 
@@ -182,29 +184,32 @@ bool arguments_ok(const Tensor& q, const Tensor& k, const Tensor& v, const std::
   return true;
 }
 
+// Mask constants as both members of the descriptor.  The whole number is what Python's int() makes of the constant, which
+// refuses NaN and infinity; what 64 bits do not hold is saturated (the library clamps further).
+void set_mask_constants(chill_mask_desc& desc, const py::tuple& mask_args) {
+  if (mask_args.size() > CHILL_MAX_MASK_ARGS) throw py::value_error("a mask takes at most 8 constants");
+  desc.n_args = (int32_t)mask_args.size();
+  for (size_t n = 0; n < mask_args.size(); ++n) {
+    const py::object x = mask_args[n];
+    const py::object whole = py::reinterpret_steal<py::object>(PyNumber_Long(x.ptr()));
+    if (!whole) throw py::error_already_set();
+    int overflow = 0;
+    const long long i = PyLong_AsLongLongAndOverflow(whole.ptr(), &overflow);
+    desc.i[n] = overflow == 0 ? i : (overflow > 0 ? INT64_MAX : INT64_MIN);
+    desc.f[n] = PyFloat_AsDouble(x.ptr());
+    if (PyErr_Occurred()) throw py::error_already_set();
+  }
+}
+
 // O, (O, LSE) when return_lse, or None when the arguments do not pass the checks.
 py::object attention(std::shared_ptr<Library> lib, const Tensor& q, const Tensor& k, const Tensor& v, std::optional<Tensor> lens,
                      const py::tuple& mask_args, double sm_scale, bool return_lse, uint32_t flags) {
   if (!arguments_ok(q, k, v, lens)) return py::none();
-  if (mask_args.size() > CHILL_MAX_MASK_ARGS) throw py::value_error("a mask takes at most 8 constants");
   auto call = c10::make_intrusive<Call>();
   call->mask = chill_mask_desc{};
   call->mask.id = lib->functor_id;
   call->lib = std::move(lib);
-  call->mask.n_args = (int32_t)mask_args.size();
-  for (size_t n = 0; n < mask_args.size(); ++n) {
-    const py::object x = mask_args[n];
-    call->mask.f[n] = PyFloat_AsDouble(x.ptr());
-    if (PyErr_Occurred()) throw py::error_already_set();
-    if (PyFloat_Check(x.ptr())) {
-      call->mask.i[n] = (int64_t)call->mask.f[n];
-    } else {
-      int overflow = 0;
-      const long long i = PyLong_AsLongLongAndOverflow(x.ptr(), &overflow);
-      if (PyErr_Occurred()) throw py::error_already_set();
-      call->mask.i[n] = overflow == 0 ? i : (overflow > 0 ? INT64_MAX : INT64_MIN);  // the library saturates further
-    }
-  }
+  set_mask_constants(call->mask, mask_args);
   call->sm_scale = sm_scale;
   call->flags = flags;
   c10::cuda::CUDAGuard guard(q.device());
@@ -248,6 +253,13 @@ PYBIND11_MODULE(_chill_torch, m) {
                        pointer<decltype(&chill_last_cuda_error)>(fn[6]), functor_id});
       }));
   m.def("attention", &attention);
+  m.def("mask_constants", [](const py::tuple& mask_args) {  // what attention() hands to the library
+    chill_mask_desc desc{};
+    set_mask_constants(desc, mask_args);
+    std::vector<std::pair<int64_t, double>> out;
+    for (int n = 0; n < desc.n_args; ++n) out.emplace_back(desc.i[n], desc.f[n]);
+    return out;
+  });
   m.def("set_deterministic", [](bool flag) { g_deterministic = flag; });
   m.def("backward_counts", [] { return std::make_pair(g_bwd_tc.load(), g_bwd_generic.load()); });
   m.attr("abi_version") = CHILL_ABI_VERSION;
