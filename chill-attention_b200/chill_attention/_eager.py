@@ -10,7 +10,8 @@ Python autograd.Function over ctypes: forward of (8, 4, 128, 128) 17 -> 8 us, fo
 138 -> 78 us, most of the latter in torch's autograd engine and in five kernel launches.
 
 The path is taken only for plain CUDA tensors outside of tracing / dispatch modes / functorch transforms
-(``usable``); everything else, and every ``torch.compile`` graph, uses the dispatcher ops.  Set
+(``usable``); everything else, and every ``torch.compile`` graph, uses the dispatcher ops.  So does every call if the
+native module is missing or does not load (the kernel library built alone, another torch than it was built for).  Set
 ``CHILL_ATTENTION_EAGER_FAST=0`` to switch it off.
 """
 from __future__ import annotations
@@ -19,6 +20,7 @@ import ctypes as C
 import importlib.util
 import os
 import threading
+import warnings
 
 import torch
 
@@ -69,9 +71,17 @@ def extension():
 
 
 def native_library(lib, functor_id):
-    """The native call object of one mask functor: the kernel library's entry points and the functor id."""
+    """The native call object of one mask functor: the kernel library's entry points and the functor id.  None, after one
+    warning, if there is no native module to make it; ``usable`` says no from then on."""
+    global ENABLED
+    try:
+        module = extension()
+    except (ImportError, OSError, _cabi.ChillLibraryError) as e:
+        ENABLED = False
+        warnings.warn(f"chill_attention: eager calls go through the dispatcher ops, which take longer on the host: {e}", stacklevel=3)
+        return None
     addresses = [C.cast(getattr(lib, name), C.c_void_p).value for name in _ENTRY_POINTS]
-    return extension().Library(addresses, functor_id)
+    return module.Library(addresses, functor_id)
 
 
 def attention(native, q, k, v, lens, mask_args, sm_scale, return_lse, flags):

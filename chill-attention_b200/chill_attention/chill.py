@@ -330,7 +330,9 @@ def chill_attention(
         # plain eager call: same kernels through the short host path (see _eager.py)
         native = _NATIVE.get(mask.name)
         if native is None and mask.name in _REGISTRY:
-            native = _NATIVE[mask.name] = _eager.native_library(*_REGISTRY[mask.name])
+            native = _eager.native_library(*_REGISTRY[mask.name])
+            if native is not None:
+                _NATIVE[mask.name] = native
         if native is not None:
             out = _eager.attention(native, q, k, v, lens, mask.constargs, sm_scale, bool(return_lse), _call_flags(precision, q.dtype))
             if out is not None:

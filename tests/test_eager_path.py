@@ -1,0 +1,53 @@
+"""The native eager call path (chill_attention/_eager.py, csrc/torch_ext.cpp): what happens when it cannot serve a call."""
+import warnings
+
+import pytest
+import torch
+
+from helpers import check_forward, check_grads, ensure_built, make_inputs, oracle_all
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    ensure_built()
+
+
+@pytest.fixture(params=["missing", "not_a_library"])
+def no_module(request, monkeypatch, tmp_path):
+    """A tree in which only the kernel library was built, or whose native module was built for another torch."""
+    from chill_attention import _eager, chill
+
+    path = tmp_path / "_chill_torch.so"
+    if request.param == "not_a_library":
+        path.write_bytes(b"nothing the loader takes")
+    monkeypatch.setattr(_eager, "EXTENSION", str(path))
+    monkeypatch.setattr(_eager, "_extension", None)
+    monkeypatch.setattr(_eager, "ENABLED", True)
+    monkeypatch.setattr(chill, "_NATIVE", {})
+
+
+def test_no_native_module_switches_the_path_off(no_module):
+    from chill_attention import _cabi, _eager
+
+    with pytest.raises((ImportError, _cabi.ChillLibraryError)):
+        _eager.extension()
+    with pytest.warns(UserWarning, match="dispatcher ops"):
+        assert _eager.native_library(_cabi.load_library(), 0) is None
+    assert _eager.ENABLED is False
+
+
+@pytest.mark.gpu
+def test_calls_without_a_native_module(no_module):
+    import chill_attention as ca
+
+    mask, dtype = ca.CausalChillMask(), torch.float16
+    q, k, v, do = make_inputs(2, 4, 2, 150, 64, dtype)
+    o_ref, lse_ref, *g_ref = oracle_all(mask, q, k, v, do)
+    qd, kd, vd = (t.cuda().requires_grad_(True) for t in (q, k, v))
+    with pytest.warns(UserWarning, match="dispatcher ops"):
+        ca.chill_attention(qd, kd, vd, mask=mask)
+    with warnings.catch_warnings():
+        warnings.simplefilter("error")  # said once
+        o, lse = ca.chill_attention(qd, kd, vd, mask=mask, return_lse=True)
+    check_forward(o, lse, o_ref, lse_ref, None, dtype)
+    check_grads(torch.autograd.grad(o, (qd, kd, vd), do.cuda()), g_ref, dtype)
