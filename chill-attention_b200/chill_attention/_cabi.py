@@ -230,11 +230,12 @@ def set_deterministic(flag: bool) -> None:
     reproducible); False (default): the single-kernel backward is used where it applies.  Also on when
     ``torch.use_deterministic_algorithms(True)`` is set or CHILL_ATTENTION_DETERMINISTIC=1."""
     global _deterministic
-    _deterministic = bool(flag)
     from . import _eager
 
-    if _eager._extension is not None:  # otherwise handed over when the extension is loaded
-        _eager._extension.set_deterministic(_deterministic)
+    with _eager._lock:  # another thread may be loading the extension, which reads the flag
+        _deterministic = bool(flag)
+        if _eager._extension is not None:  # otherwise handed over when the extension is loaded
+            _eager._extension.set_deterministic(_deterministic)
 
 
 def is_deterministic() -> bool:

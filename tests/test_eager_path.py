@@ -51,3 +51,33 @@ def test_calls_without_a_native_module(no_module):
         o, lse = ca.chill_attention(qd, kd, vd, mask=mask, return_lse=True)
     check_forward(o, lse, o_ref, lse_ref, None, dtype)
     check_grads(torch.autograd.grad(o, (qd, kd, vd), do.cuda()), g_ref, dtype)
+
+
+def test_set_deterministic_while_the_module_loads(monkeypatch):
+    """The flag is set by one thread between the moment another one hands it to the module and the moment the module is
+    published; the module must end up with the new value."""
+    import importlib.util
+    import threading
+    from types import SimpleNamespace
+
+    from chill_attention import _cabi, _eager
+
+    class Module:
+        abi_version, flag, setter = _cabi.ABI_VERSION, None, None
+
+        def set_deterministic(self, flag):
+            self.flag = flag
+            if self.setter is None:
+                self.setter = threading.Thread(target=_cabi.set_deterministic, args=(True,))
+                self.setter.start()
+                self.setter.join(0.3)  # without a lock it is through by then
+
+    module, spec = Module(), SimpleNamespace(loader=SimpleNamespace(exec_module=lambda m: None))
+    monkeypatch.setattr(importlib.util, "spec_from_file_location", lambda *a: spec)
+    monkeypatch.setattr(importlib.util, "module_from_spec", lambda s: module)
+    monkeypatch.setattr(_eager, "EXTENSION", __file__)
+    monkeypatch.setattr(_eager, "_extension", None)
+    monkeypatch.setattr(_cabi, "_deterministic", False)
+    assert _eager.extension() is module
+    module.setter.join()
+    assert _cabi.is_deterministic() and module.flag is True
