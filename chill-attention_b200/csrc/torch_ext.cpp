@@ -11,12 +11,12 @@
 #include <ATen/ops/zeros_like.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <atomic>
 #include <memory>
-#include <stdexcept>
 #include <string>
 #include <utility>
 #include <vector>
@@ -45,9 +45,11 @@ struct Library {
 std::atomic<bool> g_deterministic{false};
 std::atomic<long long> g_bwd_tc{0}, g_bwd_generic{0};
 
-// Raised as chill_attention._cabi.ChillLibraryError in Python.
-struct ChillError : std::runtime_error {
-  using std::runtime_error::runtime_error;
+// Raised as chill_attention._cabi.ChillLibraryError in Python: torch asks such an exception for its type wherever it crosses
+// over, be it out of a call of this module or out of a backward that the autograd engine runs.
+struct ChillError : torch::PyTorchError {
+  using torch::PyTorchError::PyTorchError;
+  PyObject* python_type() override { return py::module_::import("chill_attention._cabi").attr("ChillLibraryError").ptr(); }
 };
 
 struct Call : torch::CustomClassHolder {
@@ -237,13 +239,6 @@ F pointer(uint64_t address) {
 }  // namespace
 
 PYBIND11_MODULE(_chill_torch, m) {
-  py::register_exception_translator([](std::exception_ptr p) {
-    try {
-      if (p) std::rethrow_exception(p);
-    } catch (const ChillError& e) {
-      PyErr_SetString(py::module_::import("chill_attention._cabi").attr("ChillLibraryError").ptr(), e.what());
-    }
-  });
   py::class_<Library, std::shared_ptr<Library>>(m, "Library")
       .def(py::init([](const std::vector<uint64_t>& fn, int32_t functor_id) {
         if (fn.size() != 7) throw py::value_error("seven entry points");

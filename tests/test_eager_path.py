@@ -81,3 +81,24 @@ def test_set_deterministic_while_the_module_loads(monkeypatch):
     assert _eager.extension() is module
     module.setter.join()
     assert _cabi.is_deterministic() and module.flag is True
+
+
+@pytest.mark.gpu
+def test_an_error_of_the_library_has_its_own_type_in_both_directions(monkeypatch):
+    """chill_fwd or chill_bwd replaced by a host function that only returns a status."""
+    import ctypes as C
+
+    import chill_attention as ca
+    from chill_attention import _cabi, _eager, chill
+
+    refuse = C.CFUNCTYPE(C.c_int, C.c_void_p, C.c_void_p)(lambda args, stream: -4)
+    mask, lib = ca.CausalChillMask(), _cabi.load_library()
+    q = make_inputs(1, 2, 2, 64, 64, torch.float16)[0].cuda().requires_grad_(True)
+    o = ca.chill_attention(q, q, q, mask=mask)  # registers the mask
+    for name in ("chill_fwd", "chill_bwd"):
+        addresses = [C.cast(refuse if n == name else getattr(lib, n), C.c_void_p).value for n in _eager._ENTRY_POINTS]
+        monkeypatch.setitem(chill._NATIVE, mask.name, _eager.extension().Library(addresses, _cabi.MASK_CAUSAL))
+        with pytest.raises(_cabi.ChillLibraryError, match=f"{name} failed: size exceeds"):
+            o = ca.chill_attention(q, q, q, mask=mask)
+            o.sum().backward()
+    assert q.grad is None
