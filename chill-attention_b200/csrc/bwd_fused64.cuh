@@ -477,11 +477,10 @@ bwd_fused64_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 //   few CTAs:     (4,8,300) full, 96 CTAs: 11.7 / 13.5     uneven ones: (8,8,1024) causal (5 tiles): 57 / 66
 // so the line lies at four tiles, below what the uniform masks alone would allow.
 constexpr int kF64MaxTiles = 4;
-constexpr int kF64MinCtas = 2 * 148;
 template <class M>
 bool bwd_short_loops(const Geo& g, int D) {
   const int n_kt = (g.Lk + kTile - 1) / kTile;
-  if (D > 64 || (long long)n_kt * g.Hkv * g.B < kF64MinCtas) return false;
+  if (D > 64 || (long long)n_kt * g.Hkv * g.B < 2 * sm_count()) return false;
   const int kg0 = (n_kt - 1) / 2 * kTile + g.k_off;
   int lo, hi;
   tile_range<M, false>(kg0, kTile, g.seq_len, g.margs, lo, hi);

@@ -398,6 +398,19 @@ static int bwd_which(uint32_t flags) {
   return 3;
 }
 
+// CHILL_BWD_*: the kernels that serve a backward call (include/chill_b200.h).
+static int bwd_kernels(const chill_bwd_args& a) {
+  if (bwd_tc_eligible(a)) {
+    if (bwd_which(a.s.flags) != 3 || a.dq_accum == nullptr) return CHILL_BWD_TWO_KERNELS;
+    bool pair = false;
+    CHILL_MASK_SWITCH(a.s.mask.id, (pair = tc_bwd_short_loops<MaskT>(to_geo(a.s), a.s.D)))
+    return pair ? CHILL_BWD_SINGLE_PAIR : CHILL_BWD_SINGLE;
+  }
+  if (bwd_wide_eligible(a)) return CHILL_BWD_WIDE;
+  if (bwd_tf32_eligible(a)) return CHILL_BWD_TF32;
+  return CHILL_BWD_CUDA_CORES;
+}
+
 static int bwd_generic(const chill_bwd_args& a, cudaStream_t st) {
   simt::BwdParams pp;
   pp.b = to_bwdp(a);
@@ -485,7 +498,8 @@ static int bwd_tf32(const chill_bwd_args& a, cudaStream_t st) {
   return e == 0 ? CHILL_OK : cuda_fail((cudaError_t)e, "bwd_tf32 launch");
 }
 
-static int bwd_tc(const chill_bwd_args& a, cudaStream_t st, bool concurrent = true, bool fused = true) {
+// `kernels`: CHILL_BWD_TWO_KERNELS, CHILL_BWD_SINGLE or CHILL_BWD_SINGLE_PAIR
+static int bwd_tc(const chill_bwd_args& a, cudaStream_t st, int kernels, bool concurrent = true) {
   const chill_shape& s = a.s;
   CUtensorMap maps[7];
   const void* ptrs[7] = {a.q, a.k, a.v, a.d_o, a.dq, a.dk, a.dv};
@@ -493,10 +507,8 @@ static int bwd_tc(const chill_bwd_args& a, cudaStream_t st, bool concurrent = tr
   const bool is_kv[7] = {false, true, true, false, false, true, true};
   tc::BwdTcParams p;
   fill_bwd_tc_params(a, p);
-  const bool single = fused && p.which == 3 && a.dq_accum != nullptr;
-  if (single) {
-    CHILL_MASK_SWITCH(s.mask.id, (p.short_loops = tc_bwd_short_loops<MaskT>(p.g, s.D)))
-  }
+  const bool single = kernels != CHILL_BWD_TWO_KERNELS;
+  p.short_loops = kernels == CHILL_BWD_SINGLE_PAIR;
   for (int i = 0; i < 7; ++i) {
     const int rows = p.short_loops && (i == 0 || i == 3) ? tc::kF64Step : tc::kTile;
     int rc = make_map(&maps[i], ptrs[i], strs[i], s.B, is_kv[i] ? s.H_kv : s.H, is_kv[i] ? s.Lk : s.Lq, s.D, s.dtype, rows);
@@ -659,6 +671,11 @@ int chill_bwd_uses_tensor_cores(const chill_bwd_args* a) {
   return (bwd_tc_eligible(*a) || bwd_wide_eligible(*a) || bwd_tf32_eligible(*a)) ? 1 : 0;
 }
 
+int chill_bwd_kernels(const chill_bwd_args* a) {
+  int st = check_bwd(a, true);
+  return st != CHILL_OK ? st : bwd_kernels(*a);
+}
+
 int chill_fwd(const chill_fwd_args* a, void* stream) {
   int st = check_fwd(a);
   if (st != CHILL_OK) return st;
@@ -687,9 +704,11 @@ int chill_bwd_delta(const chill_bwd_args* a, void* stream) {
 int chill_bwd(const chill_bwd_args* a, void* stream) {
   int st = check_bwd(a, true);
   if (st != CHILL_OK) return st;
-  if (bwd_tc_eligible(*a)) return bwd_tc(*a, (cudaStream_t)stream);
-  if (bwd_wide_eligible(*a)) return bwd_wide(*a, (cudaStream_t)stream);
-  if (bwd_tf32_eligible(*a)) return bwd_tf32(*a, (cudaStream_t)stream);
+  const int kernels = bwd_kernels(*a);
+  if (kernels < 0) return kernels;
+  if (kernels == CHILL_BWD_WIDE) return bwd_wide(*a, (cudaStream_t)stream);
+  if (kernels == CHILL_BWD_TF32) return bwd_tf32(*a, (cudaStream_t)stream);
+  if (kernels != CHILL_BWD_CUDA_CORES) return bwd_tc(*a, (cudaStream_t)stream, kernels);
   if (a->s.flags & CHILL_FLAG_REQUIRE_TC) return CHILL_E_UNSUPPORTED;
   return bwd_generic(*a, (cudaStream_t)stream);
 }
@@ -712,7 +731,7 @@ int chill_bwd_noalloc(const chill_bwd_args* a, void* stream) {
   b.delta = scratch;
   st = delta_launch(b, (cudaStream_t)stream);
   if (st != CHILL_OK) return st;
-  if (bwd_tc_eligible(b)) return bwd_tc(b, (cudaStream_t)stream, /*concurrent=*/false, /*fused=*/false);  // one stream, no helper objects
+  if (bwd_tc_eligible(b)) return bwd_tc(b, (cudaStream_t)stream, CHILL_BWD_TWO_KERNELS, /*concurrent=*/false);  // one stream, no helper objects
   if (bwd_wide_eligible(b)) return bwd_wide(b, (cudaStream_t)stream);
   if (bwd_tf32_eligible(b)) return bwd_tf32(b, (cudaStream_t)stream);
   if (b.s.flags & CHILL_FLAG_REQUIRE_TC) return CHILL_E_UNSUPPORTED;

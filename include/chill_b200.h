@@ -249,6 +249,16 @@ size_t chill_bwd_dq_accum_bytes(const chill_shape* s);
 int chill_fwd_uses_tensor_cores(const chill_fwd_args* a);
 int chill_bwd_uses_tensor_cores(const chill_bwd_args* a);
 
+/* Which kernels chill_bwd would launch for these arguments (host-only; pointers are looked at for their alignment), or a
+ * negative status if the arguments are invalid. */
+#define CHILL_BWD_CUDA_CORES 0   /* simt.cuh */
+#define CHILL_BWD_TWO_KERNELS 1  /* dK / dV and dQ, bitwise reproducible: 16-bit without dq_accum, or one of the two alone */
+#define CHILL_BWD_SINGLE 2       /* one kernel, dQ summed in dq_accum */
+#define CHILL_BWD_SINGLE_PAIR 3  /* the same with two CTAs per SM: head dim <= 64, few query tiles per key tile */
+#define CHILL_BWD_WIDE 4         /* 16-bit head dim 256 */
+#define CHILL_BWD_TF32 5         /* fp32 with CHILL_FLAG_ALLOW_TF32 */
+int chill_bwd_kernels(const chill_bwd_args* a);
+
 /* Tabulate a mask functor on the device (all outputs optional, device pointers):
  *   dense   uint8[n*n]   mask(q, k) for q, k in [0, n)            (row = query)
  *   k_lims  int32[n*2]   k_range_for_q(q), inclusive

@@ -41,6 +41,22 @@ def make_inputs(B, H, Hkv, L, D, dtype, seed=20):
     return q, k, v, do
 
 
+def bwd_kernels(lib, mask, B, H, Hkv, L, D, dtype, flags=0, accum=True, functor=None, pointer=4096):
+    """chill_bwd_kernels for contiguous tensors of this shape (host-only: the pointers are never followed)."""
+    import ctypes as C
+
+    from chill_attention import _cabi
+
+    q, k = (torch.empty(B, h, L, D, dtype=dtype, device="meta") for h in (H, Hkv))
+    row = torch.empty(B, H, L, device="meta")
+    functor = _cabi.BUILTIN_FUNCTOR_IDS[mask.cuda_functor] if functor is None else functor
+    a = _cabi.backward_args(q, k, k, q, q, row, row, q, k, k, _cabi.make_shape(q, k, functor, mask.constargs, None, D ** -0.5, flags=flags))
+    for name in ("q", "k", "v", "o", "d_o", "lse", "delta", "dq", "dk", "dv"):
+        setattr(a, name, pointer)
+    a.dq_accum = 4096 if accum else None
+    return lib.chill_bwd_kernels(C.byref(a))
+
+
 def oracle_all(mask, q, k, v, do, lens=None, sm_scale=None):
     """fp64 oracle on the (rounded) inputs: O, LSE2, dQ, dK, dV."""
     L = q.shape[2]

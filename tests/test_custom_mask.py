@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import chill_attention as ca
-from helpers import ROOT, check_forward, check_grads, make_inputs
+from helpers import ROOT, bwd_kernels, check_forward, check_grads, make_inputs
 
 HEADER = os.path.join(ROOT, "tests", "custom_masks", "dilated_causal_mask.h")
 
@@ -78,6 +78,26 @@ def test_custom_mask_on_gpu(dtype, D):
     check_forward(o, lse, o_ref, lse_ref, None, dtype)
     check_grads((qd.grad, kd.grad, vd.grad), g_ref, dtype)
     assert hasattr(torch.ops.chill_attention, "forwardDilatedCausalChillMask")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("D", [32, 64])
+def test_custom_mask_on_gpu_with_two_ctas_per_sm(D):
+    """A functor whose visible sets are no intervals in the backward that shares an SM between two CTAs."""
+    from chill_attention import _cabi
+    from chill_attention.custom import build_custom_library
+    from oracle import attention_oracle as orc
+
+    mask, dtype, B, H, L = DilatedCausalChillMask(3), torch.float16, 2, 50, 300
+    lib = _cabi.load_library(build_custom_library(HEADER, "DilatedCausalMask"))
+    assert bwd_kernels(lib, mask, B, H, H, L, D, dtype, _cabi.FLAG_NARROW_HEAD, functor=_cabi.MASK_CUSTOM) == _cabi.BWD_SINGLE_PAIR
+    q, k, v, do = make_inputs(B, H, H, L, D, dtype)
+    pos = torch.arange(L)
+    md = DilatedCausalChillMask.mask(pos, pos, L, mask.constargs)
+    g_ref = orc.attention_backward(md, q.double(), k.double(), v.double(), do.double())
+    qd, kd, vd = (t.cuda().requires_grad_(True) for t in (q, k, v))
+    o = ca.chill_attention(qd, kd, vd, mask=mask)
+    check_grads(torch.autograd.grad(o, (qd, kd, vd), do.cuda()), g_ref, dtype)
 
 
 class OffByOneWindowChillMask(ca.ChillMask):

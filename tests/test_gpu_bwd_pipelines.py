@@ -3,7 +3,7 @@ first round of every ring, the wrap-around and the last step are each reached), 
 import pytest
 import torch
 
-from helpers import G_RTOL, big_masks, ensure_built, make_inputs, oracle_all
+from helpers import G_RTOL, big_masks, bwd_kernels, ensure_built, make_inputs, oracle_all
 
 pytestmark = pytest.mark.gpu
 
@@ -60,15 +60,17 @@ def test_head_dim_64_tiles(L, dtype):
 
 
 @pytest.mark.parametrize("kind", ["window", "one_sided", "chunkwise", "off_grid_chunks", "full", "causal"])
-def test_head_dim_64_short_loops(kind):
+def test_head_dim_64_short_loops(kind, _lib):
     """Enough key tiles and few enough query tiles for the form with two CTAs per SM (steps of 64 queries, two to a dQ tile):
     first or last half of a query tile missing, ragged last step, rows of padding only, one or two heads per key head."""
     import chill_attention as ca
+    from chill_attention import _cabi
 
     mask = {"window": ca.SlidingWindowChillMask(40, 5), "one_sided": ca.SlidingWindowChillMask(0, 70), "chunkwise": ca.ChunkwiseChillMask(64, 1),
             "off_grid_chunks": ca.ChunkwiseChillMask(48, 0), "full": ca.FullChillMask(), "causal": ca.CausalChillMask()}[kind]
     L, dtype = (200, torch.bfloat16) if kind in ("full", "causal") else (330, torch.float16)
     heads = 30 if kind in ("window", "off_grid_chunks") else 60  # these see three query tiles per key tile, the others two
+    assert bwd_kernels(_lib, mask, 5, heads, 30, L, 64, dtype) == _cabi.BWD_SINGLE_PAIR
     q, k, v, do = make_inputs(5, heads, 30, L, 64, dtype, seed=7)
     lens = torch.tensor([L, L - 1, 129, 64, 2], dtype=torch.int32)
     _, _, *refs = oracle_all(mask, q, k, v, do, lens)
@@ -98,6 +100,7 @@ def test_head_dim_64_short_loops_of_a_shard(_lib):
     part = [torch.full((1, H, head + tail, D), float("nan"), dtype=torch.float32, device="cuda") for _ in range(2)]
     g = [torch.full_like(t, float("nan")) for t in (qs, ks, vs)]
     a = _cabi.backward_args(qs, ks, vs, o, dos, lse, delta, *g, shape, accum, part=(part[0], part[1], head, tail))
+    assert _lib.chill_bwd_kernels(C.byref(a)) == _cabi.BWD_SINGLE_PAIR
     _cabi.check(_lib, _lib.chill_bwd_delta(C.byref(a), _cabi._stream()), "chill_bwd_delta")
     _cabi.check(_lib, _lib.chill_bwd(C.byref(a), _cabi._stream()), "chill_bwd")
     torch.cuda.synchronize()
