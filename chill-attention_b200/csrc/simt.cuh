@@ -63,15 +63,13 @@ __device__ __forceinline__ void store_elem(void* p, long long i, int dtype, floa
 __device__ __forceinline__ int swz(int row) { return (row >> 2) & 7; }
 
 // One tile of ROWS x DP elements, starting at row `row0` of head h of batch row b, to shared memory as fp32; rows beyond
-// rows_in (what does not exist or is padding: it may hold anything) and channels beyond D become zeros.  Returns whether
-// one of the elements this thread loaded is NaN or infinite (see accumulate).
+// rows_in (what does not exist or is padding, which may hold anything) and channels beyond D become zeros.
 template <int DP, int ROWS>
-__device__ __forceinline__ bool load_tile(float* s, const TRef& t, int b, int h, int row0, int rows_in, int D, int dtype, bool vec) {
+__device__ __forceinline__ void load_tile(float* s, const TRef& t, int b, int h, int row0, int rows_in, int D, int dtype, bool vec) {
   constexpr int kChunks = DP / 4, kPerThread = ROWS * kChunks / kThreads;
   static_assert(ROWS * kChunks % kThreads == 0, "every thread moves the same number of chunks");
   constexpr int kBatch = kPerThread < 8 ? kPerThread : 8;  // loads in flight per thread
   const long long origin = b * t.sb + h * t.sh + row0 * t.sl;
-  uint64_t probe = 0ull;  // both halves stay zero while everything is finite: x * 0 is NaN otherwise
 #pragma unroll 1
   for (int i0 = 0; i0 < kPerThread; i0 += kBatch) {
     float4 v[kBatch];
@@ -91,7 +89,6 @@ __device__ __forceinline__ bool load_tile(float* s, const TRef& t, int b, int h,
         float e[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) e[k] = (row < rows_in && c * 4 + k < D) ? load_elem(t.p, origin + row * t.sl + (c * 4 + k) * t.sd, dtype) : 0.f;
-        probe = tc::ffma2(tc::pk2(e[0], e[1]), 0ull, tc::ffma2(tc::pk2(e[2], e[3]), 0ull, probe));
         *reinterpret_cast<float4*>(s + row * DP + 4 * (c ^ swz(row))) = make_float4(e[0], e[1], e[2], e[3]);
       }
       continue;
@@ -100,13 +97,9 @@ __device__ __forceinline__ bool load_tile(float* s, const TRef& t, int b, int h,
     for (int i = 0; i < kBatch; ++i) {
       const int idx = (i0 + i) * kThreads + threadIdx.x;
       const int row = idx / kChunks, c = idx % kChunks;
-      probe = tc::ffma2(tc::pk2(v[i].x, v[i].y), 0ull, tc::ffma2(tc::pk2(v[i].z, v[i].w), 0ull, probe));
       *reinterpret_cast<float4*>(s + row * DP + 4 * (c ^ swz(row))) = v[i];
     }
   }
-  float lo, hi;
-  tc::upk2(probe, lo, hi);
-  return !(lo == 0.f && hi == 0.f);
 }
 
 // s[i][j] = sum over channels of A[row0 + i][.] * B[4 * l16 + j][.]
@@ -168,17 +161,16 @@ __device__ __forceinline__ void lane_channels(const float* X, int row, int fx, i
   }
 }
 
-// Weight of a pair that the row may not see, where that has to be told apart from a probability that has underflowed.
-constexpr uint32_t kHidden = 0x80000000u;  // -0.0f: adds nothing, and 2^x is never it
-
 // acc[i][.] += sum over the 64 streamed positions of W[row0 + i][.] * X[.][channels of this lane]
 //
-// A hidden pair must add nothing, but 0 * NaN and 0 * Inf are NaN.  So tiles of X with such an element (`finite` false, the
-// same for the whole CTA) take a loop that leaves pairs out: every zero weight, or with kKeepZeros only the kHidden ones.
-template <int DP, int RT, bool kKeepZeros = false>
-__device__ __forceinline__ void accumulate(const float* W, const float* X, int row0, int l16, uint64_t (&acc)[RT][Lane<DP>::kPairs], bool finite) {
+// A hidden pair must add nothing, but 0 * NaN and 0 * Inf are NaN.  No NaN ever leaves an accumulator again, so a CTA that ends
+// without one has met no such product; one that ends with a NaN repeats its work with `careful` set, which takes a loop that
+// leaves the pairs out for which skip(row, position, weight) is true.
+template <int DP, int RT, class Skip>
+__device__ __forceinline__ void accumulate(const float* W, const float* X, int row0, int l16, uint64_t (&acc)[RT][Lane<DP>::kPairs], bool careful,
+                                           const Skip& skip) {
   const int fa = swz(row0);
-  if (!finite) {
+  if (careful) {
 #pragma unroll 1
     for (int kx = 0; kx < kCols; ++kx) {
       uint64_t x[Lane<DP>::kPairs];
@@ -186,7 +178,7 @@ __device__ __forceinline__ void accumulate(const float* W, const float* X, int r
 #pragma unroll
       for (int i = 0; i < RT; ++i) {
         const float wk = W[(row0 + i) * kCols + 4 * ((kx >> 2) ^ (fa + (i >> 2))) + (kx & 3)];
-        if (kKeepZeros ? __float_as_uint(wk) == kHidden : wk == 0.f) continue;
+        if (skip(i, kx, wk)) continue;
         const uint64_t w2 = tc::pk2(wk, wk);
 #pragma unroll
         for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) acc[i][pidx] = tc::ffma2(w2, x[pidx], acc[i][pidx]);
@@ -213,6 +205,19 @@ __device__ __forceinline__ void accumulate(const float* W, const float* X, int r
       }
     }
   }
+}
+
+// Whether one of the accumulators is NaN (or two are opposite infinities).
+template <int DP, int N>
+__device__ __forceinline__ bool any_nan(const uint64_t (&acc)[N][Lane<DP>::kPairs]) {
+  uint64_t sum[2] = {};
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+#pragma unroll
+    for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) sum[(i + pidx) & 1] = tc::fadd2(sum[(i + pidx) & 1], acc[i][pidx]);
+  float lo, hi;
+  tc::upk2(tc::fadd2(sum[0], sum[1]), lo, hi);
+  return lo + hi != lo + hi;
 }
 
 template <int DP>
@@ -299,49 +304,52 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
   const float c = g.scale * kLog2e;
   float m[RT], l[RT];
   uint64_t acc[RT][Lane<DP>::kPairs];
-#pragma unroll
-  for (int i = 0; i < RT; ++i) {
-    m[i] = -CUDART_INF_F;
-    l[i] = 0.f;
-#pragma unroll
-    for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) acc[i][pidx] = 0ull;
-  }
-  for (int kt = kt_lo; kt < kt_hi; ++kt) {
-    const int kb = kt * kCols, kg0 = kb + g.k_off;
-    const int ncols = imin(n - kg0, g.Lk - kb);
-    __syncthreads();  // the previous step has read K and V
-    load_tile<DP, kCols>(sK, p.k, b, hk, kb, ncols, D, pp.dtype, pp.vec & kVecK);
-    const bool odd = load_tile<DP, kCols>(sV, p.v, b, hk, kb, ncols, D, pp.dtype, pp.vec & kVecV);
-    const bool finite = !__syncthreads_or(odd);
-    float s[RT][4];
-    scores<DP, RT>(sQ, sK, row0, l16, s);
-    const bool full = M::kHasKFullRange && kg0 >= full_lo && kg0 + kCols <= full_hi && ncols >= kCols;
+  for (bool careful = false;; careful = true) {
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
-      const uint32_t vis = full ? 15u : visible4<M, true>(qg0 + row0 + i, kg0, ncols, l16, n, g.margs);
+      m[i] = -CUDART_INF_F;
+      l[i] = 0.f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s[i][j] = ((vis >> j) & 1u) ? s[i][j] * c : -CUDART_INF_F;
-      float mx = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      const float m_new = fmaxf(m[i], mx);
-      const float m_safe = (m_new == -CUDART_INF_F) ? 0.f : m_new;
-      const float alpha = exp2f(m[i] - m_safe);
-      m[i] = m_new;
-      float4 w;
-      w.x = exp2f(s[i][0] - m_safe);
-      w.y = exp2f(s[i][1] - m_safe);
-      w.z = exp2f(s[i][2] - m_safe);
-      w.w = exp2f(s[i][3] - m_safe);
-      l[i] = l[i] * alpha + ((w.x + w.y) + (w.z + w.w));  // this lane's columns; summed over the row at the end
-      const uint64_t a2 = tc::pk2(alpha, alpha);
-#pragma unroll
-      for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) acc[i][pidx] = tc::fmul2(acc[i][pidx], a2);
-      *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = w;
+      for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) acc[i][pidx] = 0ull;
     }
-    __syncwarp();  // a row of W is written and read by one half-warp
-    accumulate<DP, RT>(sW, sV, row0, l16, acc, finite);
-    __syncwarp();
+    for (int kt = kt_lo; kt < kt_hi; ++kt) {
+      const int kb = kt * kCols, kg0 = kb + g.k_off;
+      const int ncols = imin(n - kg0, g.Lk - kb);
+      __syncthreads();  // the previous step has read K and V
+      load_tile<DP, kCols>(sK, p.k, b, hk, kb, ncols, D, pp.dtype, pp.vec & kVecK);
+      load_tile<DP, kCols>(sV, p.v, b, hk, kb, ncols, D, pp.dtype, pp.vec & kVecV);
+      __syncthreads();
+      float s[RT][4];
+      scores<DP, RT>(sQ, sK, row0, l16, s);
+      const bool full = M::kHasKFullRange && kg0 >= full_lo && kg0 + kCols <= full_hi && ncols >= kCols;
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        const uint32_t vis = full ? 15u : visible4<M, true>(qg0 + row0 + i, kg0, ncols, l16, n, g.margs);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[i][j] = ((vis >> j) & 1u) ? s[i][j] * c : -CUDART_INF_F;
+        float mx = fmaxf(fmaxf(s[i][0], s[i][1]), fmaxf(s[i][2], s[i][3]));
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float m_new = fmaxf(m[i], mx);
+        const float m_safe = (m_new == -CUDART_INF_F) ? 0.f : m_new;
+        const float alpha = exp2f(m[i] - m_safe);
+        m[i] = m_new;
+        float4 w;
+        w.x = exp2f(s[i][0] - m_safe);
+        w.y = exp2f(s[i][1] - m_safe);
+        w.z = exp2f(s[i][2] - m_safe);
+        w.w = exp2f(s[i][3] - m_safe);
+        l[i] = l[i] * alpha + ((w.x + w.y) + (w.z + w.w));  // this lane's columns; summed over the row at the end
+        const uint64_t a2 = tc::pk2(alpha, alpha);
+#pragma unroll
+        for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) acc[i][pidx] = tc::fmul2(acc[i][pidx], a2);
+        *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = w;
+      }
+      __syncwarp();  // a row of W is written and read by one half-warp
+      accumulate<DP, RT>(sW, sV, row0, l16, acc, careful, [](int, int, float wk) { return wk == 0.f; });
+      __syncwarp();
+    }
+    if (careful || !__syncthreads_or(any_nan<DP>(acc))) break;
   }
 #pragma unroll
   for (int i = 0; i < RT; ++i) {
@@ -413,11 +421,6 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
   uint64_t acc2[kKeyRows ? RT : 1][Lane<DP>::kPairs];     // dV
 #pragma unroll
   for (int i = 0; i < RT; ++i) {
-#pragma unroll
-    for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) {
-      acc1[i][pidx] = 0ull;
-      if (kKeyRows) acc2[kKeyRows ? i : 0][pidx] = 0ull;
-    }
     lse_r[i] = delta_r[i] = 0.f;
     if (!kKeyRows && rb + row0 + i < g.Lq) {
       const float v = p.lse[b * p.lse_sb + hr * p.lse_sh + (rb + row0 + i) * p.lse_sl];
@@ -425,64 +428,75 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
       delta_r[i] = p.delta[((long long)b * g.H + hr) * g.Lq + rb + row0 + i];
     }
   }
-  for (int gi = 0; gi < (kKeyRows ? G : 1); ++gi) {
-    const int hc = kKeyRows ? hr * G + gi : hr / G;
-    for (int ct = ct_lo; ct < ct_hi; ++ct) {
-      const int cb = ct * kCols, cg0 = cb + c_off;
-      const int ncols = imin(n - cg0, c_len - cb);
-      __syncthreads();  // the previous step has read the streamed tiles
-      bool odd = load_tile<DP, kCols>(sC1, c1, b, hc, cb, ncols, D, pp.dtype, pp.vec & (kKeyRows ? kVecQ : kVecK));
-      const bool odd2 = load_tile<DP, kCols>(sC2, c2, b, hc, cb, ncols, D, pp.dtype, pp.vec & (kKeyRows ? kVecDo : kVecV));
-      if (kKeyRows) odd = odd || odd2;  // dV accumulates C2 as well
-      float lse_c[4], delta_c[4];  // dK / dV part: of this lane's columns
-      if (kKeyRows) {
+  for (bool careful = false;; careful = true) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int q = imin(cb + 4 * l16 + j, g.Lq - 1);  // columns beyond Lq are masked out
-          const float v = p.lse[b * p.lse_sb + hc * p.lse_sh + q * p.lse_sl];
-          lse_c[j] = v == -CUDART_INF_F ? 0.f : v;
-          delta_c[j] = p.delta[((long long)b * g.H + hc) * g.Lq + q];
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int pidx = 0; pidx < Lane<DP>::kPairs; ++pidx) {
+        acc1[i][pidx] = 0ull;
+        if (kKeyRows) acc2[kKeyRows ? i : 0][pidx] = 0ull;
+      }
+    for (int gi = 0; gi < (kKeyRows ? G : 1); ++gi) {
+      const int hc = kKeyRows ? hr * G + gi : hr / G;
+      for (int ct = ct_lo; ct < ct_hi; ++ct) {
+        const int cb = ct * kCols, cg0 = cb + c_off;
+        const int ncols = imin(n - cg0, c_len - cb);
+        __syncthreads();  // the previous step has read the streamed tiles
+        load_tile<DP, kCols>(sC1, c1, b, hc, cb, ncols, D, pp.dtype, pp.vec & (kKeyRows ? kVecQ : kVecK));
+        load_tile<DP, kCols>(sC2, c2, b, hc, cb, ncols, D, pp.dtype, pp.vec & (kKeyRows ? kVecDo : kVecV));
+        float lse_c[4], delta_c[4];  // dK / dV part: of this lane's columns
+        if (kKeyRows) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int q = imin(cb + 4 * l16 + j, g.Lq - 1);  // columns beyond Lq are masked out
+            const float v = p.lse[b * p.lse_sb + hc * p.lse_sh + q * p.lse_sl];
+            lse_c[j] = v == -CUDART_INF_F ? 0.f : v;
+            delta_c[j] = p.delta[((long long)b * g.H + hc) * g.Lq + q];
+          }
         }
-      }
-      const bool finite = !__syncthreads_or(odd);
-      const bool has_full = kKeyRows ? M::kHasQFullRange : M::kHasKFullRange;
-      const bool full = has_full && cg0 >= full_lo && cg0 + kCols <= full_hi && ncols >= kCols && rows_valid == kRows;
-      float w[RT][4];
-      scores<DP, RT>(sR1, sC1, row0, l16, w);
-#pragma unroll
-      for (int i = 0; i < RT; ++i) {
-        uint32_t vis = 15u;
-        if (!full) vis = row0 + i < rows_in ? visible4<M, !kKeyRows>(rg0 + row0 + i, cg0, ncols, l16, n, g.margs) : 0u;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float pe = exp2f(fmaf(w[i][j], c, -(kKeyRows ? lse_c[j] : lse_r[i])));
-          w[i][j] = ((vis >> j) & 1u) ? pe : __uint_as_float(kHidden);
-        }
-        if (kKeyRows)
-          *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = make_float4(w[i][0], w[i][1], w[i][2], w[i][3]);
-      }
-      if constexpr (kKeyRows) {
-        __syncwarp();
-        accumulate<DP, RT, true>(sW, sC2, row0, l16, acc2, finite);
-        __syncwarp();
-      }
-      {
-        float dp[RT][4];
-        scores<DP, RT>(sR2, sC2, row0, l16, dp);
+        __syncthreads();
+        const bool has_full = kKeyRows ? M::kHasQFullRange : M::kHasKFullRange;
+        const bool full = has_full && cg0 >= full_lo && cg0 + kCols <= full_hi && ncols >= kCols && rows_valid == kRows;
+        float w[RT][4];
+        scores<DP, RT>(sR1, sC1, row0, l16, w);
 #pragma unroll
         for (int i = 0; i < RT; ++i) {
+          uint32_t vis = 15u;
+          if (!full) vis = row0 + i < rows_in ? visible4<M, !kKeyRows>(rg0 + row0 + i, cg0, ncols, l16, n, g.margs) : 0u;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {  // a select, not the product with zero: dP and delta of a hidden pair may be anything
-            const float ds = w[i][j] * (dp[i][j] - (kKeyRows ? delta_c[j] : delta_r[i]));
-            w[i][j] = __float_as_uint(w[i][j]) == kHidden ? 0.f : ds;
+          for (int j = 0; j < 4; ++j) {
+            const float pe = exp2f(fmaf(w[i][j], c, -(kKeyRows ? lse_c[j] : lse_r[i])));
+            w[i][j] = ((vis >> j) & 1u) ? pe : 0.f;
           }
-          *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = make_float4(w[i][0], w[i][1], w[i][2], w[i][3]);
+          if (kKeyRows)
+            *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = make_float4(w[i][0], w[i][1], w[i][2], w[i][3]);
         }
+        auto hidden = [&](int i, int kx) {
+          const int r = rg0 + row0 + i, cc = cg0 + kx;
+          return row0 + i >= rows_valid || kx >= ncols || !(kKeyRows ? M::mask(cc, r, n, g.margs) : M::mask(r, cc, n, g.margs));
+        };
+        if constexpr (kKeyRows) {
+          __syncwarp();
+          accumulate<DP, RT>(sW, sC2, row0, l16, acc2, careful, [&](int i, int kx, float) { return hidden(i, kx); });
+          __syncwarp();
+        }
+        {
+          float dp[RT][4];
+          scores<DP, RT>(sR2, sC2, row0, l16, dp);
+#pragma unroll
+          for (int i = 0; i < RT; ++i) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[i][j] *= dp[i][j] - (kKeyRows ? delta_c[j] : delta_r[i]);  // hidden pairs: 0 * anything
+            *reinterpret_cast<float4*>(sW + (row0 + i) * kCols + 4 * (l16 ^ swz(row0 + i))) = make_float4(w[i][0], w[i][1], w[i][2], w[i][3]);
+          }
+        }
+        __syncwarp();
+        accumulate<DP, RT>(sW, sC1, row0, l16, acc1, careful, [&](int i, int kx, float wk) { return wk == 0.f || hidden(i, kx); });
+        __syncwarp();
       }
-      __syncwarp();
-      accumulate<DP, RT>(sW, sC1, row0, l16, acc1, finite);
-      __syncwarp();
     }
+    const bool nan = any_nan<DP>(acc1) || (kKeyRows && any_nan<DP>(acc2));
+    if (careful || !__syncthreads_or(nan)) break;
   }
   if constexpr (kKeyRows) {
 #pragma unroll
