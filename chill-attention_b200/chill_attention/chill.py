@@ -35,7 +35,7 @@ _BWD_PATHS = {"tensor_core": 0, "generic": 0}  # calls through the dispatcher op
 
 
 def backward_path_counts() -> dict:
-    """Copy of the per-process counters of backward calls served by the tensor-core and by the generic kernels."""
+    """Copy of the per-process counters of backward calls served by the tensor-core and by the CUDA-core kernels."""
     counts = dict(_BWD_PATHS)
     if _eager._extension is not None:
         tc, generic = _eager._extension.backward_counts()
@@ -47,7 +47,7 @@ def backward_path_counts() -> dict:
 def _backward_operand(do: torch.Tensor) -> torch.Tensor:
     """The incoming gradient as the kernels want it.  Autograd often hands over an expanded tensor (all strides 0
     after ``o.sum().backward()``) or a transposed view; the tensor-core kernels cannot describe those to TMA and
-    the call would otherwise be served by the ~1000x slower generic kernels.  One L x D copy fixes that (the
+    the call would otherwise be served by the CUDA-core kernels (about 30 TFLOP/s).  One L x D copy fixes that (the
     reference asserts ``do.stride(-1) == 1`` at this point, chill.py:270)."""
     return do if _cabi.tma_compatible(do) else do.contiguous()
 
@@ -55,7 +55,7 @@ def _backward_operand(do: torch.Tensor) -> torch.Tensor:
 def _tensor_core_operands(q, k, v):
     """16-bit q, k, v with a head dimension the tensor-core kernels serve, but in a memory layout TMA cannot describe
     (channel stride != 1, a broadcast dimension, rows not 16-byte aligned): one packing copy each puts them on the
-    tensor-core path, ~1000x faster than the generic kernels that would otherwise take the call.  The reference reads
+    tensor-core path instead of the CUDA-core kernels (about 30 TFLOP/s).  The reference reads
     such tensors through block pointers at full speed (chill_fwd.py:74-98); results are identical either way."""
     if q.dtype == torch.float32:
         return q, k, v

@@ -25,9 +25,9 @@
 //     S^T(u+2)
 // At D = 64 the dQ tile has columns of its own, so dP^T(u+1) does not wait for dQ(u) and its drain: it is issued first,
 // and the compute warps go from dS^T(u) to the exponentials of S^T(u+1) to dS^T(u+1) without a pause.
-// Q and dO of a stage complete on barriers of their own, and the compute warps walk heads and tiles without divisions (these
-// took about 500 of the 4400 clocks of a tile).  Together, fp16 (4,16,4096,64) full 905 -> 845 us, bf16 (8,16,4096,128) causal
-// 1281 -> 1266 us.  At D = 128 the period is set by the issuing thread: dQ, dK, the drain of dQ (about 1000 clocks from the
+// Q and dO of a stage complete on barriers of their own, and the compute warps walk heads and tiles without divisions (150 to
+// 250 of the 4000 to 4700 clocks of a tile).  Together, fp16 (4,16,4096,64) full 905 -> 845 us; bf16 (8,16,4096,128) causal
+// 1281 -> 1266 us, too little to show in a training step (2338 / 2348 us, runs of one side differ by 2 %).  At D = 128 the period is set by the issuing thread: dQ, dK, the drain of dQ (about 1000 clocks from the
 // commit until the columns are free), dP^T, dV, S^T.
 //
 // Roles (512 threads, register budgets re-balanced per warpgroup with setmaxnreg): warps 0-7 compute (thread
@@ -361,7 +361,7 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bool ok = true;
     // LSE / delta of this lane's two query columns, fetched one tile ahead (tile qi_next of head h_next).  The loaded
     // values are not touched until the next iteration (any dependent instruction here would stall on the global load).
-    // The walk over heads and tiles is incremental: the divisions it replaces took 500 of a tile's ~4400 clocks.
+    // The walk over heads and tiles is incremental (no divisions).
     int h_next = hk * G, qi_next = qt_lo;
     float nl_next[2], nd_next[2];
     auto fetch_rows = [&]() {

@@ -7,10 +7,11 @@
 // S^T 64 | dP^T 64 | dV 64 | dK 64 = 256 columns, shared memory K, V, two 64-query stages of [Q | dO] and the dS^T tile
 // (113 KB), so one CTA's fixed part and the latencies of its chain overlap the other's MMAs.
 // Chunkwise (128, 2) fp16 (4,32,16384,64): 1131 -> 968 us, window(16, 16) (8,12,2085,64): 124 -> 89 us against that kernel.
-// What bounds it now is the chain of each CTA (about 3400 clocks per step, of which 1000 exponentials): tensor pipe 24 % active,
-// shared-memory pipe 36 %, DRAM 31 %.  Leaving out the dQ reductions alone gains 8 %, the exponentials 5 %; persistent CTAs
-// that overlap one tile's stores with the next one's loads measured 1026 against 993 us, four compute warps instead of eight
-// 981 (and 95 against 89 us on the narrow window).
+// What bounds it now is the chain of each CTA (about 3400 clocks per step, of which 1000 exponentials): of the kernel's time on
+// (4,8,16384,64) the tensor pipe is active 24 %, the shared-memory pipe 36 %, instructions issue 51 %, DRAM delivers 2.3 TB/s.
+// Leaving out the dQ reductions alone gains 8 %, the exponentials 5 %.  Variants, both against 993 us of an earlier state of
+// this kernel: persistent CTAs that overlap one tile's stores with the next one's loads 1026 us; four compute warps instead of
+// eight 981 us, but 95 against 89 us on the narrow window.
 //
 // A step is 64 queries; two steps form a query tile, the unit of the dQ GEMM (M = 128 queries) and of the accumulator:
 //     S^T = K Q^T, dP^T = V dO^T, dV += P^T dO, dK += dS^T Q          every step

@@ -105,8 +105,8 @@ __global__ void __launch_bounds__(kGenericWarps * 32) delta_kernel(TRef o, TRef 
   if (lane == 0) delta[((long long)b * H + h) * Lq + row] = acc;
 }
 
-// Contiguous 16-bit rows of 64 or 128 channels: 8 lanes x 16 B (D=64) or 16 lanes x 16 B cover one
-// row, so a warp streams 4 or 2 rows per step.  Bandwidth-bound: 2 reads of B*H*L*D elements.
+// Contiguous 16-bit rows of 16, 32, 64 or 128 channels: 2, 4, 8 or 16 lanes x 16 B cover one
+// row, so a warp streams 16 to 2 rows per step.  Bandwidth-bound: 2 reads of B*H*L*D elements.
 template <typename T, int D>
 __global__ void __launch_bounds__(256) delta_rows16_kernel(const T* __restrict__ o, const T* __restrict__ d_o,
                                                            float* __restrict__ delta, long long o_sb, long long o_sh,

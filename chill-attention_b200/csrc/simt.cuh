@@ -19,11 +19,15 @@
 // bandwidth and RT = 4 three quarters of it.  Rows of 16-byte chunks are stored with the chunk index XORed by
 // (row / 4) % 8, which makes the lanes' reads of four consecutive rows conflict-free (measured: 3 wavefronts per read).
 //
-// Measured, fp32 full mask (2, 8, 1000, 64): forward 155 us, dK / dV and dQ together 459 us, i.e. 26 / 31 TFLOP/s of the
+// Measured, fp32 full mask (2, 8, 1000, 64): forward 143 us, dK / dV and dQ together 444 us, i.e. 29 / 32 TFLOP/s of the
 // 74 that 148 SMs issue (one warp per output row and 32 positions per step, the form before: 4831 and 17126 us, every
 // dot product re-reading its row of K or V from L1).  What is left is latency: 240 registers a thread leave eight
 // warps on an SM, which keep the FMA pipe 50 % busy; RT = 4 doubles the warps and their shared-memory reads per FMA
-// (forward 164-182 us).
+// (forward 164-182 against 155 us when it was tried).
+//
+// What a row may not see does not reach it, whatever the value: padding enters the tiles as zeros, and see accumulate for
+// what the mask hides.  The check of the accumulators and the second loop cost the backward 1 to 4 % (444 against 437 us) and
+// the forward nothing; a probe of every tile for NaN and Inf as it is loaded cost both 2 to 6 %.
 #pragma once
 #include "generic.cuh"
 #include "tc_common.cuh"
