@@ -5,7 +5,8 @@
 Each mask functor's tensor-core kernels and its CUDA-core kernels are translation units of their own
 (csrc/tc_inst.cu, csrc/simt_inst.cu with -DCHILL_INST_MASK=<functor>), compiled in parallel.
 ``build_library`` is also what ``chill_attention.custom`` calls to produce a private
-library for a user-defined mask functor.
+library for a user-defined mask functor.  The objects of the built-in functors, nine tenths of a build, are kept beside the
+library and linked into such private libraries as they are.
 """
 from __future__ import annotations
 
@@ -65,7 +66,7 @@ def build_library(out_path=None, custom_header=None, custom_functor=None, verbos
     os.makedirs(os.path.dirname(out_path), exist_ok=True)
     # CHILL_B200_NVCC_FLAGS: extra compiler flags, e.g. "-DCHILL_FWD_POLY_NUM=1 -DCHILL_FWD_POLY_DEN=4"
     defines, functors = os.environ.get("CHILL_B200_NVCC_FLAGS", "").split(), list(BUILTIN_FUNCTORS)
-    extra = tuple(defines)
+    extra = common = tuple(defines)
     if custom_header is not None:
         custom_header = os.path.abspath(custom_header)
         with open(custom_header, "rb") as f:
@@ -77,25 +78,38 @@ def build_library(out_path=None, custom_header=None, custom_functor=None, verbos
     if not force and os.path.exists(out_path) and os.path.exists(stamp) and open(stamp).read() == digest:
         return out_path
     obj_dir = os.path.join(os.path.dirname(out_path), "obj_" + os.path.basename(out_path))
-    os.makedirs(obj_dir, exist_ok=True)
-    nvcc = _nvcc()
-    jobs = [([nvcc] + NVCC_FLAGS + defines + ["-c", os.path.join(CSRC, src + ".cu"), "-o",
-                                               os.path.join(obj_dir, src + ".o")]) for src in ("chill_abi", "host_pipeline")]
+    kept_dir = os.path.join(LIB_DIR, "obj_builtin_" + _sources_digest(common)[:16])
+    for d in (obj_dir, kept_dir):
+        os.makedirs(d, exist_ok=True)
+    nvcc = [_nvcc()] + (["-Xptxas", "-v"] if verbose else []) + NVCC_FLAGS
+
+    def compile_unit(unit):
+        flags, src, obj = unit
+        if os.path.dirname(obj) == kept_dir and os.path.exists(obj) and not force:
+            return ""
+        part = f"{obj}.{os.getpid()}.o"  # a build that is cut off leaves no half-written object under the final name
+        out = _run(nvcc + flags + ["-c", os.path.join(CSRC, src), "-o", part])
+        os.replace(part, obj)
+        return out
+
+    units = [(defines, src + ".cu", os.path.join(obj_dir, src + ".o")) for src in ("chill_abi", "host_pipeline")]
     for fn in functors:
+        builtin = fn in BUILTIN_FUNCTORS
         for unit in ("tc", "simt"):
-            jobs.append([nvcc] + NVCC_FLAGS + defines + [f"-DCHILL_INST_MASK={fn}", "-c", os.path.join(CSRC, f"{unit}_inst.cu"),
-                                                          "-o", os.path.join(obj_dir, f"{unit}_{fn}.o")])
-    if verbose:
-        jobs = [j[:1] + ["-Xptxas", "-v"] + j[1:] for j in jobs]
-    with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
-        outs = list(ex.map(_run, jobs))
+            units.append((list(common if builtin else defines) + [f"-DCHILL_INST_MASK={fn}"], f"{unit}_inst.cu",
+                          os.path.join(kept_dir if builtin else obj_dir, f"{unit}_{fn}.o")))
+    with cf.ThreadPoolExecutor(max_workers=8) as ex:
+        outs = list(ex.map(compile_unit, units))
     if verbose:
         print("\n".join(outs))
-    objs = [j[j.index("-o") + 1] for j in jobs]
-    _run([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", out_path] + objs)
+    _run([_nvcc(), "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", out_path] + [obj for _, _, obj in units])
     with open(stamp, "w") as f:
         f.write(digest)
-    shutil.rmtree(obj_dir, ignore_errors=True)  # objects are not needed once linked
+    shutil.rmtree(obj_dir, ignore_errors=True)  # not needed once linked
+    if custom_header is None:
+        for name in os.listdir(LIB_DIR):  # objects of other sources or flags
+            if name.startswith("obj_builtin_") and os.path.join(LIB_DIR, name) != kept_dir:
+                shutil.rmtree(os.path.join(LIB_DIR, name), ignore_errors=True)
     return out_path
 
 

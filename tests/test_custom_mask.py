@@ -59,6 +59,32 @@ def test_custom_library_builds_and_exports(tmp_path):
     assert _cabi.load_library().chill_mask_traits(_cabi.MASK_CUSTOM) == -2  # the stock library has no custom functor
 
 
+def test_custom_library_reuses_the_objects_of_the_builtin_functors(tmp_path, monkeypatch):
+    """Only the functor's own kernels and the entry points are compiled for it; everything is linked.  (No compiler runs here.)"""
+    from chill_attention.custom import _build_module
+
+    build, commands = _build_module(), []
+
+    def run(cmd):
+        commands.append(cmd)
+        open(cmd[cmd.index("-o") + 1], "w").close()
+        return ""
+
+    monkeypatch.setattr(build, "LIB_DIR", str(tmp_path))
+    monkeypatch.setattr(build, "_run", run)
+    build.build_library()
+    assert len(commands) == 2 + 2 * 5 + 1
+    del commands[:]
+    build.build_library(out_path=str(tmp_path / "custom.so"), custom_header=HEADER, custom_functor="DilatedCausalMask")
+    compiled, link = [c for c in commands if "-c" in c], commands[-1]
+    assert sorted(f for c in compiled for f in c if f.startswith("-DCHILL_INST_MASK=")) == ["-DCHILL_INST_MASK=DilatedCausalMask"] * 2
+    assert len(compiled) == 4 and sum(f.endswith(".o") for f in link) == 2 + 2 * 6
+    del commands[:]
+    monkeypatch.setenv("CHILL_B200_NVCC_FLAGS", "-DCHILL_FWD_POLY_NUM=1")  # other flags, other objects
+    build.build_library()
+    assert len(commands) == 2 + 2 * 5 + 1
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype,D", [(torch.bfloat16, 128), (torch.float32, 32), (torch.float16, 256), (torch.bfloat16, 32)], ids=str)
 def test_custom_mask_on_gpu(dtype, D):
