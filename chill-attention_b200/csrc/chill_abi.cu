@@ -228,6 +228,31 @@ static uint32_t vec_bit(uint32_t bit, const void* p, const int64_t* st, int dtyp
   return (st[0] % 4 == 0 && st[1] % 4 == 0 && st[2] % 4 == 0) ? bit : 0;
 }
 
+// Whether an fp32 call of IEEE accuracy goes to the tensor cores with split operands (split.cuh): head dim <= 64, and enough
+// work, as steps of 128 queries x 64 keys times the channels the CUDA-core kernels would multiply, to make up for the longer
+// set-up; a single step per tile never does.  Forward, us, CUDA cores / split, full mask, head dim 64: (1,2,128) 8.6 / 14.3,
+// (1,8,256), 64 steps: 14.1 / 17.8, (8,8,128), 128 steps: 17.4 / 14.6, (1,1,2048), 512 steps: 90 / 72, (2,8,1000): 143 / 44,
+// (4,8,2048): 938 / 274; (8,16,64), one step each: 11.4 / 12.5; head dim 32 (2,4,1000): 62 / 41, with window(32, 0), 192 steps:
+// 13.5 / 16.3.  Backward: (1,4,257), 60 steps: 27 / 33, (1,8,256): 29.9 / 29.0, window(32, 0) (2,4,512), 96 steps: 30 / 26,
+// (2,8,1000): 442 / 135.
+static bool split_pays(const chill_shape& s, long long least) {
+  if (s.dtype != CHILL_F32 || s.D > 64 || s.D % 16 != 0 || (s.flags & CHILL_FLAG_FORCE_GENERIC)) return false;
+  long long total = 0;
+  int most = 0;
+  switch (s.mask.id) {
+    case CHILL_MASK_FULL: split_count_steps<FullMask>(to_geo(s), total, most); break;
+    case CHILL_MASK_CAUSAL: split_count_steps<CausalMask>(to_geo(s), total, most); break;
+    case CHILL_MASK_SLIDING: split_count_steps<SlidingWindowMask>(to_geo(s), total, most); break;
+    case CHILL_MASK_CHUNKWISE: split_count_steps<ChunkwiseMask>(to_geo(s), total, most); break;
+    case CHILL_MASK_PREFIXLM: split_count_steps<PrefixLMMask>(to_geo(s), total, most); break;
+#ifdef CHILL_CUSTOM_MASK
+    case CHILL_MASK_CUSTOM: split_count_steps<CHILL_CUSTOM_MASK>(to_geo(s), total, most); break;
+#endif
+    default: return false;
+  }
+  return most >= 2 && total * (s.D <= 32 ? 32 : 64) >= least;
+}
+
 static int fwd_generic(const chill_fwd_args& a, cudaStream_t st) {
   simt::FwdParams pp;
   FwdP& p = pp.f;
@@ -241,6 +266,15 @@ static int fwd_generic(const chill_fwd_args& a, cudaStream_t st) {
   pp.vec = vec_bit(simt::kVecQ, a.q, a.q_strides, dt, D) | vec_bit(simt::kVecK, a.k, a.k_strides, dt, D) |
            vec_bit(simt::kVecV, a.v, a.v_strides, dt, D) | vec_bit(simt::kVecO, a.o, a.o_strides, dt, D);
   int e = 0;
+  if (pp.vec == (simt::kVecQ | simt::kVecK | simt::kVecV | simt::kVecO) && split_pays(a.s, 8192)) {
+    split::FwdParams sp;
+    sp.f = p;
+    sp.status = device_status_ptr();
+    CHILL_MASK_SWITCH(a.s.mask.id, (e = split_launch_fwd<MaskT>(sp, st)))
+    if (e != 0) return cuda_fail((cudaError_t)e, "split_fwd launch");
+    g_launches += 1;
+    pp.repair = true;
+  }
   CHILL_MASK_SWITCH(a.s.mask.id, (e = simt_launch_fwd<MaskT>(pp, st)))
   if (e == 0) g_launches += 1;
   return e == 0 ? CHILL_OK : cuda_fail((cudaError_t)e, "fwd_generic launch");
@@ -421,6 +455,15 @@ static int bwd_generic(const chill_bwd_args& a, cudaStream_t st) {
            vec_bit(simt::kVecDq, a.dq, a.dq_strides, dt, D) | vec_bit(simt::kVecDk, a.dk, a.dk_strides, dt, D) |
            vec_bit(simt::kVecDv, a.dv, a.dv_strides, dt, D);
   int e = 0;
+  if (pp.vec == (255u & ~(uint32_t)simt::kVecO) && a.dk_part == nullptr && split_pays(a.s, 5120)) {
+    split::BwdParams sp;
+    sp.b = pp.b;
+    sp.status = device_status_ptr();
+    CHILL_MASK_SWITCH(a.s.mask.id, (e = split_launch_bwd<MaskT>(sp, bwd_which(a.s.flags), st)))
+    if (e != 0) return cuda_fail((cudaError_t)e, "split_bwd launch");
+    g_launches += 1;
+    pp.repair = true;
+  }
   CHILL_MASK_SWITCH(a.s.mask.id, (e = simt_launch_bwd<MaskT>(pp, bwd_which(a.s.flags), st)))
   if (e == 0) g_launches += 1;
   return e == 0 ? CHILL_OK : cuda_fail((cudaError_t)e, "bwd_generic launch");

@@ -1,7 +1,8 @@
 // CUDA-core kernels (fp32 arithmetic): any dtype, any head dim <= 256, any strides.
 //
-// They serve every call the tensor-core kernels cannot take: fp32 tensors with IEEE precision (the default for fp32),
-// 16-bit tensors whose layout TMA cannot describe, sm_scale <= 0.
+// They serve every call the tensor-core kernels cannot take: fp32 tensors with IEEE precision (the default for fp32) where
+// split.cuh does not pay (head dims above 64, little work) or cannot load them, 16-bit tensors whose layout TMA cannot
+// describe, sm_scale <= 0.  Behind split.cuh they repeat the rows it has marked (`repair`).
 //
 //   simt_fwd_kernel   O, LSE            (reference math: chill_attention/chill_fwd.py:188-359)
 //   simt_bwd_kernel   dK, dV and dQ     (chill_attention/chill_bwd_dkdv.py:15-277, chill_bwd_dq.py:15-229)
@@ -30,6 +31,7 @@
 // the forward nothing; a probe of every tile for NaN and Inf as it is loaded cost both 2 to 6 %.
 #pragma once
 #include "generic.cuh"
+#include "split.cuh"
 #include "tc_common.cuh"
 
 namespace chill {
@@ -43,11 +45,13 @@ struct BwdParams {
   int n_key_ctas;    // the first n_key_ctas CTAs compute dK / dV, the others dQ
   uint32_t vec;      // kVec*: tensors whose rows are read / written in 16-byte vectors (fp32 only)
   int dtype;
+  bool repair = false;  // only tiles with a row that split.cuh has marked
 };
 struct FwdParams {
   FwdP f;
   uint32_t vec;
   int dtype;
+  bool repair = false;
 };
 enum : uint32_t { kVecQ = 1, kVecK = 2, kVecV = 4, kVecO = 8, kVecDo = 16, kVecDq = 32, kVecDk = 64, kVecDv = 128 };
 
@@ -62,6 +66,16 @@ __device__ __forceinline__ void store_elem(void* p, long long i, int dtype, floa
   if (dtype == 0) static_cast<float*>(p)[i] = v;
   else if (dtype == 1) static_cast<__half*>(p)[i] = from_f<__half>(v);
   else static_cast<__nv_bfloat16*>(p)[i] = from_f<__nv_bfloat16>(v);
+}
+
+// Rows of a half-warp whose fp32 result carries the mark of a row that split.cuh left to these kernels: bit i = row0 + i.
+template <int RT>
+__device__ __forceinline__ uint32_t marked(const TRef& t, int b, int h, int row0, int end) {
+  uint32_t bits = 0;
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+    if (row0 + i < end && __float_as_uint(static_cast<const float*>(t.p)[b * t.sb + h * t.sh + (row0 + i) * t.sl]) == kRepairMark) bits |= 1u << i;
+  return bits;
 }
 
 __device__ __forceinline__ int swz(int row) { return (row >> 2) & 7; }
@@ -293,6 +307,11 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
   const int n = valid_len(g, b), D = g.D;
   const int qg0 = qb + g.q_off;
   const int rows_in = imin(kRows, g.Lq - qb);
+  uint32_t keep = ~0u;  // rows to store
+  if (pp.repair) {
+    keep = marked<RT>(p.o, b, h, qb + row0, g.Lq);
+    if (!__syncthreads_or(keep != 0)) return;
+  }
   int kt_lo = 0, kt_hi = 0, full_lo = 0, full_hi = 0;
   if (qg0 < n) {
     int lo, hi;
@@ -361,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const int row = qb + row0 + i;
-    if (row >= g.Lq) continue;
+    if (row >= g.Lq || !((keep >> i) & 1u)) continue;
     const bool valid = row + g.q_off < n;  // padded query rows: O = 0, LSE = 0
     const float inv = sum != 0.f ? 1.f / sum : 0.f;
     store_row<DP>(p.o.p, b * p.o.sb + h * p.o.sh + row * p.o.sl, p.o.sd, D, pp.dtype, pp.vec & kVecO, l16, acc[i], inv, valid);
@@ -398,6 +417,11 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
   const int hr = kKeyRows ? unit % g.Hkv : unit % g.H, b = kKeyRows ? unit / g.Hkv : unit / g.H;
   const int rb = rt * kRows, rg0 = rb + (kKeyRows ? g.k_off : g.q_off);
   const int rows_in = imin(kRows, (kKeyRows ? g.Lk : g.Lq) - rb);
+  uint32_t keep = ~0u;  // rows to store
+  if (pp.repair) {
+    keep = marked<RT>(kKeyRows ? p.dk : p.dq, b, hr, rb + row0, rb + rows_in);
+    if (!__syncthreads_or(keep != 0)) return;
+  }
   const int c_off = kKeyRows ? g.q_off : g.k_off, c_len = kKeyRows ? g.Lq : g.Lk;
   const int n = valid_len(g, b), D = g.D;
   int ct_lo = 0, ct_hi = 0, full_lo = 0, full_hi = 0;
@@ -506,7 +530,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       const int j = rb + row0 + i;
-      if (j >= g.Lk) continue;
+      if (j >= g.Lk || !((keep >> i) & 1u)) continue;
       const bool valid = row0 + i < rows_valid;
       store_row<DP>(p.dk.p, b * p.dk.sb + hr * p.dk.sh + j * p.dk.sl, p.dk.sd, D, pp.dtype, pp.vec & kVecDk, l16, acc1[i], g.scale, valid);
       store_row<DP>(p.dv.p, b * p.dv.sb + hr * p.dv.sh + j * p.dv.sl, p.dv.sd, D, pp.dtype, pp.vec & kVecDv, l16, acc2[i], 1.f, valid);
@@ -520,7 +544,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       const int row = rb + row0 + i;
-      if (row < g.Lq)
+      if (row < g.Lq && ((keep >> i) & 1u))
         store_row<DP>(p.dq.p, b * p.dq.sb + hr * p.dq.sh + row * p.dq.sl, p.dq.sd, D, pp.dtype, pp.vec & kVecDq, l16, acc1[i], g.scale,
                       row0 + i < rows_valid);
     }

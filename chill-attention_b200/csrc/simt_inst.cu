@@ -1,5 +1,6 @@
 // Instantiates the CUDA-core kernels for ONE mask functor: compile with -DCHILL_INST_MASK=<functor struct>
 #include "simt.cuh"
+#include "split.cuh"
 #include "tc_launch.h"
 
 #ifndef CHILL_INST_MASK
@@ -37,6 +38,7 @@ template <int DP>
 static int fwd_dim(const FwdParams& p, cudaStream_t st) {
   constexpr int RT = fwd_rows(DP);
   const Geo& g = p.f.g;
+  if (p.repair) return fwd_one<DP, RT>(p, st);
   const long long ctas = (long long)((g.Lq + 8 * RT - 1) / (8 * RT)) * g.H * g.B;
   if (2 * ctas < sm_count()) return fwd_one<DP, 2>(p, st);
   return fwd_one<DP, RT>(p, st);
@@ -62,6 +64,7 @@ static int bwd_one(BwdParams p, int which, cudaStream_t st) {
 template <int DP>
 static int bwd_dim(const BwdParams& p, int which, cudaStream_t st) {
   constexpr int RT = bwd_rows(DP);
+  if (p.repair) return bwd_one<DP, RT>(p, which, st);
   if constexpr (RT > 2) {
     const Geo& g = p.b.g;
     const long long ctas = (long long)((g.Lk + 8 * RT - 1) / (8 * RT)) * g.Hkv * g.B + (long long)((g.Lq + 8 * RT - 1) / (8 * RT)) * g.H * g.B;
@@ -71,6 +74,41 @@ static int bwd_dim(const BwdParams& p, int which, cudaStream_t st) {
 }
 
 }  // namespace simt
+
+template <>
+int split_launch_fwd<InstMask>(const split::FwdParams& p, cudaStream_t st) {
+  auto kern = split::split_fwd_kernel<InstMask>;
+  constexpr int smem = split::FwdSmem::kDynamic;
+  static_assert(smem <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
+  struct Tag {};
+  cudaError_t e = ensure_dynamic_smem<Tag>(kern, smem, /*prefer_max_carveout=*/true);
+  if (e != cudaSuccess) return (int)e;
+  const Geo& g = p.f.g;
+  kern<<<dim3((unsigned)((g.Lq + split::kRows - 1) / split::kRows), (unsigned)g.H, (unsigned)g.B), split::kFwdThreads, smem, st>>>(p);
+  return (int)cudaGetLastError();
+}
+
+template <>
+void split_count_steps<InstMask>(const Geo& g, long long& total, int& most) {
+  split::count_steps<InstMask>(g, total, most);
+}
+
+template <>
+int split_launch_bwd<InstMask>(split::BwdParams p, int which, cudaStream_t st) {
+  auto kern = split::split_bwd_kernel<InstMask>;
+  constexpr int smem = split::BwdSmem::kDynamic;
+  static_assert(smem <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
+  struct Tag {};
+  cudaError_t e = ensure_dynamic_smem<Tag>(kern, smem, /*prefer_max_carveout=*/true);
+  if (e != cudaSuccess) return (int)e;
+  const Geo& g = p.b.g;
+  const long long nk = (which & 1) ? (long long)((g.Lk + split::kRows - 1) / split::kRows) * g.Hkv * g.B : 0;
+  const long long nq = (which & 2) ? (long long)((g.Lq + split::kRows - 1) / split::kRows) * g.H * g.B : 0;
+  if (nk + nq > 0x7fffffffll) return (int)cudaErrorInvalidConfiguration;
+  p.n_key_ctas = (int)nk;
+  kern<<<(unsigned)(nk + nq), split::kBwdThreads, smem, st>>>(p);
+  return (int)cudaGetLastError();
+}
 
 template <>
 int simt_launch_fwd<InstMask>(const simt::FwdParams& p, cudaStream_t st) {

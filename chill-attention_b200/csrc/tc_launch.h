@@ -18,6 +18,10 @@ namespace simt {
 struct FwdParams;
 struct BwdParams;
 }  // namespace simt
+namespace split {
+struct FwdParams;
+struct BwdParams;
+}  // namespace split
 
 // Raises a kernel's dynamic shared-memory limit the first time the kernel is launched on a device.  The attribute
 // is per (kernel, device); the record of where it has been set is per call site (pass a distinct `Tag` per kernel)
@@ -56,6 +60,15 @@ template <class M>
 int simt_launch_fwd(const simt::FwdParams& p, cudaStream_t st);
 template <class M>
 int simt_launch_bwd(const simt::BwdParams& p, int which, cudaStream_t st);
+
+// fp32 on the tensor cores as three bf16 parts (split.cuh), head dim <= 64; the caller launches the CUDA-core kernel with
+// `repair` set behind it.
+template <class M>
+int split_launch_fwd(const split::FwdParams& p, cudaStream_t st);
+template <class M>
+void split_count_steps(const Geo& g, long long& total, int& most);
+template <class M>
+int split_launch_bwd(split::BwdParams p, int which, cudaStream_t st);
 
 // maps: Q, K, V, O.  Returns a cudaError_t cast to int.
 template <class M>

@@ -245,13 +245,15 @@ size_t chill_bwd_scratch_bytes(const chill_shape* s);
 size_t chill_bwd_dq_accum_bytes(const chill_shape* s);
 
 /* 1 if chill_fwd / chill_bwd would run the tcgen05 tensor-core kernels for these
- * arguments, 0 if the generic kernels, negative status if the arguments are invalid. */
+ * arguments, 0 if the generic kernels, negative status if the arguments are invalid.  fp32 in IEEE accuracy is "generic"
+ * whichever units compute it: large calls of head dim <= 64 split every operand into three bf16 parts for the tensor cores,
+ * with results at least as close to the exact ones. */
 int chill_fwd_uses_tensor_cores(const chill_fwd_args* a);
 int chill_bwd_uses_tensor_cores(const chill_bwd_args* a);
 
 /* Which kernels chill_bwd would launch for these arguments (host-only; pointers are looked at for their alignment), or a
  * negative status if the arguments are invalid. */
-#define CHILL_BWD_CUDA_CORES 0   /* simt.cuh */
+#define CHILL_BWD_CUDA_CORES 0   /* generic: simt.cuh, or split.cuh for large fp32 calls of head dim <= 64 */
 #define CHILL_BWD_TWO_KERNELS 1  /* dK / dV and dQ, bitwise reproducible: 16-bit without dq_accum, or one of the two alone */
 #define CHILL_BWD_SINGLE 2       /* one kernel, dQ summed in dq_accum */
 #define CHILL_BWD_SINGLE_PAIR 3  /* the same with two CTAs per SM: head dim <= 64, few query tiles per key tile */

@@ -1,0 +1,110 @@
+"""fp32 attention of IEEE accuracy on the tensor cores (csrc/split.cuh: every operand as three bf16 parts, head dim <= 64).
+
+A CTA owns 128 rows and takes the other axis in steps of 64 positions (the forward in two streams of alternate steps); the
+CUDA-core kernels (FLAG_FORCE_GENERIC) serve as the reference for accuracy and for non-finite values."""
+import pytest
+import torch
+
+from helpers import all_masks, big_masks, check_forward, check_grads, ensure_built, make_inputs, oracle_all
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    ensure_built()
+
+
+def run(q, k, v, do, mask, lens=None, split=True, blhd=False, **where):
+    """O, LSE, dQ, dK, dV through the C ABI, and which route was taken (the split kernels launch the CUDA-core ones behind them)."""
+    from chill_attention import _cabi
+
+    def place(t):
+        return t.transpose(1, 2).contiguous().cuda().transpose(1, 2) if blhd else t.cuda()
+
+    lib = _cabi.load_library()
+    q, k, v, do = (place(t) for t in (q, k, v, do))
+    lens = None if lens is None else lens.cuda()
+    o, dq, dk, dv = (torch.full_like(t, float("nan")) for t in (q, q, k, v))
+    lse, delta = (torch.empty(q.shape[:3], device="cuda") for _ in range(2))
+    shape = _cabi.make_shape(q, k, _cabi.BUILTIN_FUNCTOR_IDS[mask.cuda_functor], mask.constargs, lens, q.shape[-1] ** -0.5,
+                             flags=0 if split else _cabi.FLAG_FORCE_GENERIC, **where)
+    before = lib.chill_launch_count()
+    _cabi.forward(lib, q, k, v, o, lse, shape)
+    middle = lib.chill_launch_count()
+    _cabi.backward(lib, q, k, v, o, do, lse, delta, dq, dk, dv, shape)
+    routes = middle - before == 2, lib.chill_launch_count() - middle == 3
+    torch.cuda.synchronize()
+    assert lib.chill_read_device_status() == 0
+    return (o, lse, dq, dk, dv), routes
+
+
+@pytest.mark.parametrize("D", [16, 32, 64])
+@pytest.mark.parametrize("L", [65, 127, 128, 129, 192, 193, 320, 511])
+@pytest.mark.parametrize("mask_no", range(5))
+def test_tile_edges(mask_no, L, D):
+    mask = all_masks()[mask_no]
+    q, k, v, do = make_inputs(6, 24, 12, L, D, torch.float32, seed=L + D)
+    lens = torch.tensor([L, L // 2, 1, 0, L + 1, 64], dtype=torch.int32) if L % 2 else None
+    o_ref, lse_ref, *g_ref = oracle_all(mask, q, k, v, do, lens)
+    (o, lse, *grads), routes = run(q, k, v, do, mask, lens, blhd=L % 3 == 0)
+    assert routes == (True, True)
+    check_forward(o, lse, o_ref, lse_ref, lens, torch.float32)
+    check_grads(grads, g_ref, torch.float32, lens)
+
+
+@pytest.mark.parametrize("mask_no", range(7))
+def test_no_further_from_the_exact_result_than_rounded_fma_chains(mask_no):
+    """N(0, 1) inputs: each result at most as far from the 64-bit one as the CUDA-core kernels' (measured 0.3 to 0.95 of it)."""
+    mask = big_masks()[mask_no]
+    for L, D in ((700, 64), (500, 32)):
+        inputs = make_inputs(2, 16, 8, L, D, torch.float32, seed=L)
+        exact = oracle_all(mask, *inputs)
+        mine, routes = run(*inputs, mask)
+        fma, _ = run(*inputs, mask, split=False)
+        assert routes == (True, True)
+        for name, a, b, r in zip(("o", "lse", "dq", "dk", "dv"), mine, fma, exact):
+            if name != "lse":
+                assert (a.cpu().double() - r).norm() <= (b.cpu().double() - r).norm(), name
+
+
+def test_sequence_shard():
+    """Global offsets: queries 100.. of the sequence against keys 150.., rows of the shard that see none of its keys."""
+    import chill_attention as ca
+
+    mask, L = ca.SlidingWindowChillMask(90, 20), 400
+    q, k, v, do = make_inputs(4, 16, 8, L, 64, torch.float32, seed=5)
+    where = dict(q_offset=100, k_offset=150, seq_len=900)
+    a, routes = run(q, k, v, do, mask, **where)
+    b, _ = run(q, k, v, do, mask, split=False, **where)
+    assert routes == (True, True)
+    assert torch.equal(torch.isfinite(a[1]), torch.isfinite(b[1])) and not torch.isfinite(a[1]).all()
+    for x, y in zip((a[0], *a[2:]), (b[0], *b[2:])):
+        assert (x - y).norm() <= 2e-6 * y.norm()  # each within 1e-6 of the exact result
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), -float("inf"), 3.4e38], ids=str)
+@pytest.mark.parametrize("where", ["q", "k", "v", "do"])
+@pytest.mark.parametrize("D", [32, 64])
+def test_values_bf16_cannot_hold(D, where, value):
+    """The same results, non-finite ones included, as the CUDA-core kernels; bitwise those without the value out of its reach."""
+    import chill_attention as ca
+
+    mask, L, pos, ch = ca.SlidingWindowChillMask(40, 30), 330, 200, 3
+    clean = make_inputs(4, 16, 16, L, D, torch.float32, seed=D)
+    dirty = [t.clone() for t in clean]
+    dirty["q k v do".split().index(where)][:, 3:, pos, ch] = value
+    base, routes = run(*clean, mask)
+    a, _ = run(*dirty, mask)
+    b, _ = run(*dirty, mask, split=False)
+    assert routes == (True, True)
+    for name, x, y in zip(("o", "lse", "dq", "dk", "dv"), a, b):
+        assert torch.equal(torch.isnan(x), torch.isnan(y)), name
+        fin = torch.isfinite(y)
+        assert torch.equal(x[~fin].nan_to_num(7.0), y[~fin].nan_to_num(7.0)), name
+        assert ((x[fin].double() - y[fin].double()).abs() <= 1e-5 * y[fin].double().abs().max()).all(), name
+    see = mask.make_mask(L, device="cpu")
+    rows = see[:, pos] if where in "kv" else torch.arange(L) == pos
+    keys = see[rows].any(0)
+    for x, y, hit in zip(a, base, (rows, rows, rows, keys, keys)):
+        assert torch.equal(x[:, :, ~hit.to(x.device)], y[:, :, ~hit.to(x.device)])
