@@ -9,12 +9,21 @@
 //   kWideDQ  one CTA per (batch, head, 128 queries):   S = Q K^T,   dP = dO V^T,     W = P (dP - delta),     dQ += W K
 //
 // with P = 2^(S c - LSE) from the stored LSE (no running maximum).  The "row" operands (K / V, resp. Q / dO: 64 KB
-// each) stay in shared memory, the other axis streams through in tiles of 64 positions (one stage: 2 x 32 KB; the
-// tile that only a score GEMM reads is refilled while the step is still running), clipped by the mask functor's
-// range function.  Roles as in fwd_tc.cuh: warps 0-3 own one tile row each per thread and turn the fp32 scores in
-// TMEM into the 16-bit W (written over the scores, A operand of the accumulating GEMM), warp 4 is the TMA producer,
-// warp 5 owns TMEM and issues the MMAs.
-// TMEM columns: [0,64) S (W over its first 32), [64,128) dP, [128,384) accumulator.
+// each) stay in shared memory, the other axis streams through in tiles of 64 positions, clipped by the mask functor's
+// range function.  Two buffers of scores in TMEM and two stages of the "late" tile, which the accumulating GEMM reads (the
+// "early" one, read by a score GEMM only, has what shared memory leaves: one stage, for dV two), let the issuing thread run
+//     scores(j + 1)   accumulate(j)   scores(j + 2) ...
+// so the elementwise work of a step hides behind the scores of the next one and the loads behind both.  Roles: warps 0-7 own one
+// tile row per thread and one half of the 64 positions and turn the fp32 scores in TMEM into the 16-bit W (written over the
+// scores that the same thread has read, A operand of the accumulating GEMM), warp 8 is the TMA producer, warp 9 owns TMEM and
+// issues the MMAs.
+// TMEM columns: [0,128) two buffers of S (W over them), [128,256) of dP, [256,512) accumulator.
+//
+// Measured (causal bf16 (2,16,4096,256), dV / dK / dQ in us): 338 / 522 / 558 with one stage, one buffer of scores and four
+// elementwise warps (each step a chain of load, scores, elementwise, accumulate), 250 / 403 / 436 with two, 253 / 378 / 432 with
+// eight warps as well, which masked tiles need (chunkwise(100, 3) (2,8/4,2048): all three 580 -> 521 -> 323).  What bounds them now:
+// the streamed tiles leave the L2 at 5.6 (dK) to 8.5 TB/s (dV), and a score MMA with N = 64 reads 6 KB of shared memory in its 48
+// clocks.
 // Reference math: chill_attention/chill_bwd_dkdv.py:347-508, chill_bwd_dq.py:300-394.
 #pragma once
 #include "bwd_tc.cuh"
@@ -23,36 +32,37 @@ namespace chill {
 namespace tc {
 
 enum : int { kWideDV = 0, kWideDK = 1, kWideDQ = 2 };
-constexpr int kWideThreads = 256;  // warps 0-3 elementwise + epilogue, 4 TMA producer, 5 MMA issuer, 6-7 idle
-constexpr int kWideComputeRegs = 200, kWideOtherRegs = 56;  // 128 * 200 + 128 * 56 = 256 * 128
+constexpr int kWideThreads = 384;  // warps 0-7 elementwise + epilogue, 8 TMA producer, 9 MMA issuer, 10-11 idle
 
-template <int D>
+template <int D, int MODE>
 struct WideSmem {
   static constexpr int kRowBytes = kTile * D * 2;      // a 128-row operand
   static constexpr int kColBytes = kWideCols * D * 2;  // a 64-row streamed tile
+  static constexpr int kEarly = MODE == kWideDV ? 2 : 1;  // stages of the tile that only a score GEMM reads
   static constexpr int kR1 = 0;
   static constexpr int kR2 = kR1 + kRowBytes;
-  static constexpr int kC1 = kR2 + kRowBytes;
-  static constexpr int kC2 = kC1 + kColBytes;
-  static constexpr int kVec = kC2 + kColBytes;         // per warp: -LSE and -delta of the 64 streamed columns
-  static constexpr int kBars = kVec + 4 * 2 * kWideCols * 4;
-  static constexpr int kNumBars = 8;
+  static constexpr int kE = MODE == kWideDV ? kR2 : kR2 + kRowBytes;
+  static constexpr int kL = kE + kEarly * kColBytes;   // two stages of the tile the accumulating GEMM reads
+  static constexpr int kVec = kL + 2 * kColBytes;      // per warp: -LSE and -delta of 32 streamed columns
+  static constexpr int kBars = kVec + 8 * 2 * 32 * 4;
+  static constexpr int kNumBars = 14;
   static constexpr int kMisc = kBars + 8 * kNumBars;
   static constexpr int kTotal = kMisc + 16;
-  static constexpr int kDynamic = kTotal + 1024;
+  // 1 KB for aligning the base by hand, or what is left of it (dynamic shared memory starts aligned as a rule)
+  static constexpr int kDynamic = kTotal + 1024 <= 232448 ? kTotal + 1024 : 232448;
 };
 
-enum : int { kStWideProducer = 501, kStWideMma = 502, kStWideCompute = 503, kStWideEpilogue = 504 };
+enum : int { kStWideProducer = 501, kStWideMma = 502, kStWideCompute = 503, kStWideEpilogue = 504, kStWideAlign = 505 };
 
 // maps: R1, R2 = 128-row boxes of the row operands; C1, C2 = 64-row boxes of the streamed operands; OUT = 128-row
 // box of the gradient written.  kWideDV: R1 = K, (R2 unused), C1 = Q, C2 = dO, OUT = dV.  kWideDK: R1 = K, R2 = V,
 // C1 = Q, C2 = dO, OUT = dK.  kWideDQ: R1 = Q, R2 = dO, C1 = K, C2 = V, OUT = dQ.
 template <typename T, int D, class M, int MODE>
-__global__ void __launch_bounds__(kWideThreads, 2)  // 2: 128 registers at launch, the pool setmaxnreg redistributes
+__global__ void __launch_bounds__(kWideThreads, 1)
 bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant__ CUtensorMap tmR2,
                 const __grid_constant__ CUtensorMap tmC1, const __grid_constant__ CUtensorMap tmC2,
                 const __grid_constant__ CUtensorMap tmOut, BwdTcParams p) {
-  using L = WideSmem<D>;
+  using L = WideSmem<D, MODE>;
   constexpr bool kKeyRows = MODE != kWideDQ;   // tile rows are keys (dV, dK) or queries (dQ)
   constexpr bool kTwoScores = MODE != kWideDV;  // dP is needed as well
   constexpr int CT = kWideCols;
@@ -104,35 +114,37 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t sR1 = base + L::kR1, sR2 = base + L::kR2, sC1 = base + L::kC1, sC2 = base + L::kC2;
-  float* vec_s = reinterpret_cast<float*>(gen_base + L::kVec);  // [warp][0: -lse, 1: -delta][64]
+  if (base + L::kTotal > smem_u32(smem_raw) + L::kDynamic) {  // the base was not aligned: nothing is computed
+    if (threadIdx.x == 0) atomicCAS(p.status, 0, kStWideAlign);
+    return;
+  }
+  const uint32_t sR1 = base + L::kR1, sR2 = base + L::kR2, sE = base + L::kE, sL = base + L::kL;
   const uint32_t bars = base + L::kBars;
-  // The two streamed tiles have different lifetimes: the "early" one (Q for dV, dO / V for dK / dQ) is only read by
-  // a score GEMM and can be refilled while the step is still running; the "late" one is the B operand of the
-  // accumulating GEMM.  e_done = the early tile's GEMM has finished (for dV that is also "scores ready").
-  const uint32_t bar_r_full = bars, bar_ce_full = bars + 8, bar_cl_full = bars + 16, bar_e_done = bars + 24,
-                 bar_cl_empty = bars + 32, bar_t_full = bars + 40, bar_w_full = bars + 48, bar_acc_full = bars + 56;
-  const uint32_t sEarly = MODE == kWideDV ? sC1 : sC2, sLate = MODE == kWideDV ? sC2 : sC1;
+  // "Early" tile: Q for dV, dO / V for dK / dQ, read by one score GEMM (e_done: that GEMM has finished).  "Late" tile: also, or
+  // only, the B operand of the accumulating GEMM.  Per stage + 8 s.  t_full: the scores of a step are there.
+  const uint32_t bar_r_full = bars, bar_acc_full = bars + 8, bar_e_full = bars + 16, bar_e_done = bars + 32, bar_l_full = bars + 48,
+                 bar_l_empty = bars + 64, bar_t_full = bars + 80, bar_w_full = bars + 96;
+  constexpr int NE = L::kEarly;
   const CUtensorMap* tmEarly = MODE == kWideDV ? &tmC1 : &tmC2;
   const CUtensorMap* tmLate = MODE == kWideDV ? &tmC2 : &tmC1;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen_base + L::kMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_base + L::kMisc + 4);
   const Guard guard{p.status, abort_flag};
-  // streamed tile `it`: head and first local position
-  auto col_head = [&](int it) { return kKeyRows ? hk * G + it / n_ct : hk; };
-  auto col_pos = [&](int it) { return (ct_lo + it % n_ct) * CT; };
+  const int col_head0 = kKeyRows ? hk * G : hk;  // head of the first streamed tile
 
-  if (warp == 4) {
+  if (warp == 8) {
     if (lane == 0) {
       *abort_flag = 0;
       mbar_init(bar_r_full, 1);
-      mbar_init(bar_ce_full, 1);
-      mbar_init(bar_cl_full, 1);
-      mbar_init(bar_e_done, 1);
-      mbar_init(bar_cl_empty, 1);
-      mbar_init(bar_t_full, 1);
-      mbar_init(bar_w_full, 4);
       mbar_init(bar_acc_full, 1);
+      for (int s = 0; s < 2; ++s) {
+        mbar_init(bar_e_full + 8 * s, 1);
+        mbar_init(bar_e_done + 8 * s, 1);
+        mbar_init(bar_l_full + 8 * s, 1);
+        mbar_init(bar_l_empty + 8 * s, 1);
+        mbar_init(bar_t_full + 8 * s, 1);
+        mbar_init(bar_w_full + 8 * s, 8);
+      }
       fence_barrier_init();
       fence_proxy_async_smem();
       mbar_arrive_expect_tx(bar_r_full, (kTwoScores ? 2 : 1) * L::kRowBytes);
@@ -140,14 +152,8 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
         tma_load_4d(sR1 + c * kChunkBytes, &tmR1, bar_r_full, c * 64, rb, hr, b);
         if (kTwoScores) tma_load_4d(sR2 + c * kChunkBytes, &tmR2, bar_r_full, c * 64, rb, hr, b);
       }
-      mbar_arrive_expect_tx(bar_ce_full, L::kColBytes);
-      for (int c = 0; c < kChunks; ++c)
-        tma_load_4d(sEarly + c * kColChunkBytes, tmEarly, bar_ce_full, c * 64, col_pos(0), col_head(0), b);
-      mbar_arrive_expect_tx(bar_cl_full, L::kColBytes);
-      for (int c = 0; c < kChunks; ++c)
-        tma_load_4d(sLate + c * kColChunkBytes, tmLate, bar_cl_full, c * 64, col_pos(0), col_head(0), b);
     }
-  } else if (warp == 5) {
+  } else if (warp == 9) {
     tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_slot)), 512);
     tmem_relinquish();
   }
@@ -155,42 +161,46 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem, tdP = tmem + CT, tAcc = tmem + 2 * CT;
+  // two buffers of scores: + CT per buffer
+  const uint32_t tS = tmem, tdP = tmem + 2 * CT, tAcc = tmem + 4 * CT;
 
-  if (warp == 4) {
-    reg_dealloc<kWideOtherRegs>();
+  if (warp == 8) {
     // ------------------------------------------------------------------- TMA producer
     if (lane == 0) {
       bool ok = true;
-      for (int it = 1; it < n_it && ok; ++it) {  // tile 0 was issued during set-up
-        const uint32_t prev = (uint32_t)(it - 1) & 1u;
-        ok = mbar_wait(bar_e_done, prev, guard, kStWideProducer);
+      int ct = ct_lo, hc = col_head0;
+      for (int it = 0; it < n_it && ok; ++it) {
+        const uint32_t es = (uint32_t)(it % NE), ls = (uint32_t)it & 1u;
+        ok = it < NE || mbar_wait(bar_e_done + 8 * es, (uint32_t)(it / NE - 1) & 1u, guard, kStWideProducer);
         if (!ok) break;
-        mbar_arrive_expect_tx(bar_ce_full, L::kColBytes);
+        mbar_arrive_expect_tx(bar_e_full + 8 * es, L::kColBytes);
         for (int c = 0; c < kChunks; ++c)
-          tma_load_4d(sEarly + c * kColChunkBytes, tmEarly, bar_ce_full, c * 64, col_pos(it), col_head(it), b);
-        ok = mbar_wait(bar_cl_empty, prev, guard, kStWideProducer);
+          tma_load_4d(sE + es * L::kColBytes + c * kColChunkBytes, tmEarly, bar_e_full + 8 * es, c * 64, ct * CT, hc, b);
+        ok = it < 2 || mbar_wait(bar_l_empty + 8 * ls, (uint32_t)((it >> 1) - 1) & 1u, guard, kStWideProducer);
         if (!ok) break;
-        mbar_arrive_expect_tx(bar_cl_full, L::kColBytes);
+        mbar_arrive_expect_tx(bar_l_full + 8 * ls, L::kColBytes);
         for (int c = 0; c < kChunks; ++c)
-          tma_load_4d(sLate + c * kColChunkBytes, tmLate, bar_cl_full, c * 64, col_pos(it), col_head(it), b);
+          tma_load_4d(sL + ls * L::kColBytes + c * kColChunkBytes, tmLate, bar_l_full + 8 * ls, c * 64, ct * CT, hc, b);
+        if (++ct == ct_hi) {
+          ct = ct_lo;
+          ++hc;
+        }
       }
       if (!ok) {
         const uint64_t t0 = globaltimer_ns();
         while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
       }
     }
-  } else if (warp == 5) {
-    reg_dealloc<kWideOtherRegs>();
+  } else if (warp == 9) {
     // --------------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc<T>(kTile, CT, false, false);
       constexpr uint32_t idesc_acc = make_idesc<T>(kTile, D, false, true);  // A from TMEM, B MN-major
       constexpr uint32_t hi_k = desc_hi_sw128(1024);
       const uint32_t r1_lo = desc_lo_sw128(sR1, 16), r2_lo = desc_lo_sw128(sR2, 16);
-      const uint32_t c1_lo = desc_lo_sw128(sC1, 16), c2_lo = desc_lo_sw128(sC2, 16);
-      // the streamed tile that multiplies W: dO for dV, Q for dK, K for dQ; MN-major, channel blocks one chunk apart
-      const uint32_t x_lo = desc_lo_sw128(MODE == kWideDV ? sC2 : sC1, kColChunkBytes);
+      const uint32_t e_lo = desc_lo_sw128(sE, 16), l_lo = desc_lo_sw128(sL, 16);
+      const uint32_t x_lo = desc_lo_sw128(sL, kColChunkBytes);  // MN-major, channel blocks one chunk apart
+      constexpr uint32_t kStage = L::kColBytes / 16;
       bool ok = mbar_wait(bar_r_full, 0, guard, kStWideMma);
       auto score = [&](uint32_t t_dst, uint32_t r_lo, uint32_t c_lo) {  // rows x 64 positions, contraction over D
 #pragma unroll
@@ -198,40 +208,43 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
           mma_ss_lh(t_dst, r_lo + kmajor_step(kk), c_lo + (uint32_t)((kk / 4) * (kColChunkBytes / 16) + (kk % 4) * 2), hi_k,
                     idesc_s, kk > 0 ? 1u : 0u);
       };
-      for (int it = 0; it < n_it && ok; ++it) {
-        const uint32_t par = (uint32_t)it & 1u;
-        // the GEMM that reads the early tile: S for dV, dP for dK / dQ
-        ok = mbar_wait(bar_ce_full, par, guard, kStWideMma);
-        if (!ok) break;
+      // Scores of step `it` into buffer it % 2: over W and dP of step it - 2, whose accumulating GEMM was issued before.
+      auto scores = [&](int it) -> bool {
+        const uint32_t es = (uint32_t)(it % NE), buf = (uint32_t)it & 1u;
+        if (!mbar_wait(bar_e_full + 8 * es, (uint32_t)(it / NE) & 1u, guard, kStWideMma)) return false;
         tc_fence_after();
-        if (MODE == kWideDV) score(tS, r1_lo, c1_lo);
-        else score(tdP, r2_lo, c2_lo);
-        mma_commit(bar_e_done);
-        ok = mbar_wait(bar_cl_full, par, guard, kStWideMma);
-        if (!ok) break;
-        tc_fence_after();
+        if (MODE == kWideDV) score(tS + buf * CT, r1_lo, e_lo + es * kStage);
+        else score(tdP + buf * CT, r2_lo, e_lo + es * kStage);
+        mma_commit(bar_e_done + 8 * es);
         if (kTwoScores) {
-          score(tS, r1_lo, c1_lo);
-          mma_commit(bar_t_full);
+          if (!mbar_wait(bar_l_full + 8 * buf, (uint32_t)(it >> 1) & 1u, guard, kStWideMma)) return false;
+          tc_fence_after();
+          score(tS + buf * CT, r1_lo, l_lo + buf * kStage);
         }
-        ok = mbar_wait(bar_w_full, par, guard, kStWideMma);
-        if (!ok) break;
+        mma_commit(bar_t_full + 8 * buf);
+        return true;
+      };
+      if (ok) ok = scores(0);
+      for (int it = 0; it < n_it && ok; ++it) {
+        const uint32_t buf = (uint32_t)it & 1u, par = (uint32_t)(it >> 1) & 1u;
+        if (it + 1 < n_it && !(ok = scores(it + 1))) break;  // runs during the elementwise work of step `it`
+        if (!kTwoScores && !(ok = mbar_wait(bar_l_full + 8 * buf, par, guard, kStWideMma))) break;
+        if (!(ok = mbar_wait(bar_w_full + 8 * buf, par, guard, kStWideMma))) break;
         tc_fence_after();
         // accumulator += W X: W (16-bit) from TMEM, 16 streamed positions = 8 columns of W and 2 KB of X per MMA
 #pragma unroll
         for (int kk = 0; kk < CT / 16; ++kk)
-          mma_ts_lh(tAcc, tS + kk * 8, x_lo + kk * 128, hi_k, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(bar_cl_empty);  // the late tile, S and dP may be overwritten
+          mma_ts_lh(tAcc, tS + buf * CT + (kk / 2) * 32 + (kk % 2) * 8, x_lo + buf * kStage + kk * 128, hi_k, idesc_acc, (it > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(bar_l_empty + 8 * buf);
       }
       if (ok) mma_commit(bar_acc_full);
     }
-  } else if (warp >= 6) {
-    reg_dealloc<kWideOtherRegs>();
-  } else {
-    reg_alloc<kWideComputeRegs>();
+  } else if (warp < 8) {
     // --------------------------------------------------------- elementwise + epilogue warps
-    const int r = warp * 32 + lane;  // row inside the tile == TMEM lane
-    const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
+    const int wg = warp >> 2;               // half of the streamed positions: [32 wg, 32 wg + 32)
+    const int r = (warp & 3) * 32 + lane;   // row inside the tile == TMEM lane
+    const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+    const int c0 = 32 * wg;
     const int rg = rg0 + r;  // global position of this thread's row (a key, or a query for kWideDQ)
     const bool row_ok = rg < n && r < rows_here;
     const float c = g.scale * kLog2e;
@@ -249,67 +262,75 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
       else M::k_full_range_for_q(rg0, kTile, n, g.margs, full_lo, full_hi);
     }
     bool ok = true;
+    float* vb = reinterpret_cast<float*>(gen_base + L::kVec) + warp * 64;  // warp-private copy: no barrier across warps inside the loop
+    int ct = ct_lo, hc = col_head0;
+    // LSE and delta of this lane's query column, fetched a step ahead
+    float nl_next = 0.f, nd_next = 0.f;
+    auto fetch_cols = [&]() {
+      const int q = imin(ct * CT + c0 + lane, g.Lq - 1);
+      nl_next = __ldg(p.lse + b * p.lse_sb + hc * p.lse_sh + q * p.lse_sl);
+      if (kTwoScores) nd_next = __ldg(p.delta + ((long long)b * g.H + hc) * g.Lq + q);
+    };
+    if (kKeyRows) fetch_cols();
     for (int it = 0; it < n_it; ++it) {
-      const uint32_t par = (uint32_t)it & 1u;
-      const int cpos = col_pos(it);  // first local position of the streamed tile
+      const uint32_t par = (uint32_t)(it >> 1) & 1u, buf = (uint32_t)it & 1u;
+      const int cpos = ct * CT;  // first local position of the streamed tile
       const int cg0 = cpos + (kKeyRows ? g.q_off : g.k_off);
       const int clim = imin(n - cg0, (kKeyRows ? g.Lq : g.Lk) - cpos);  // streamed positions >= clim do not exist
-      float* vb = vec_s + warp * (2 * CT);  // warp-private copy: no barrier across warps inside the loop
-      if (kKeyRows) {
-        // -LSE and -delta of the 64 query columns: two of each per lane
-        const int h = col_head(it);
-        __syncwarp();  // the previous step's reads of vb are done
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int cc = lane + 32 * e;
-          const int q = imin(cpos + cc, g.Lq - 1);
-          const float lv = p.lse[b * p.lse_sb + h * p.lse_sh + q * p.lse_sl];
-          vb[cc] = (lv == -CUDART_INF_F) ? 0.f : -lv;
-          vb[CT + cc] = -p.delta[((long long)b * g.H + h) * g.Lq + q];
-        }
-        __syncwarp();
+      if (++ct == ct_hi) {
+        ct = ct_lo;
+        ++hc;
       }
-      ok = mbar_wait(kTwoScores ? bar_t_full : bar_e_done, par, guard, kStWideCompute);
+      if (kKeyRows) {
+        __syncwarp();  // the previous step's reads of vb are done
+        vb[lane] = nl_next == -CUDART_INF_F ? 0.f : -nl_next;
+        if (kTwoScores) vb[32 + lane] = -nd_next;
+        __syncwarp();
+        if (it + 1 < n_it) fetch_cols();
+      }
+      ok = mbar_wait(bar_t_full + 8 * buf, par, guard, kStWideCompute);
       ok = __all_sync(0xffffffffu, ok);  // keep the warp converged for the .sync.aligned TMEM accesses
       if (!ok) break;
       tc_fence_after();
       const bool full = kHasFull && cg0 >= full_lo && cg0 + CT <= full_hi && clim >= CT;
-      uint32_t w[CT / 2];
+      uint32_t w[CT / 4];
       auto body = [&](auto masked_tag) {  // two copies: full tiles run without any mask arithmetic
         constexpr bool kMasked = decltype(masked_tag)::value;
+        uint32_t sreg[32], dreg[32];
+        tmem_ld32(tS + buf * CT + lane_sel + c0, sreg);
+        if (kTwoScores) tmem_ld32(tdP + buf * CT + lane_sel + c0, dreg);
+        tmem_wait_ld();
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {  // 32 streamed positions at a time
-          uint32_t sreg[32], dreg[32];
-          tmem_ld32(tS + lane_sel + half * 32, sreg);
-          if (kTwoScores) tmem_ld32(tdP + lane_sel + half * 32, dreg);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            float wv[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int cc = half * 32 + i + e;
-              const float nl = kKeyRows ? vb[cc] : row_nl;
-              const float nd = kKeyRows ? vb[CT + cc] : row_nd;
-              float pv = ex2(fmaf(__uint_as_float(sreg[i + e]), c, nl));
-              if (kMasked) {
-                const int qg = kKeyRows ? cg0 + cc : rg, kg = kKeyRows ? rg : cg0 + cc;
-                pv = (row_ok && cc < clim && M::mask(qg, kg, n, g.margs)) ? pv : 0.f;
-              }
-              if (kTwoScores) pv *= __uint_as_float(dreg[i + e]) + nd;
-              wv[e] = pv;
-            }
-            w[half * 16 + i / 2] = pack2<T>(wv[0], wv[1]);
+        for (int i = 0; i < 32; i += 4) {
+          float4 nl4 = make_float4(row_nl, row_nl, row_nl, row_nl), nd4 = make_float4(row_nd, row_nd, row_nd, row_nd);
+          if (kKeyRows) {
+            nl4 = *reinterpret_cast<const float4*>(vb + i);
+            if (kTwoScores) nd4 = *reinterpret_cast<const float4*>(vb + 32 + i);
           }
+          const float nl[4] = {nl4.x, nl4.y, nl4.z, nl4.w}, nd[4] = {nd4.x, nd4.y, nd4.z, nd4.w};
+          float wv[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int cc = c0 + i + e;
+            float pv = ex2(fmaf(__uint_as_float(sreg[i + e]), c, nl[e]));
+            if (kMasked) {
+              const int qg = kKeyRows ? cg0 + cc : rg, kg = kKeyRows ? rg : cg0 + cc;
+              pv = (row_ok && cc < clim && M::mask(qg, kg, n, g.margs)) ? pv : 0.f;
+            }
+            if (kTwoScores) pv *= __uint_as_float(dreg[i + e]) + nd[e];
+            wv[e] = pv;
+          }
+          w[i / 2] = pack2<T>(wv[0], wv[1]);
+          w[i / 2 + 1] = pack2<T>(wv[2], wv[3]);
         }
       };
       if (full) body(std::false_type{});
       else body(std::true_type{});
-      tmem_st32(tS + lane_sel, w);  // CT / 2 = 32 columns of 16-bit pairs over the scores just consumed
+      tmem_st16(tS + buf * CT + lane_sel + c0, w);  // 16 columns of 16-bit pairs over scores that only this thread reads
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_w_full);
+      if (lane == 0) mbar_arrive(bar_w_full + 8 * buf);
     }
 
     // ---- epilogue: accumulator (x sm_scale for dK, dQ) -> 16-bit -> swizzled shared memory (R1's buffer) -> TMA store
@@ -320,7 +341,7 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
     // optional un-rounded fp32 copy of this key row's dV / dK (first / last key rows of the call, see PartOut)
     float* part_row = kKeyRows ? p.part.row(MODE == kWideDV ? p.part.dv : p.part.dk, b, hr, rb + r, g.Lk) : nullptr;
 #pragma unroll 1
-    for (int q4 = 0; q4 < D / 32; ++q4) {
+    for (int q4 = wg * (D / 64); q4 < (wg + 1) * (D / 64); ++q4) {
       uint32_t acc[32];
       if (ok) {
         tmem_ld32(tAcc + lane_sel + q4 * 32, acc);
@@ -330,7 +351,7 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
       if (part_row != nullptr) store_part32(part_row + q4 * 32, acc, mul, ok && row_ok);
     }
     fence_proxy_async_smem();
-    named_bar_sync(1, 128);
+    named_bar_sync(1, 256);
     if (threadIdx.x == 0) {
       for (int cc = 0; cc < kChunks; ++cc) tma_store_4d(&tmOut, sR1 + cc * kChunkBytes, cc * 64, rb, hr, b);
       tma_store_commit();
@@ -340,21 +361,21 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 5) tmem_dealloc(tmem, 512);
+  if (warp == 9) tmem_dealloc(tmem, 512);
 }
 
 // maps: 0 Q128, 1 K128, 2 V128, 3 dO128 (128-row boxes), 4 Q64, 5 K64, 6 V64, 7 dO64 (64-row boxes), 8 dQ, 9 dK, 10 dV
 template <typename T, class M>
 int launch_bwd_wide(const CUtensorMap* maps, const BwdTcParams& p, cudaStream_t st) {
   constexpr int D = 256;
-  constexpr int smem = WideSmem<D>::kDynamic;
-  static_assert(smem <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
+  static_assert(WideSmem<D, kWideDK>::kDynamic <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
   const Geo& g = p.g;
   const unsigned key_ctas = (unsigned)(((g.Lk + kTile - 1) / kTile) * g.Hkv * g.B);
   const unsigned query_ctas = (unsigned)(((g.Lq + kTile - 1) / kTile) * g.H * g.B);
   cudaError_t e;
   {
     auto kern = bwd_wide_kernel<T, D, M, kWideDV>;
+    constexpr int smem = WideSmem<D, kWideDV>::kDynamic;
     struct Tag {};
     if ((e = ensure_dynamic_smem<Tag>(kern, smem)) != cudaSuccess) return (int)e;
     kern<<<key_ctas, kWideThreads, smem, st>>>(maps[1], maps[2], maps[4], maps[7], maps[10], p);
@@ -362,6 +383,7 @@ int launch_bwd_wide(const CUtensorMap* maps, const BwdTcParams& p, cudaStream_t 
   }
   {
     auto kern = bwd_wide_kernel<T, D, M, kWideDK>;
+    constexpr int smem = WideSmem<D, kWideDK>::kDynamic;
     struct Tag {};
     if ((e = ensure_dynamic_smem<Tag>(kern, smem)) != cudaSuccess) return (int)e;
     kern<<<key_ctas, kWideThreads, smem, st>>>(maps[1], maps[2], maps[4], maps[7], maps[9], p);
@@ -369,6 +391,7 @@ int launch_bwd_wide(const CUtensorMap* maps, const BwdTcParams& p, cudaStream_t 
   }
   {
     auto kern = bwd_wide_kernel<T, D, M, kWideDQ>;
+    constexpr int smem = WideSmem<D, kWideDQ>::kDynamic;
     struct Tag {};
     if ((e = ensure_dynamic_smem<Tag>(kern, smem)) != cudaSuccess) return (int)e;
     kern<<<query_ctas, kWideThreads, smem, st>>>(maps[0], maps[3], maps[5], maps[6], maps[8], p);
