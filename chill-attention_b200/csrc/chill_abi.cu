@@ -175,7 +175,8 @@ static int make_map(CUtensorMap* m, const void* p, const int64_t* st, int B, int
 #define CHILL_CUSTOM_CASE(CALL)
 #endif
 
-#define CHILL_MASK_SWITCH(ID, CALL)                                        \
+#define CHILL_MASK_SWITCH(ID, CALL) CHILL_MASK_SWITCH_OR(ID, CALL, return CHILL_E_UNSUPPORTED)
+#define CHILL_MASK_SWITCH_OR(ID, CALL, OTHERWISE)                          \
   switch (ID) {                                                            \
     case CHILL_MASK_FULL: { using MaskT = FullMask; CALL; break; }         \
     case CHILL_MASK_CAUSAL: { using MaskT = CausalMask; CALL; break; }     \
@@ -183,7 +184,7 @@ static int make_map(CUtensorMap* m, const void* p, const int64_t* st, int B, int
     case CHILL_MASK_CHUNKWISE: { using MaskT = ChunkwiseMask; CALL; break; } \
     case CHILL_MASK_PREFIXLM: { using MaskT = PrefixLMMask; CALL; break; } \
     CHILL_CUSTOM_CASE(CALL)                                                \
-    default: return CHILL_E_UNSUPPORTED;                                   \
+    default: OTHERWISE;                                                    \
   }
 
 #define CHILL_DTYPE_SWITCH(DT, CALL)                                  \
@@ -239,17 +240,7 @@ static bool split_pays(const chill_shape& s, long long least) {
   if (s.dtype != CHILL_F32 || s.D > 64 || s.D % 16 != 0 || (s.flags & CHILL_FLAG_FORCE_GENERIC)) return false;
   long long total = 0;
   int most = 0;
-  switch (s.mask.id) {
-    case CHILL_MASK_FULL: split_count_steps<FullMask>(to_geo(s), total, most); break;
-    case CHILL_MASK_CAUSAL: split_count_steps<CausalMask>(to_geo(s), total, most); break;
-    case CHILL_MASK_SLIDING: split_count_steps<SlidingWindowMask>(to_geo(s), total, most); break;
-    case CHILL_MASK_CHUNKWISE: split_count_steps<ChunkwiseMask>(to_geo(s), total, most); break;
-    case CHILL_MASK_PREFIXLM: split_count_steps<PrefixLMMask>(to_geo(s), total, most); break;
-#ifdef CHILL_CUSTOM_MASK
-    case CHILL_MASK_CUSTOM: split_count_steps<CHILL_CUSTOM_MASK>(to_geo(s), total, most); break;
-#endif
-    default: return false;
-  }
+  CHILL_MASK_SWITCH_OR(s.mask.id, count_steps<MaskT>(to_geo(s), total, most), return false)
   return most >= 2 && total * (s.D <= 32 ? 32 : 64) >= least;
 }
 

@@ -14,6 +14,10 @@
 //              O += P V (P from TMEM, V from shared memory, MN-major), completion signalled to
 //              mbarriers with tcgen05.commit.
 //
+// The form with two streams (NS = 2) has the softmax warps, the issuer and the TMEM columns twice; see fwd_two_streams.
+// The first key tile starts at the first key the tile of queries can see, not at a multiple of its size: a window(16, 16) then
+// takes three 64-key tiles instead of four (fp16 (8,12,2085,64): 46 -> 39 us).
+//
 // TMEM columns: kSBufs buffers of KT fp32 columns for S, each overlaid by its P (16-bit, first KT / 2
 // columns); then D columns of O.
 // Head dims 16 and 32 run the head-dim-64 kernels (here and in the backward): the tensor maps have the true width, so TMA
@@ -26,6 +30,7 @@
 
 #include "generic.cuh"
 #include "tc_common.cuh"
+#include "tc_launch.h"
 
 namespace chill {
 namespace tc {
@@ -71,18 +76,23 @@ constexpr int kTmemColsFwd = 256;     // TF32 forward: S 128 + O 128 columns
 // D = 256: S 128 + O 256 columns and 192 KB of Q / K / V tiles leave room for one CTA per SM only.
 // A CTA's register pool is threads x launch registers, and the softmax warpgroup's setmaxnreg.inc is only ever
 // granted if softmax + other <= 2 x launch.
-template <int D>
+// NS = 2: two streams in one CTA, see fwd_two_streams; each has what a CTA with NS = 1 has, only Q is shared.
+template <int D, int NS = 1>
 struct FwdShape {
+  static_assert(NS == 1 || D <= 128, "TMEM holds one stream of head dim 256");
   static constexpr int kKeys = (D <= 128) ? 64 : 128;      // keys per tile
   static constexpr int kSBufs = (D == 128) ? 2 : 1;        // S / P buffers in TMEM
-  static constexpr int kCtasPerSm = (D == 64) ? 4 : (D == 128 ? 2 : 1);
+  static constexpr int kCtasPerSm = ((D == 64) ? 4 : (D == 128 ? 2 : 1)) / NS;
   static constexpr int kStages = (D <= 128) ? 2 : 1;       // K / V ring depth
   static constexpr int kSO = kSBufs * kKeys + D;           // columns in use: S buffers, then O
-  static constexpr int kTmemCols = (kSO <= 128) ? 128 : (kSO <= 256 ? 256 : 512);
-  static constexpr int kLaunchRegs = (65536 / (kCtasPerSm * kFwdThreads) > 128) ? 128 : 65536 / (kCtasPerSm * kFwdThreads);
-  static constexpr int kSoftmaxRegs = (D == 64) ? 96 : 200;
-  static constexpr int kOtherRegs = (D == 64) ? 32 : 56;
-  static_assert(kSoftmaxRegs + kOtherRegs <= 2 * kLaunchRegs, "setmaxnreg.inc would never be granted");
+  static constexpr int kStreamCols = (kSO <= 128) ? 128 : (kSO <= 256 ? 256 : 512);
+  static constexpr int kTmemCols = NS * kStreamCols;
+  static constexpr int kThreads = NS == 1 ? kFwdThreads : 384;  // NS = 2: warps 0-7 softmax, 8 TMA producer, 9 / 10 MMA issuers, 11 idle
+  static constexpr int kLaunchRegs = NS == 1 ? ((65536 / (kCtasPerSm * kThreads) > 128) ? 128 : 65536 / (kCtasPerSm * kThreads))
+                                             : 65536 / (kCtasPerSm * kThreads) / 8 * 8;
+  static constexpr int kSoftmaxRegs = NS == 1 ? ((D == 64) ? 96 : 200) : ((D == 64) ? 96 : 208);
+  static constexpr int kOtherRegs = NS == 1 ? ((D == 64) ? 32 : 56) : ((D == 64) ? 48 : 88);
+  static_assert(NS * kSoftmaxRegs + kOtherRegs <= (NS + 1) * kLaunchRegs, "setmaxnreg.inc would never be granted");
   static_assert(kCtasPerSm * kTmemCols <= 512, "TMEM columns of an SM");
 };
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
@@ -96,17 +106,20 @@ struct FwdTcParams {
   int* status;
 };
 
-template <int D, int NSTAGE, int KT = kTile>
+template <int D, int NSTAGE, int KT = kTile, int NS = 1>
 struct FwdSmem {
   static constexpr int kTileBytes = kTile * D * 2;  // one 128 x D tile of 16-bit elements (Q)
   static constexpr int kKvBytes = KT * D * 2;       // one K or V tile: KT keys
   static constexpr int kQ = 0;
   static constexpr int kK = kQ + kTileBytes;
   static constexpr int kV = kK + NSTAGE * kKvBytes;
-  static constexpr int kBars = kV + NSTAGE * kKvBytes;
-  static constexpr int kNumBars = 8 + 4 * NSTAGE;
-  static constexpr int kMisc = kBars + 8 * kNumBars;
+  static constexpr int kStream = 2 * NSTAGE * kKvBytes;  // K and V rings of a stream; at the end of stream 1 its O, fp32
+  static constexpr int kBars = kK + NS * kStream;
+  static constexpr int kNumBars = 8 + 4 * NSTAGE;   // per stream
+  static constexpr int kMerge = kBars + 8 * NS * kNumBars;  // NS = 2: maximum and sum of stream 1's rows
+  static constexpr int kMisc = kMerge + (NS == 2 ? kTile * 8 : 0);
   static constexpr int kTotal = kMisc + 16;
+  static_assert(NS == 1 || kTile * D * 4 <= kStream, "stream 1 hands its O over in its K / V rings");
   static constexpr int kDynamic = kTotal + 1024;  // slack for manual 1024-byte alignment
 };
 
@@ -210,11 +223,15 @@ __device__ __forceinline__ void softmax_tile(uint32_t tS, uint32_t tO, uint32_t 
 
 // Normalise this thread's O row, convert to 16 bits and stage it in the 128B-swizzled TMA box layout;
 // also writes the row's LSE.  `have` = the accumulator holds data (at least one key tile was processed).
-template <typename T, int D>
+// `other` (kMerge): the row's O from a second stream, [D / 4][128 rows][4], to be weighted with `w_other` where the accumulator
+// has weight `w`.
+template <typename T, int D, bool kMerge = false>
 __device__ __forceinline__ void stage_output_row(uint8_t* sO, uint32_t tO, uint32_t lane_sel, int r, bool have,
-                                                 bool row_valid, float l, float m_used, float* lse_ptr) {
+                                                 bool row_valid, float l, float m_used, float* lse_ptr, const float4* other = nullptr,
+                                                 float w = 1.f, float w_other = 0.f) {
   const float l_safe = (l == 0.f) ? 1.f : l;
   const float inv = 1.f / l_safe;
+  if (kMerge) w_other *= inv;
 #pragma unroll
   for (int q4 = 0; q4 < D / 32; ++q4) {
     uint32_t oreg[32];
@@ -227,8 +244,13 @@ __device__ __forceinline__ void stage_output_row(uint8_t* sO, uint32_t tO, uint3
     for (int i = 0; i < 16; ++i) {
       float a = 0.f, bb = 0.f;
       if (have && row_valid && l != 0.f) {
-        a = __uint_as_float(oreg[2 * i]) * inv;
-        bb = __uint_as_float(oreg[2 * i + 1]) * inv;
+        a = __uint_as_float(oreg[2 * i]) * (kMerge ? w * inv : inv);
+        bb = __uint_as_float(oreg[2 * i + 1]) * (kMerge ? w * inv : inv);
+        if (kMerge && other != nullptr) {
+          const float4 x = other[(q4 * 8 + i / 2) * kTile];
+          a = fmaf((i & 1) ? x.z : x.x, w_other, a);
+          bb = fmaf((i & 1) ? x.w : x.y, w_other, bb);
+        }
       }
       packed[i] = pack2<T>(a, bb);
     }
@@ -248,14 +270,16 @@ __device__ __forceinline__ void stage_output_row(uint8_t* sO, uint32_t tO, uint3
   }
 }
 
-template <typename T, int D, class M>
-__global__ void __launch_bounds__(kFwdThreads, (FwdShape<D>::kCtasPerSm > 1 ? FwdShape<D>::kCtasPerSm : 2))
+template <typename T, int D, class M, int NS>
+__global__ void __launch_bounds__(FwdShape<D, NS>::kThreads, (NS == 2 || FwdShape<D, NS>::kCtasPerSm > 1 ? FwdShape<D, NS>::kCtasPerSm : 2))
 fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
               const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO, FwdTcParams p) {
-  using SH = FwdShape<D>;
+  using SH = FwdShape<D, NS>;
   constexpr int NSTAGE = SH::kStages;
   constexpr int KT = SH::kKeys;                // keys per tile
-  using L = FwdSmem<D, NSTAGE, KT>;
+  using L = FwdSmem<D, NSTAGE, KT, NS>;
+  constexpr int kThreads = SH::kThreads;
+  constexpr int kProducer = 4 * NS;            // warps: softmax of stream 0 (, 1), TMA producer, MMA issuer of stream 0 (, 1)
   constexpr int kChunks = D / 64;              // 64-channel (128-byte) column blocks per tile
   constexpr int kChunkBytes = kTile * 128;     // one column block of Q / O: 128 rows x 128 bytes
   constexpr int kKvChunkBytes = KT * 128;      // one column block of a K / V tile: KT rows x 128 bytes
@@ -278,17 +302,17 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     T* obase = reinterpret_cast<T*>(p.o) + b * p.o_sb + h * p.o_sh;
     const int rows = imin(kTile, g.Lq - qb);
     const int units = g.D / 8;
-    for (int idx = threadIdx.x; idx < rows * units; idx += kFwdThreads) {
+    for (int idx = threadIdx.x; idx < rows * units; idx += kThreads) {
       const int r = idx / units, c = idx % units;
       *reinterpret_cast<uint4*>(obase + (qb + r) * p.o_sl + c * 8) = make_uint4(0, 0, 0, 0);
     }
     if (p.lse != nullptr)
-      for (int r = threadIdx.x; r < rows; r += kFwdThreads) p.lse[b * p.lse_sb + h * p.lse_sh + (qb + r) * p.lse_sl] = 0.f;
+      for (int r = threadIdx.x; r < rows; r += kThreads) p.lse[b * p.lse_sb + h * p.lse_sh + (qb + r) * p.lse_sl] = 0.f;
     return;
   }
 
   // ---- key-tile range of this query tile (same arithmetic in every role)
-  int kt_lo = 0, kt_hi = 0;  // [kt_lo, kt_hi) in units of KT local key rows
+  int k_row0 = 0, n_tiles = 0;  // first local key row of the first tile; the tiles need not start at a multiple of KT
   int full_lo = 0, full_hi = 0;  // global, half-open: keys visible to every row of the tile
   {
     int lo, hi;
@@ -296,18 +320,18 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const int lo_l = imax(lo - g.k_off, 0);
     const int hi_l = imin(imin(hi, n - 1) - g.k_off, g.Lk - 1);
     if (hi_l >= lo_l) {
-      kt_lo = lo_l / KT;
-      kt_hi = hi_l / KT + 1;
+      k_row0 = lo_l;
+      n_tiles = (hi_l - lo_l) / KT + 1;
     }
     if (M::kHasKFullRange) M::k_full_range_for_q(qg0, kTile, n, g.margs, full_lo, full_hi);
   }
-  const int n_tiles = kt_hi - kt_lo;
 
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t sQ = base + L::kQ, sK = base + L::kK, sV = base + L::kV;
+  const uint32_t sQ = base + L::kQ, sK = base + L::kK, sV = base + L::kV;  // + kStream per stream
   const uint32_t bars = base + L::kBars;
+  constexpr uint32_t kBarStream = 8 * L::kNumBars;                          // barriers (but for Q's): + kBarStream per stream
   constexpr int NSB = SH::kSBufs;
   // One tcgen05.commit per MMA batch is free, a second one costs the issuing thread ~48 clocks (measured), so a
   // batch signals ONE barrier with several waiters: s_full[j % NSTAGE] tells the softmax warps that S(j) is there
@@ -315,7 +339,7 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   // and a softmax warp that has to rescale O that O += P(j) V(j) has finished.  Per barrier at most one phase can
   // be ahead of any waiter (the next commit on it needs that waiter's own progress), so the parity tests hold.
   // p_full: one barrier per S buffer.
-  const uint32_t bar_q_full = bars, bar_s_full = bars + 8, bar_p_full = bars + 24, bar_o_full = bars + 40;
+  const uint32_t bar_q_full = bars, bar_s_full = bars + 8, bar_p_full = bars + 24, bar_o_full = bars + 40, bar_merge = bars + 48;
   const uint32_t bar_k_full = bars + 64, bar_v_full = bar_k_full + 8 * NSTAGE, bar_v_empty = bar_v_full + 8 * NSTAGE;
   const uint32_t bar_k_empty = bar_s_full;  // same barriers: S(j) complete == K stage j % NSTAGE consumed
   static_assert(NSTAGE <= 2 && NSB <= 2, "barrier layout");
@@ -323,19 +347,23 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_base + L::kMisc + 4);
   const Guard guard{p.status, abort_flag};
 
-  if (warp == 4) {
+  if (warp == kProducer) {
     // The producer thread initialises the barriers itself, so it can put Q and the first K/V tile in flight
     // before the CTA-wide set-up (TMEM allocation, __syncthreads) completes instead of after it.
     if (lane == 0) {
       *abort_flag = 0;
       mbar_init(bar_q_full, 1);
-      for (int i = 0; i < NSB; ++i) mbar_init(bar_p_full + 8 * i, 4);
-      mbar_init(bar_o_full, 1);
-      for (int s = 0; s < NSTAGE; ++s) {
-        mbar_init(bar_s_full + 8 * s, 1);
-        mbar_init(bar_k_full + 8 * s, 1);
-        mbar_init(bar_v_full + 8 * s, 1);
-        mbar_init(bar_v_empty + 8 * s, 1);
+      if (NS == 2) mbar_init(bar_merge, 4);
+      for (int w = 0; w < NS; ++w) {
+        const uint32_t o = w * kBarStream;
+        for (int i = 0; i < NSB; ++i) mbar_init(bar_p_full + o + 8 * i, 4);
+        mbar_init(bar_o_full + o, 1);
+        for (int s = 0; s < NSTAGE; ++s) {
+          mbar_init(bar_s_full + o + 8 * s, 1);
+          mbar_init(bar_k_full + o + 8 * s, 1);
+          mbar_init(bar_v_full + o + 8 * s, 1);
+          mbar_init(bar_v_empty + o + 8 * s, 1);
+        }
       }
       fence_barrier_init();
       fence_proxy_async_smem();
@@ -343,9 +371,9 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         mbar_arrive_expect_tx(bar_q_full, L::kTileBytes);
         for (int c = 0; c < kChunks; ++c) tma_load_4d(sQ + c * kChunkBytes, &tmQ, bar_q_full, c * 64, qb, h, b);
         mbar_arrive_expect_tx(bar_k_full, L::kKvBytes);
-        for (int c = 0; c < kChunks; ++c) tma_load_4d(sK + c * kKvChunkBytes, &tmK, bar_k_full, c * 64, kt_lo * KT, hk, b);
+        for (int c = 0; c < kChunks; ++c) tma_load_4d(sK + c * kKvChunkBytes, &tmK, bar_k_full, c * 64, k_row0, hk, b);
         mbar_arrive_expect_tx(bar_v_full, L::kKvBytes);
-        for (int c = 0; c < kChunks; ++c) tma_load_4d(sV + c * kKvChunkBytes, &tmV, bar_v_full, c * 64, kt_lo * KT, hk, b);
+        for (int c = 0; c < kChunks; ++c) tma_load_4d(sV + c * kKvChunkBytes, &tmV, bar_v_full, c * 64, k_row0, hk, b);
       }
     }
     __syncwarp();
@@ -356,28 +384,29 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tS = tmem;            // S / P columns: NSB buffers of KT columns
+  const uint32_t tS = tmem;            // S / P columns: NSB buffers of KT columns; + kStreamCols per stream
   const uint32_t tO = tmem + NSB * KT; // O columns
 
-  if (warp == 4) {
+  if (warp == kProducer) {
     reg_dealloc<SH::kOtherRegs>();
     // ------------------------------------------------------------------- TMA producer
     if (lane == 0 && n_tiles > 0) {
       bool ok = true;
-      for (int j = 1; j < n_tiles && ok; ++j) {  // tile 0 was issued during set-up
-        const int s = j % NSTAGE;
+      for (int t = 1; t < n_tiles && ok; ++t) {  // tile 0 was issued during set-up
+        const uint32_t w = (uint32_t)(t % NS), bo = w * kBarStream, so = w * L::kStream;
+        const int j = t / NS, s = j % NSTAGE;  // tile j of stream w
         const uint32_t ph = (uint32_t)(j / NSTAGE) & 1u;
-        const int krow = (kt_lo + j) * KT;
-        ok = mbar_wait(bar_k_empty + 8 * s, ph ^ 1u, guard, kStProducer);
+        const int krow = k_row0 + t * KT;
+        ok = mbar_wait(bar_k_empty + bo + 8 * s, ph ^ 1u, guard, kStProducer);
         if (!ok) break;
-        mbar_arrive_expect_tx(bar_k_full + 8 * s, L::kKvBytes);
+        mbar_arrive_expect_tx(bar_k_full + bo + 8 * s, L::kKvBytes);
         for (int c = 0; c < kChunks; ++c)
-          tma_load_4d(sK + s * L::kKvBytes + c * kKvChunkBytes, &tmK, bar_k_full + 8 * s, c * 64, krow, hk, b);
-        ok = mbar_wait(bar_v_empty + 8 * s, ph ^ 1u, guard, kStProducer);
+          tma_load_4d(sK + so + s * L::kKvBytes + c * kKvChunkBytes, &tmK, bar_k_full + bo + 8 * s, c * 64, krow, hk, b);
+        ok = mbar_wait(bar_v_empty + bo + 8 * s, ph ^ 1u, guard, kStProducer);
         if (!ok) break;
-        mbar_arrive_expect_tx(bar_v_full + 8 * s, L::kKvBytes);
+        mbar_arrive_expect_tx(bar_v_full + bo + 8 * s, L::kKvBytes);
         for (int c = 0; c < kChunks; ++c)
-          tma_load_4d(sV + s * L::kKvBytes + c * kKvChunkBytes, &tmV, bar_v_full + 8 * s, c * 64, krow, hk, b);
+          tma_load_4d(sV + so + s * L::kKvBytes + c * kKvChunkBytes, &tmV, bar_v_full + bo + 8 * s, c * 64, krow, hk, b);
       }
       if (!ok) {
         // give copies already in flight time to land before the CTA's shared memory goes away
@@ -385,10 +414,12 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
       }
     }
-  } else if (warp == 5) {
+  } else if (warp > kProducer && warp <= kProducer + NS) {
     reg_dealloc<SH::kOtherRegs>();
     // --------------------------------------------------------------------- MMA issuer
-    if (lane == 0 && n_tiles > 0) {
+    const uint32_t w = NS == 1 ? 0u : (uint32_t)(warp - kProducer - 1), bo = w * kBarStream, so = w * L::kStream, to = w * SH::kStreamCols;
+    const int my_tiles = (n_tiles - (int)w + NS - 1) / NS;
+    if (lane == 0 && my_tiles > 0) {
       constexpr uint32_t idesc_s = make_idesc<T>(kTile, KT, false, false);
       constexpr uint32_t idesc_o = make_idesc<T>(kTile, D, false, true);
       constexpr uint32_t hi_k = desc_hi_sw128(1024);  // both operand kinds: 8-row groups 1 KB apart
@@ -396,33 +427,33 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
       bool ok = mbar_wait(bar_q_full, 0, guard, kStMma);
       auto issue_s = [&](int j) -> bool {  // S(j) = Q K(j)^T into S buffer j % NSB: both K-major, 16 channels per MMA
         const int s = j % NSTAGE;
-        const uint32_t k_lo = desc_lo_sw128(sK + s * L::kKvBytes, 16);
-        if (!mbar_wait(bar_k_full + 8 * s, (uint32_t)(j / NSTAGE) & 1u, guard, kStMma)) return false;
+        const uint32_t k_lo = desc_lo_sw128(sK + so + s * L::kKvBytes, 16);
+        if (!mbar_wait(bar_k_full + bo + 8 * s, (uint32_t)(j / NSTAGE) & 1u, guard, kStMma)) return false;
         tc_fence_after();
-        const uint32_t ts = tS + (uint32_t)((j % NSB) * KT);
+        const uint32_t ts = tS + to + (uint32_t)((j % NSB) * KT);
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)  // Q chunks are 128 rows apart, K chunks KT rows
           mma_ss_lh(ts, q_lo + kmajor_step(kk), k_lo + (uint32_t)((kk / 4) * (kKvChunkBytes / 16) + (kk % 4) * 2), hi_k, idesc_s,
                     kk > 0 ? 1u : 0u);
-        mma_commit(bar_s_full + 8 * s);
+        mma_commit(bar_s_full + bo + 8 * s);
         return true;
       };
       auto issue_pv = [&](int j) -> bool {  // O += P(j) V(j): P (16-bit) from TMEM, 16 keys = 8 columns per MMA
         const int s = j % NSTAGE;
-        const uint32_t v_lo = desc_lo_sw128(sV + s * L::kKvBytes, kKvChunkBytes);  // MN-major: channel blocks one chunk apart
-        if (!mbar_wait(bar_p_full + 8 * (j % NSB), (uint32_t)(j / NSB) & 1u, guard, kStMma)) return false;
-        if (!mbar_wait(bar_v_full + 8 * s, (uint32_t)(j / NSTAGE) & 1u, guard, kStMma)) return false;
+        const uint32_t v_lo = desc_lo_sw128(sV + so + s * L::kKvBytes, kKvChunkBytes);  // MN-major: channel blocks one chunk apart
+        if (!mbar_wait(bar_p_full + bo + 8 * (j % NSB), (uint32_t)(j / NSB) & 1u, guard, kStMma)) return false;
+        if (!mbar_wait(bar_v_full + bo + 8 * s, (uint32_t)(j / NSTAGE) & 1u, guard, kStMma)) return false;
         tc_fence_after();
-        const uint32_t tp = tS + (uint32_t)((j % NSB) * KT);
+        const uint32_t tp = tS + to + (uint32_t)((j % NSB) * KT);
 #pragma unroll
         for (int kk = 0; kk < KT / 16; ++kk)
-          mma_ts_lh(tO, tp + kk * 8, v_lo + kk * 128, hi_k, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
-        mma_commit(bar_v_empty + 8 * s);
+          mma_ts_lh(tO + to, tp + kk * 8, v_lo + kk * 128, hi_k, idesc_o, (j > 0 || kk > 0) ? 1u : 0u);
+        mma_commit(bar_v_empty + bo + 8 * s);
         return true;
       };
       if (NSB == 1) {
         // one S buffer: S(j+1) overwrites P(j), so the two GEMMs of a tile alternate
-        for (int j = 0; j < n_tiles && ok; ++j) {
+        for (int j = 0; j < my_tiles && ok; ++j) {
           ok = issue_s(j);
           if (ok) ok = issue_pv(j);
         }
@@ -430,63 +461,126 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
         // S(j+1) goes to the other buffer and is issued ahead of O += P(j) V(j): it runs during softmax(j).
         // MMAs execute in issue order, so S(j+2) cannot overtake the P V(j) that still reads its buffer.
         if (ok) ok = issue_s(0);
-        for (int j = 0; j < n_tiles && ok; ++j) {
-          if (j + 1 < n_tiles) ok = issue_s(j + 1);
+        for (int j = 0; j < my_tiles && ok; ++j) {
+          if (j + 1 < my_tiles) ok = issue_s(j + 1);
           if (ok) ok = issue_pv(j);
         }
       }
-      if (ok) mma_commit(bar_o_full);
+      if (ok) mma_commit(bar_o_full + bo);
     }
-  } else if (warp >= 6) {
-    reg_dealloc<SH::kOtherRegs>();  // idle warps of the second warpgroup only give their registers back
+  } else if (warp > kProducer + NS) {
+    reg_dealloc<SH::kOtherRegs>();  // idle warps of the last warpgroup only give their registers back
   } else {
     reg_alloc<SH::kSoftmaxRegs>();
     // --------------------------------------------------------- softmax + epilogue warps
-    const int r = warp * 32 + lane;  // row inside the tile == TMEM lane
-    const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
+    const uint32_t w = NS == 1 ? 0u : (uint32_t)(warp >> 2), bo = w * kBarStream;  // stream
+    const int r = (NS == 1 ? warp : warp & 3) * 32 + lane;                          // row inside the tile == TMEM lane
+    const uint32_t lane_sel = ((uint32_t)((NS == 1 ? warp : warp & 3) * 32) << 16) + w * SH::kStreamCols;
     const int qg = qg0 + r;
     const float c = g.scale * kLog2e;
     float m_used = -CUDART_INF_F, l = 0.f;
     bool ok = true;
-    for (int j = 0; j < n_tiles; ++j) {
-      const int kt = kt_lo + j;
-      const int kg0 = kt * KT + g.k_off;
-      ok = mbar_wait(bar_s_full + 8 * (j % NSTAGE), (uint32_t)(j / NSTAGE) & 1u, guard, kStSoftmax);
+    const int my_tiles = (n_tiles - (int)w + NS - 1) / NS;
+    for (int j = 0; j < my_tiles; ++j) {
+      const int krow = k_row0 + (j * NS + (int)w) * KT;
+      const int kg0 = krow + g.k_off;
+      ok = mbar_wait(bar_s_full + bo + 8 * (j % NSTAGE), (uint32_t)(j / NSTAGE) & 1u, guard, kStSoftmax);
       ok = __all_sync(0xffffffffu, ok);  // keep the warp converged for the .sync.aligned TMEM accesses
       if (!ok) break;
       tc_fence_after();
       const bool full = M::kHasKFullRange && kg0 >= full_lo && kg0 + KT <= full_hi && kg0 + KT <= n &&
-                        kt * KT + KT <= g.Lk;
-      const int klim = imin(n - kg0, g.Lk - kt * KT);  // columns >= klim do not exist
+                        krow + KT <= g.Lk;
+      const int klim = imin(n - kg0, g.Lk - krow);  // columns >= klim do not exist
       softmax_tile<T, D, M, KT>(tS + (uint32_t)((j % NSB) * KT), tO, lane_sel, j == 0, full, klim, qg, kg0, n, g.margs, c,
-                                m_used, l, NSB > 1 ? bar_v_empty + 8 * (uint32_t)((j - 1) % NSTAGE) : 0u,
+                                m_used, l, NSB > 1 ? bar_v_empty + bo + 8 * (uint32_t)((j - 1) % NSTAGE) : 0u,
                                 (uint32_t)((j - 1) / NSTAGE) & 1u, &guard);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_p_full + 8 * (j % NSB));  // one arrival per softmax warp
+      if (lane == 0) mbar_arrive(bar_p_full + bo + 8 * (j % NSB));  // one arrival per softmax warp
     }
 
     // ---- epilogue: O / l -> 16-bit -> swizzled shared memory (Q's buffer) -> TMA store
-    if (ok && n_tiles > 0) ok = mbar_wait(bar_o_full, 0, guard, kStEpilogue);
+    if (ok && my_tiles > 0) ok = mbar_wait(bar_o_full + bo, 0, guard, kStEpilogue);
     ok = __all_sync(0xffffffffu, ok);
     tc_fence_after();
     const bool row_valid = qg < n;
-    stage_output_row<T, D>(gen_base + L::kQ, tO, lane_sel, r, n_tiles > 0 && ok, row_valid, l, m_used,
-                           (p.lse != nullptr && qb + r < g.Lq) ? p.lse + b * p.lse_sb + h * p.lse_sh + (qb + r) * p.lse_sl
-                                                                : nullptr);
-    fence_proxy_async_smem();
-    named_bar_sync(1, 128);
-    if (threadIdx.x == 0) {
-      for (int cc = 0; cc < kChunks; ++cc) tma_store_4d(&tmO, base + L::kQ + cc * kChunkBytes, cc * 64, qb, h, b);
-      tma_store_commit();
-      tma_store_wait_read();  // shared memory may be released; the global writes complete by kernel end
+    float* lse_ptr = (p.lse != nullptr && qb + r < g.Lq) ? p.lse + b * p.lse_sb + h * p.lse_sh + (qb + r) * p.lse_sl : nullptr;
+    if constexpr (NS == 2) {
+      // Stream 1 hands maximum, sum and O of its rows over (its K / V rings are not read any more); stream 0 merges.
+      float4* other = reinterpret_cast<float4*>(gen_base + L::kK + L::kStream) + r;
+      float2* ml = reinterpret_cast<float2*>(gen_base + L::kMerge) + r;
+      if (w == 1) {
+        if (ok && my_tiles > 0) {
+#pragma unroll
+          for (int q4 = 0; q4 < D / 32; ++q4) {
+            uint32_t oreg[32];
+            tmem_ld32(tO + lane_sel + q4 * 32, oreg);
+            tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              *reinterpret_cast<uint4*>(other + (q4 * 8 + i) * kTile) = make_uint4(oreg[4 * i], oreg[4 * i + 1], oreg[4 * i + 2], oreg[4 * i + 3]);
+          }
+          *ml = make_float2(m_used, l);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar_merge);
+        }
+      } else {
+        float w0 = 1.f, w1 = 0.f;
+        const bool both = n_tiles > 1;
+        if (ok && both) {
+          ok = mbar_wait(bar_merge, 0, guard, kStEpilogue);
+          ok = __all_sync(0xffffffffu, ok);
+          if (ok) {
+            const float2 v = *ml;
+            const float m_all = fmaxf(m_used, v.x), m_safe = (m_all == -CUDART_INF_F) ? 0.f : m_all;
+            w0 = ex2(m_used - m_safe);
+            w1 = ex2(v.x - m_safe);
+            l = l * w0 + v.y * w1;
+            m_used = m_all;
+          }
+        }
+        stage_output_row<T, D, true>(gen_base + L::kQ, tO, lane_sel, r, n_tiles > 0 && ok, row_valid, l, m_used, lse_ptr, both ? other : nullptr,
+                                     w0, w1);
+      }
+    } else {
+      stage_output_row<T, D>(gen_base + L::kQ, tO, lane_sel, r, n_tiles > 0 && ok, row_valid, l, m_used, lse_ptr);
+    }
+    if (NS == 1 || w == 0) {
+      fence_proxy_async_smem();
+      named_bar_sync(1, 128);
+      if (threadIdx.x == 0) {
+        for (int cc = 0; cc < kChunks; ++cc) tma_store_4d(&tmO, base + L::kQ + cc * kChunkBytes, cc * 64, qb, h, b);
+        tma_store_commit();
+        tma_store_wait_read();  // shared memory may be released; the global writes complete by kernel end
+      }
     }
   }
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) tmem_dealloc(tmem, SH::kTmemCols);
+  if (warp == kProducer) tmem_dealloc(tmem, SH::kTmemCols);
+}
+
+// Whether a forward of head dim 64 or 128 with `ctas` tiles of 128 queries takes the form with two streams: one CTA then works on
+// two chains of key tiles (even and odd ones) of the same queries and merges them at the end, so a tile of queries takes about
+// half as long, but an SM holds half as many CTAs and a CTA has the merge (2 to 3 us) to make up for.  It pays where all CTAs are
+// resident at once all the same and the loops are long, or, at head dim 64, where a few long loops outlast the rest.  One / two
+// streams in us (bf16; graph replays):
+//   D = 128  (1,4,4096) full, 128 CTAs of 64 steps: 52.5 / 37.6   (1,8,1000), 16 steps: 16.8 / 16.2   (1,32,512), 8 steps: 11.2 / 12.3
+//            (1,16,2048), 256 CTAs: 35.4 / 45.1
+//   D = 64   (1,4,4096) full: 78.8 / 57.5   (1,16,2048), 256 CTAs: 46.8 / 39.7   (1,32,512): 13.5 / 12.3   window(256, 0), 6 steps:
+//            11.8 / 11.4   (2,8,300), 5 steps: 9.9 / 10.3   512 CTAs: full (2,16,2048) 66.9 / 72.7, causal (2,16,2048), 32 steps at
+//            most: 55.2 / 53.4, causal (2,4,8192): 161 / 121, causal (8,8,1024), 16 at most: 35.5 / 36.6
+template <class M>
+bool fwd_two_streams(const Geo& g, int D, int ctas) {
+  const int sms = sm_count(), resident = sms * FwdShape<64, 2>::kCtasPerSm;
+  if (ctas > (D == 128 ? sms : 2 * resident)) return false;
+  long long total;
+  int most;
+  count_steps<M>(g, total, most);
+  if (D == 128) return most >= 16;
+  return ctas <= resident ? most >= 6 : most >= 32 && 3 * total <= 2ll * most * ctas;
 }
 
 }  // namespace tc

@@ -87,6 +87,26 @@ __device__ __forceinline__ int valid_len(const Geo& g, int b) {
   return n;
 }
 
+// Steps of 128 queries x 64 keys of a call, over all heads: `total`, and the most a tile of queries has (for the rules that choose
+// between kernels).  At most 32 tiles are looked at (four where a tile's range takes a loop over its rows); lens is not known here.
+template <class M>
+void count_steps(const Geo& g, long long& total, int& most) {
+  constexpr int kRows = 128, kCols = 64, kLooks = M::kKLimsContinuous ? 32 : 4;
+  const int n_rt = (g.Lq + kRows - 1) / kRows, every = (n_rt + kLooks - 1) / kLooks;
+  long long sum = 0, looks = 0;
+  most = 0;
+  for (int t = n_rt - 1; t >= 0; t -= every, ++looks) {
+    int lo, hi;
+    tile_range<M, true>(t * kRows + g.q_off, imin(kRows, g.Lq - t * kRows), g.seq_len, g.margs, lo, hi);
+    lo = imax(lo - g.k_off, 0);
+    hi = imin(imin(hi, g.seq_len - 1) - g.k_off, g.Lk - 1);
+    const int n = hi >= lo ? (hi - lo) / kCols + 1 : 0;
+    sum += n;
+    most = imax(most, n);
+  }
+  total = sum * n_rt / looks * g.B * g.H;
+}
+
 // --------------------------------------------------------------------------------- delta
 // delta[b,h,t] = sum_d O*dO in fp32; one warp per row, every row (no `lens`), like the reference.
 template <typename T>

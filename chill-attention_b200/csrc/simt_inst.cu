@@ -89,11 +89,6 @@ int split_launch_fwd<InstMask>(const split::FwdParams& p, cudaStream_t st) {
 }
 
 template <>
-void split_count_steps<InstMask>(const Geo& g, long long& total, int& most) {
-  split::count_steps<InstMask>(g, total, most);
-}
-
-template <>
 int split_launch_bwd<InstMask>(split::BwdParams p, int which, cudaStream_t st) {
   auto kern = split::split_bwd_kernel<InstMask>;
   constexpr int smem = split::BwdSmem::kDynamic;

@@ -229,26 +229,6 @@ __device__ __forceinline__ void store_row_f32(float* dst, const float* v, int n)
   for (int i = 0; i < n; i += 4) *reinterpret_cast<float4*>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
 }
 
-// ------------------------------------------------------------------------------- dispatch
-// Steps (tiles of 128 queries x 64 keys) of a call, over all heads: `total`, and the most a query tile has.  Long sequences are
-// sampled; lens is not known on the host.
-template <class M>
-void count_steps(const Geo& g, long long& total, int& most) {
-  const int n_rt = (g.Lq + kRows - 1) / kRows, every = (n_rt + 31) / 32;
-  long long sum = 0;
-  most = 0;
-  for (int t = every / 2; t < n_rt; t += every) {
-    int lo, hi;
-    tile_range<M, true>(t * kRows + g.q_off, imin(kRows, g.Lq - t * kRows), g.seq_len, g.margs, lo, hi);
-    lo = imax(lo - g.k_off, 0);
-    hi = imin(imin(hi, g.seq_len - 1) - g.k_off, g.Lk - 1);
-    const int n = hi >= lo ? hi / kCols - lo / kCols + 1 : 0;
-    sum += (long long)n * imin(every, n_rt);
-    most = imax(most, n);
-  }
-  total = sum * g.B * g.H;
-}
-
 // ------------------------------------------------------------------------------- forward
 // One CTA per SM owns 128 query rows.  Two softmax warpgroups take the key tiles in turn (even / odd), each with scores, product,
 // maximum and sums of its own, and the two results are merged at the end: the chain of a tile (scores, softmax, product) is

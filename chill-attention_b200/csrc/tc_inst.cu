@@ -16,31 +16,33 @@ namespace chill {
 
 using InstMask = CHILL_INST_MASK;
 
-template <typename T, int D>
+template <typename T, int D, int NS>
 static int launch_fwd_one(const CUtensorMap* maps, const tc::FwdTcParams& p, dim3 grid, cudaStream_t st) {
-  auto kern = tc::fwd_tc_kernel<T, D, InstMask>;
-  using SH = tc::FwdShape<D>;
-  constexpr int smem = tc::FwdSmem<D, SH::kStages, SH::kKeys>::kDynamic;
+  auto kern = tc::fwd_tc_kernel<T, D, InstMask, NS>;
+  using SH = tc::FwdShape<D, NS>;
+  constexpr int smem = tc::FwdSmem<D, SH::kStages, SH::kKeys, NS>::kDynamic;
   static_assert(SH::kCtasPerSm * smem <= 232448, "the CTAs that are to share an SM must fit its shared memory");
   struct Tag {};
   cudaError_t e = ensure_dynamic_smem<Tag>(kern, smem, /*prefer_max_carveout=*/true);
   if (e != cudaSuccess) return (int)e;
-  kern<<<grid, tc::kFwdThreads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], p);
+  kern<<<grid, SH::kThreads, smem, st>>>(maps[0], maps[1], maps[2], maps[3], p);
   return (int)cudaGetLastError();
+}
+
+template <typename T>
+static int launch_fwd_dim(int D, const CUtensorMap* maps, const tc::FwdTcParams& p, dim3 grid, cudaStream_t st) {
+  const bool two = D <= 128 && tc::fwd_two_streams<InstMask>(p.g, D, (int)grid.x);
+  if (D == 128) return two ? launch_fwd_one<T, 128, 2>(maps, p, grid, st) : launch_fwd_one<T, 128, 1>(maps, p, grid, st);
+  if (D == 64) return two ? launch_fwd_one<T, 64, 2>(maps, p, grid, st) : launch_fwd_one<T, 64, 1>(maps, p, grid, st);
+  if (D == 256) return launch_fwd_one<T, 256, 1>(maps, p, grid, st);
+  return (int)cudaErrorInvalidValue;
 }
 
 template <>
 int tc_launch_fwd<InstMask>(int dtype, int D, const CUtensorMap* maps, const tc::FwdTcParams& p, dim3 grid,
                             cudaStream_t st) {
-  if (dtype == 2) {
-    if (D == 128) return launch_fwd_one<__nv_bfloat16, 128>(maps, p, grid, st);
-    if (D == 64) return launch_fwd_one<__nv_bfloat16, 64>(maps, p, grid, st);
-    if (D == 256) return launch_fwd_one<__nv_bfloat16, 256>(maps, p, grid, st);
-  } else if (dtype == 1) {
-    if (D == 128) return launch_fwd_one<__half, 128>(maps, p, grid, st);
-    if (D == 64) return launch_fwd_one<__half, 64>(maps, p, grid, st);
-    if (D == 256) return launch_fwd_one<__half, 256>(maps, p, grid, st);
-  }
+  if (dtype == 2) return launch_fwd_dim<__nv_bfloat16>(D, maps, p, grid, st);
+  if (dtype == 1) return launch_fwd_dim<__half>(D, maps, p, grid, st);
   return (int)cudaErrorInvalidValue;
 }
 

@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "generic.cuh"
@@ -48,10 +49,16 @@ static cudaError_t ensure_dynamic_smem(Kern kern, int smem_bytes, bool prefer_ma
   return cudaSuccess;
 }
 
-// SMs of the current device.
+// SMs of the current device (asked of the driver once per device and copy of this function: the rules of the dispatch need it in
+// every call).
 static inline int sm_count() {
+  constexpr int kMaxDevices = 64;
+  static std::atomic<int> known[kMaxDevices];
   int dev = 0, n = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 148;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+  if (dev >= 0 && dev < kMaxDevices && (n = known[dev].load(std::memory_order_relaxed)) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 148;
+  if (dev >= 0 && dev < kMaxDevices) known[dev].store(n, std::memory_order_relaxed);
   return n;
 }
 
@@ -65,8 +72,6 @@ int simt_launch_bwd(const simt::BwdParams& p, int which, cudaStream_t st);
 // `repair` set behind it.
 template <class M>
 int split_launch_fwd(const split::FwdParams& p, cudaStream_t st);
-template <class M>
-void split_count_steps(const Geo& g, long long& total, int& most);
 template <class M>
 int split_launch_bwd(split::BwdParams p, int which, cudaStream_t st);
 
