@@ -105,19 +105,18 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (g.lens != nullptr) n = imin(n, g.lens[b]);
 
   // query-tile range that can see this key tile
-  int qt_lo = 0, qt_hi = 0, full_lo = 0, full_hi = 0;
+  int q_row0 = 0, n_qt = 0, full_lo = 0, full_hi = 0;  // tiles from the 32-row group of the first such query on
   if (kg0 < n) {
     int lo, hi;
     tile_range<M, false>(kg0, imin(kTile, g.Lk - kb), n, g.margs, lo, hi);
     const int lo_l = imax(lo - g.q_off, 0);
     const int hi_l = imin(imin(hi, n - 1) - g.q_off, g.Lq - 1);
     if (hi_l >= lo_l) {
-      qt_lo = lo_l / kTile;
-      qt_hi = hi_l / kTile + 1;
+      n_qt = (hi_l - (lo_l & ~31)) / kTile + 1;
+      q_row0 = imin(lo_l & ~31, (n_qt_total - n_qt) * kTile);  // the last tile ends inside the accumulator
     }
     if (M::kHasQFullRange) M::q_full_range_for_k(kg0, kTile, n, g.margs, full_lo, full_hi);
   }
-  const int n_qt = qt_hi - qt_lo;
   const int n_it = n_qt * G;
   if (n_it == 0) {
     // nobody attends these keys (padding, or outside every query's range on this shard)
@@ -169,12 +168,12 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_arrive_expect_tx(bar_q_full, 2 * L::kTileBytes);
       for (int c = 0; c < kChunks; ++c) {
         tma_load_4d(sK + c * kChunkBytes, &tmK, bar_q_full, c * 64, kb, hk, b);
-        tma_load_4d(sRing + c * kChunkBytes, &tmQ, bar_q_full, c * 64, qt_lo * kTile, hk * G, b);
+        tma_load_4d(sRing + c * kChunkBytes, &tmQ, bar_q_full, c * 64, q_row0, hk * G, b);
       }
       mbar_arrive_expect_tx(bar_do_full, 2 * L::kTileBytes);
       for (int c = 0; c < kChunks; ++c) {
         tma_load_4d(sV + c * kChunkBytes, &tmV, bar_do_full, c * 64, kb, hk, b);
-        tma_load_4d(sRing + L::kTileBytes + c * kChunkBytes, &tmdO, bar_do_full, c * 64, qt_lo * kTile, hk * G, b);
+        tma_load_4d(sRing + L::kTileBytes + c * kChunkBytes, &tmdO, bar_do_full, c * 64, q_row0, hk * G, b);
       }
     }
     __syncwarp();
@@ -197,7 +196,7 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           const int s = it % L::kStages;
           const uint32_t ph = (uint32_t)(it / L::kStages) & 1u;
           const int h = hk * G + it / n_qt;
-          const int qrow = (qt_lo + it % n_qt) * kTile;
+          const int qrow = q_row0 + it % n_qt * kTile;
           ok = mbar_wait(bar_ring_empty + 8 * s, ph ^ 1u, guard, kStFusProducer);
           if (!ok) break;
           const uint32_t dst = sRing + s * 2 * L::kTileBytes;
@@ -309,8 +308,8 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     bool ok = true;
     for (int it = 0; it < n_it; ++it) {
       const int h = hk * G + it / n_qt;
-      const int qi = qt_lo + it % n_qt;
-      float* dst = p.dq_accum + (((size_t)b * g.H + h) * n_qt_total + qi) * (size_t)(kTile * D) + rg * (32 * D);
+      const int qi = it % n_qt;
+      float* dst = p.dq_accum + (((size_t)b * g.H + h) * n_qt_total + qi) * (size_t)(kTile * D) + (rg * 32 + q_row0) * D;
       ok = mbar_wait(bar_dq_full, (uint32_t)it & 1u, guard, kStFusDrain);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
@@ -362,14 +361,14 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // LSE / delta of this lane's two query columns, fetched one tile ahead (tile qi_next of head h_next).  The loaded
     // values are not touched until the next iteration (any dependent instruction here would stall on the global load).
     // The walk over heads and tiles is incremental (no divisions).
-    int h_next = hk * G, qi_next = qt_lo;
+    int h_next = hk * G, qi_next = 0;
     float nl_next[2], nd_next[2];
     auto fetch_rows = [&]() {
       const float* lse_h = p.lse + b * p.lse_sb + h_next * p.lse_sh;
       const float* delta_h = p.delta + ((long long)b * g.H + h_next) * g.Lq;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int qrow = qi_next * kTile + c0 + e * 32 + lane;
+        const int qrow = q_row0 + qi_next * kTile + c0 + e * 32 + lane;
         const int row = qrow < g.Lq ? qrow : 0;  // row 0 stands in for rows beyond Lq: those columns are masked out anyway
         nl_next[e] = __ldg(lse_h + row * p.lse_sl);
         nd_next[e] = __ldg(delta_h + row);
@@ -378,10 +377,9 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     fetch_rows();
     for (int it = 0; it < n_it; ++it) {
       const uint32_t par = (uint32_t)it & 1u;
-      const int qi = qi_next;
-      const int qg0 = qi * kTile + g.q_off;
-      if (++qi_next == qt_hi) {
-        qi_next = qt_lo;
+      const int q0 = q_row0 + qi_next * kTile, qg0 = q0 + g.q_off;
+      if (++qi_next == n_qt) {
+        qi_next = 0;
         ++h_next;
       }
       __syncwarp();
@@ -393,8 +391,8 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       __syncwarp();
       if (it + 1 < n_it) fetch_rows();
       const bool full = M::kHasQFullRange && qg0 >= full_lo && qg0 + kTile <= full_hi && qg0 + kTile <= n &&
-                        qi * kTile + kTile <= g.Lq && kg0 + kTile <= n && kb + kTile <= g.Lk;
-      const int qlim = imin(n - qg0, g.Lq - qi * kTile);
+                        q0 + kTile <= g.Lq && kg0 + kTile <= n && kb + kTile <= g.Lk;
+      const int qlim = imin(n - qg0, g.Lq - q0);
       int w_lo = 0, w_hi = -1;  // visible query columns of this key row inside the tile (interval functors)
       if (interval_rows<M>::value && !full && key_ok) row_window<M, false>(kg, qg0, qlim, n, g.margs, w_lo, w_hi);
 

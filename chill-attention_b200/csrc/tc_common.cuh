@@ -36,24 +36,18 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// Upper bound (ns) the hardware may keep the thread suspended inside one try_wait; a waiter wakes
-// as soon as the phase completes, so a generous hint only cuts down on polling instructions that
-// would otherwise compete for issue slots with the warps doing the math.
-#ifndef CHILL_SUSPEND_HINT_NS
-#define CHILL_SUSPEND_HINT_NS 200000u
-#endif
-constexpr uint32_t kSuspendHintNs = CHILL_SUSPEND_HINT_NS;
-
+// Without a suspend-time hint: with one (any length) the instruction takes 50 clocks instead of 16 on a completed phase, and a
+// single waiting lane sees an arrival after 317 clocks instead of 151 (two warps handing an mbarrier to and fro).
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t"
       ".reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t"
       "}\n"
       : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(kSuspendHintNs)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
