@@ -45,7 +45,7 @@ struct BwdParams {
   int n_key_ctas;    // the first n_key_ctas CTAs compute dK / dV, the others dQ
   uint32_t vec;      // kVec*: tensors whose rows are read / written in 16-byte vectors (fp32 only)
   int dtype;
-  bool repair = false;  // only tiles with a row that split.cuh has marked
+  bool repair = false;  // only rows that split.cuh has marked (kRepair)
 };
 struct FwdParams {
   FwdP f;
@@ -290,7 +290,8 @@ struct FwdSmem {
   static constexpr int kBytes = (kW + kRows * kCols) * 4;
 };
 
-template <int DP, int RT, class M>
+// kRepair: only the rows that split.cuh has marked.  A form of its own: at head dim 128 the test at the stores alone costs 4 %.
+template <int DP, int RT, class M, bool kRepair>
 __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2))) simt_fwd_kernel(const __grid_constant__ FwdParams pp) {
   using L = FwdSmem<DP, RT>;
   constexpr int kRows = L::kRows;
@@ -308,7 +309,7 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
   const int qg0 = qb + g.q_off;
   const int rows_in = imin(kRows, g.Lq - qb);
   uint32_t keep = ~0u;  // rows to store
-  if (pp.repair) {
+  if (kRepair) {
     keep = marked<RT>(p.o, b, h, qb + row0, g.Lq);
     if (!__syncthreads_or(keep != 0)) return;
   }
@@ -380,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const int row = qb + row0 + i;
-    if (row >= g.Lq || !((keep >> i) & 1u)) continue;
+    if (row >= g.Lq || (kRepair && !((keep >> i) & 1u))) continue;
     const bool valid = row + g.q_off < n;  // padded query rows: O = 0, LSE = 0
     const float inv = sum != 0.f ? 1.f / sum : 0.f;
     store_row<DP>(p.o.p, b * p.o.sb + h * p.o.sh + row * p.o.sl, p.o.sd, D, pp.dtype, pp.vec & kVecO, l16, acc[i], inv, valid);
@@ -400,7 +401,7 @@ struct BwdSmem {
 // dK / dV part: rows are keys, R1 = K, R2 = V, the streamed tiles C1 = Q and C2 = dO of every query head of the group:
 //     S = K Q^T, dP = V dO^T, P = 2^(S c - LSE), dV += P dO, dS = P (dP - delta), dK += dS Q
 // dQ part: rows are queries, R1 = Q, R2 = dO, C1 = K, C2 = V:   S = Q K^T, dP = dO V^T, dQ += dS K
-template <int DP, int RT, class M, bool kKeyRows>
+template <int DP, int RT, class M, bool kKeyRows, bool kRepair>
 __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int tile_id) {
   using L = BwdSmem<DP, RT>;
   constexpr int kRows = L::kRows;
@@ -418,7 +419,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
   const int rb = rt * kRows, rg0 = rb + (kKeyRows ? g.k_off : g.q_off);
   const int rows_in = imin(kRows, (kKeyRows ? g.Lk : g.Lq) - rb);
   uint32_t keep = ~0u;  // rows to store
-  if (pp.repair) {
+  if (kRepair) {
     keep = marked<RT>(kKeyRows ? p.dk : p.dq, b, hr, rb + row0, rb + rows_in);
     if (!__syncthreads_or(keep != 0)) return;
   }
@@ -530,7 +531,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       const int j = rb + row0 + i;
-      if (j >= g.Lk || !((keep >> i) & 1u)) continue;
+      if (j >= g.Lk || (kRepair && !((keep >> i) & 1u))) continue;
       const bool valid = row0 + i < rows_valid;
       store_row<DP>(p.dk.p, b * p.dk.sb + hr * p.dk.sh + j * p.dk.sl, p.dk.sd, D, pp.dtype, pp.vec & kVecDk, l16, acc1[i], g.scale, valid);
       store_row<DP>(p.dv.p, b * p.dv.sb + hr * p.dv.sh + j * p.dv.sl, p.dv.sd, D, pp.dtype, pp.vec & kVecDv, l16, acc2[i], 1.f, valid);
@@ -544,7 +545,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       const int row = rb + row0 + i;
-      if (row < g.Lq && ((keep >> i) & 1u))
+      if (row < g.Lq && (!kRepair || ((keep >> i) & 1u)))
         store_row<DP>(p.dq.p, b * p.dq.sb + hr * p.dq.sh + row * p.dq.sl, p.dq.sd, D, pp.dtype, pp.vec & kVecDq, l16, acc1[i], g.scale,
                       row0 + i < rows_valid);
     }
@@ -553,12 +554,12 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
 
 // One launch for both halves of the backward: dQ does not depend on dK / dV, so its CTAs fill the SMs as the last dK / dV
 // CTAs drain.
-template <int DP, int RT, class M>
+template <int DP, int RT, class M, bool kRepair>
 __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2))) simt_bwd_kernel(const __grid_constant__ BwdParams pp) {
   extern __shared__ float4 smem4[];
   float* sm = reinterpret_cast<float*>(smem4);
-  if ((int)blockIdx.x < pp.n_key_ctas) bwd_body<DP, RT, M, true>(pp, sm, (int)blockIdx.x);
-  else bwd_body<DP, RT, M, false>(pp, sm, (int)blockIdx.x - pp.n_key_ctas);
+  if ((int)blockIdx.x < pp.n_key_ctas) bwd_body<DP, RT, M, true, kRepair>(pp, sm, (int)blockIdx.x);
+  else bwd_body<DP, RT, M, false, kRepair>(pp, sm, (int)blockIdx.x - pp.n_key_ctas);
 }
 
 }  // namespace simt

@@ -20,9 +20,9 @@ namespace simt {
 constexpr int fwd_rows(int DP) { return DP <= 128 ? 8 : 4; }
 constexpr int bwd_rows(int DP) { return DP <= 64 ? 8 : (DP == 128 ? 4 : 2); }
 
-template <int DP, int RT>
+template <int DP, int RT, bool kRepair = false>
 static int fwd_one(const FwdParams& p, cudaStream_t st) {
-  auto kern = simt_fwd_kernel<DP, RT, InstMask>;
+  auto kern = simt_fwd_kernel<DP, RT, InstMask, kRepair>;
   constexpr int smem = FwdSmem<DP, RT>::kBytes;
   static_assert(smem <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
   struct Tag {};
@@ -38,15 +38,17 @@ template <int DP>
 static int fwd_dim(const FwdParams& p, cudaStream_t st) {
   constexpr int RT = fwd_rows(DP);
   const Geo& g = p.f.g;
-  if (p.repair) return fwd_one<DP, RT>(p, st);
+  if constexpr (DP <= 64) {  // the head dims of split.cuh
+    if (p.repair) return fwd_one<DP, RT, true>(p, st);
+  }
   const long long ctas = (long long)((g.Lq + 8 * RT - 1) / (8 * RT)) * g.H * g.B;
   if (2 * ctas < sm_count()) return fwd_one<DP, 2>(p, st);
   return fwd_one<DP, RT>(p, st);
 }
 
-template <int DP, int RT>
+template <int DP, int RT, bool kRepair = false>
 static int bwd_one(BwdParams p, int which, cudaStream_t st) {
-  auto kern = simt_bwd_kernel<DP, RT, InstMask>;
+  auto kern = simt_bwd_kernel<DP, RT, InstMask, kRepair>;
   constexpr int smem = BwdSmem<DP, RT>::kBytes;
   static_assert(smem <= 232448, "exceeds the 227 KB of shared memory a CTA can opt in to");
   struct Tag {};
@@ -64,7 +66,9 @@ static int bwd_one(BwdParams p, int which, cudaStream_t st) {
 template <int DP>
 static int bwd_dim(const BwdParams& p, int which, cudaStream_t st) {
   constexpr int RT = bwd_rows(DP);
-  if (p.repair) return bwd_one<DP, RT>(p, which, st);
+  if constexpr (DP <= 64) {
+    if (p.repair) return bwd_one<DP, RT, true>(p, which, st);
+  }
   if constexpr (RT > 2) {
     const Geo& g = p.b.g;
     const long long ctas = (long long)((g.Lk + 8 * RT - 1) / (8 * RT)) * g.Hkv * g.B + (long long)((g.Lq + 8 * RT - 1) / (8 * RT)) * g.H * g.B;
