@@ -1,4 +1,4 @@
-// fp32 attention in IEEE-like accuracy on the tensor cores (sm_100a): head dim <= 64, every operand as THREE bf16 parts.
+// fp32 attention in IEEE-like accuracy on the tensor cores (sm_100a): head dims 16, 32, 48 and 64, every operand as THREE bf16 parts.
 //
 // An fp32 number is exactly the sum of three bf16 numbers x = h + m + l (8 + 8 + 8 significand bits), and a product of two
 // bf16 numbers is exact in fp32.  Of the nine products of two such sums the kernels form six, hh, hm, mh, hl, mm and lh; the
@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
       float* orow = static_cast<float*>(p.o.p) + b * p.o.sb + h * p.o.sh + row * p.o.sl;
       store_row_f32(orow, o, 16);
       if (D > 16) store_row_f32(orow + 16, o + 16, 16);
-      if (D > 32) store_row_f32(orow + 32, o + 32, 32);
+      if (D > 32) store_row_f32(orow + 32, o + 32, 16);
+      if (D > 48) store_row_f32(orow + 48, o + 48, 16);
       if (p.lse != nullptr)
         p.lse[b * p.lse_sb + h * p.lse_sh + row * p.lse_sl] = valid ? (l == 0.f ? -CUDART_INF_F : m + log2f(l)) : 0.f;
     }

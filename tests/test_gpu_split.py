@@ -108,3 +108,52 @@ def test_values_bf16_cannot_hold(D, where, value):
     keys = see[rows].any(0)
     for x, y, hit in zip(a, base, (rows, rows, rows, keys, keys)):
         assert torch.equal(x[:, :, ~hit.to(x.device)], y[:, :, ~hit.to(x.device)])
+
+
+@pytest.mark.parametrize("mask_no", [0, 2])
+@pytest.mark.parametrize("layout", ["bhld", "blhd", "wide_rows"])
+@pytest.mark.parametrize("D", [16, 32, 48, 64])
+def test_nothing_but_the_rows_is_written(D, layout, mask_no):
+    """Every head dim the kernels take, 48 among them: results inside buffers whose other elements (before, between and behind the
+    rows) keep their value.  Rows 4 channels apart, heads in between ([batch, position, head, channel]), packed."""
+    from chill_attention import _cabi
+
+    mask, B, H, L, guard, fill = all_masks()[mask_no], 3, 24, 193, 256, 7.0
+    row = D + 4 if layout == "wide_rows" else D
+    strides = (L * H * row, row, H * row, 1) if layout == "blhd" else (H * L * row, L * row, row, 1)
+
+    def buffer():
+        return torch.full((B * H * L * row + 2 * guard,), fill, device="cuda")
+
+    def view(buf):
+        return buf.as_strided((B, H, L, D), strides, guard)
+
+    q, k, v, do = make_inputs(B, H, H, L, D, torch.float32, seed=D)
+    o_ref, lse_ref, *g_ref = oracle_all(mask, q, k, v, do)
+    q, k, v, do = (t.cuda() for t in (q, k, v, do))
+    buffers = [buffer() for _ in range(4)]
+    o, dq, dk, dv = (view(b) for b in buffers)
+    lse, delta = (torch.empty(B, H, L, device="cuda") for _ in range(2))
+    lib = _cabi.load_library()
+    shape = _cabi.make_shape(q, k, _cabi.BUILTIN_FUNCTOR_IDS[mask.cuda_functor], mask.constargs, None, D ** -0.5)
+    before = lib.chill_launch_count()
+    _cabi.forward(lib, q, k, v, o, lse, shape)
+    _cabi.backward(lib, q, k, v, o, do, lse, delta, dq, dk, dv, shape)
+    assert lib.chill_launch_count() - before == 5  # the split kernels ran, forward and backward
+    check_forward(o, lse, o_ref, lse_ref, None, torch.float32)
+    check_grads((dq, dk, dv), g_ref, torch.float32)
+    for buf in buffers:
+        view(buf).fill_(fill)
+        assert (buf == fill).all()
+
+
+def test_head_dim_48_from_host_memory():
+    """attention_fwd_bwd_host takes any head dim: packed heads, so that a row's neighbour is the next one."""
+    from chill_attention.host import attention_fwd_bwd_host
+
+    mask = all_masks()[1]
+    inputs = make_inputs(2, 16, 8, 257, 48, torch.float32, seed=48)
+    o_ref, _, *g_ref = oracle_all(mask, *inputs)
+    o, *grads = attention_fwd_bwd_host(*(t.pin_memory() for t in inputs), mask)
+    check_forward(o, None, o_ref, None, None, torch.float32)
+    check_grads(grads, g_ref, torch.float32)
