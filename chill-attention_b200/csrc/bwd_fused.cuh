@@ -113,7 +113,9 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int hi_l = imin(imin(hi, n - 1) - g.q_off, g.Lq - 1);
     if (hi_l >= lo_l) {
       n_qt = (hi_l - (lo_l & ~31)) / kTile + 1;
-      q_row0 = imin(lo_l & ~31, (n_qt_total - n_qt) * kTile);  // the last tile ends inside the accumulator
+      // The last tile does not end beyond the multiple of 128 behind the last such query: inside the accumulator, and before padding
+      // that starts there and may hold anything (0 * NaN is NaN).
+      q_row0 = imin(lo_l & ~31, (hi_l / kTile + 1 - n_qt) * kTile);
     }
     if (M::kHasQFullRange) M::q_full_range_for_k(kg0, kTile, n, g.margs, full_lo, full_hi);
   }

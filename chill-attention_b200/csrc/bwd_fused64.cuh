@@ -97,7 +97,8 @@ bwd_fused64_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int hi_l = imin(imin(hi, n - 1) - g.q_off, g.Lq - 1);
     if (hi_l >= lo_l) {
       n_qs = (hi_l - (lo_l & ~31)) / kF64Step + 1;
-      q_row0 = imin(lo_l & ~31, n_qt_total * kTile - n_qs * kF64Step);  // the last step ends inside the accumulator
+      // The last step does not end beyond the multiple of 64 behind the last such query (see bwd_fused.cuh).
+      q_row0 = imin(lo_l & ~31, (hi_l / kF64Step + 1 - n_qs) * kF64Step);
     }
     if (M::kHasQFullRange) M::q_full_range_for_k(kg0, kTile, n, g.margs, full_lo, full_hi);
   }

@@ -16,7 +16,9 @@
 //
 // The form with two streams (NS = 2) has the softmax warps, the issuer and the TMEM columns twice; see fwd_two_streams.
 // The first key tile starts at the first key the tile of queries can see, not at a multiple of its size: a window(16, 16) then
-// takes three 64-key tiles instead of four (fp16 (8,12,2085,64): 46 -> 39 us).
+// takes three 64-key tiles instead of four (fp16 (8,12,2085,64): 46 -> 39 us).  It starts earlier where the last tile would end
+// beyond the multiple of the tile size behind the last visible key: no key is multiplied that tiles at such multiples would leave
+// out, so padding that starts there may hold anything (0 * NaN is NaN).
 //
 // TMEM columns: kSBufs buffers of KT fp32 columns for S, each overlaid by its P (16-bit, first KT / 2
 // columns); then D columns of O.
@@ -320,8 +322,8 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     const int lo_l = imax(lo - g.k_off, 0);
     const int hi_l = imin(imin(hi, n - 1) - g.k_off, g.Lk - 1);
     if (hi_l >= lo_l) {
-      k_row0 = lo_l;
       n_tiles = (hi_l - lo_l) / KT + 1;
+      k_row0 = imin(lo_l, (hi_l / KT + 1 - n_tiles) * KT);
     }
     if (M::kHasKFullRange) M::k_full_range_for_q(qg0, kTile, n, g.margs, full_lo, full_hi);
   }

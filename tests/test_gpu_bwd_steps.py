@@ -66,3 +66,22 @@ def test_rows_whose_offset_needs_64_bits():
     g_ref = orc.attention_backward(md, q_l.double(), kc, vc, do_l.double(), **where)
     check_grads((dq[:, :, -live:], dk, dv), g_ref, dtype)
     assert not dq[:, :, :-live].any()
+
+
+@pytest.mark.parametrize("D,B", [(32, 40), (64, 2), (64, 40), (128, 2), (256, 2)])
+@pytest.mark.parametrize("mask_no", range(4))
+def test_padding_behind_the_last_tile_may_hold_anything(mask_no, D, B):
+    """lens at multiples of 128, NaN in all padded rows: tiles and steps that start between such multiples do not reach beyond them."""
+    import chill_attention as ca
+
+    mask = (ca.SlidingWindowChillMask(16, 16), ca.SlidingWindowChillMask(100, 0), ca.SlidingWindowChillMask(0, 70), ca.ChunkwiseChillMask(96, 1))[mask_no]
+    L, dtype = 512, torch.float16
+    clean = make_inputs(B, 3, 3, L, D, dtype, seed=D)
+    lens = torch.tensor(([384, 512, 128, 256] * B)[:B], dtype=torch.int32)
+    o_ref, lse_ref, *g_ref = oracle_all(mask, *clean, lens)
+    dirty = [t.masked_fill(torch.arange(L)[None, None, :, None] >= lens[:, None, None, None], float("nan")).cuda() for t in clean]
+    q, k, v = (t.requires_grad_(True) for t in dirty[:3])
+    o, lse = ca.chill_attention(q, k, v, mask=mask, lens=lens.cuda(), return_lse=True)
+    grads = torch.autograd.grad(o, (q, k, v), dirty[3])
+    check_forward(o, lse, o_ref, lse_ref, lens, dtype)
+    check_grads(grads, g_ref, dtype, lens)
