@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, (DP == 256 ? 1 : (RT == 2 ? 4 : 2)))
   const float c = g.scale * kLog2e;
   float m[RT], l[RT];
   uint64_t acc[RT][Lane<DP>::kPairs];
-  for (bool careful = false;; careful = true) {
+  for (bool careful = kRepair;; careful = true) {  // marked rows have met a non-finite number as a rule
 #pragma unroll
     for (int i = 0; i < RT; ++i) {
       m[i] = -CUDART_INF_F;
@@ -457,7 +457,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, float* sm, int til
       delta_r[i] = p.delta[((long long)b * g.H + hr) * g.Lq + rb + row0 + i];
     }
   }
-  for (bool careful = false;; careful = true) {
+  for (bool careful = kRepair;; careful = true) {  // marked rows have met a non-finite number as a rule
 #pragma unroll
     for (int i = 0; i < RT; ++i)
 #pragma unroll

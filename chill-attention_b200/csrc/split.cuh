@@ -13,8 +13,9 @@
 // Numbers bf16 cannot hold (NaN, Inf, |x| > 3.39e38) would make 0 * NaN of what the mask hides.  In a streamed tile they enter
 // the parts as zeros, the tile says which of its positions have one, and a row that sees such a position is not stored but
 // marked (kRepairMark in its first channel); so is a row that ends with a NaN of its own.  The CUDA-core kernel is launched
-// behind these and replaces the marked rows, all others keep their bits.  (A non-finite V only concerns its own channel of O:
-// the forward adds its product in fp32 and marks nothing.)
+// behind these and replaces the marked rows, all others keep their bits.  A non-finite V only concerns its own channel of O: the
+// forward adds up to four of them per row and stream to their channels and marks nothing; rows that see more are marked.  Time
+// with NaN in every element, (2,8,1000), split and repair / CUDA cores alone, us: q 284 / 377, k and v 331 / 377, backward 1110 / 1200.
 //
 // Measured against simt.cuh (full mask, head dim 64, us): (2,8,1000) forward 143 -> 44, backward 442 -> 130; (4,8,2048) forward
 // 938 -> 274, backward 2975 -> 825.  Distance from the 64-bit result (N(0, 1) inputs, 2-norm): O 5.9e-7 -> 2.0e-7, dQ, dK and dV
@@ -135,15 +136,17 @@ __device__ __forceinline__ uint32_t clean(TileRegs<kCols>& t) {
   }
   return rows;
 }
-// Positions with a replaced element, from the words of the four loader warps; f(position) for each.
+// Positions that clean() has found in the two streamed tiles of a step; words: of the four loader warps, for the first tile and for
+// the second.  f(position, in the first, in the second) for each.
 template <class F>
-__device__ __forceinline__ void for_unfit(const uint4 words, const F& f) {
-  if ((words.x | words.y | words.z | words.w) == 0) return;
+__device__ __forceinline__ void for_unfit(const uint4* words, const F& f) {
+  const uint4 a = words[0], b = words[1];
+  if ((a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w) == 0) return;
 #pragma unroll 1
   for (int pos = 0; pos < kCols; ++pos) {
-    const int w = (pos >> 2) & 3;
-    const uint32_t word = w == 0 ? words.x : (w == 1 ? words.y : (w == 2 ? words.z : words.w));
-    if ((word >> (4 * (pos >> 4) + (pos & 3))) & 1u) f(pos);
+    const int w = (pos >> 2) & 3, bit = 4 * (pos >> 4) + (pos & 3);
+    const bool in_a = (reinterpret_cast<const uint32_t*>(words)[w] >> bit) & 1u, in_b = (reinterpret_cast<const uint32_t*>(words)[4 + w] >> bit) & 1u;
+    if (in_a || in_b) f(pos, in_a, in_b);
   }
 }
 // The tile is visible to the tensor cores; one arrival per loader warp.
@@ -244,7 +247,9 @@ struct FwdSmem {
   static constexpr int kUnfit = kKv + 2 * kStream;  // per stream, for every other of its tiles: words of K, words of V (four each)
   static constexpr int kBars = kUnfit + 4 * 32;
   static constexpr int kMisc = kBars + 8 * 12;
-  static constexpr int kDynamic = kMisc + 16 + 1024;
+  static constexpr int kSeenV = 4;               // positions a row remembers (softmax threads: 256)
+  static constexpr int kSeen = kMisc + 16;
+  static constexpr int kDynamic = kSeen + kSeenV * 256 * 4 + 1024;
   static_assert(kRows * (64 + 4) * 4 <= kStream, "the merge uses the stream's tiles");
 };
 
@@ -345,17 +350,18 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
       TileRegs<kCols> rk, rv;
       rk.fetch(p.k, b, hk, kb, rows, D, tid);
       rv.fetch(p.v, b, hk, kb, rows, D, tid);
-      // The words of tile j - 4 have been read: its softmax was over before the scores of tile j - 2 were issued.
+      // The words of tile j - 4 have been read when P of tile j - 2 has been sent.
       uint32_t* words = reinterpret_cast<uint32_t*>(gen + L::kUnfit + 64 * w + 32 * ((j >> 1) & 1)) + (warp - 8);
-      const uint32_t bad_k = clean(rk), bad_v = clean(rv);
+      const uint32_t bad_k = clean(rk);
       if (j >= 2 && !warp_wait(bar_s + 8 * w, prev, guard, kStSplitLoad)) break;  // the scores of tile j - 2 have read K
+      rk.put(kv, kColPart, tid);
+      publish(bar_k + 8 * w, lane);
+      const uint32_t bad_v = clean(rv);
+      if (j >= 2 && !warp_wait(bar_o + 8 * w, prev, guard, kStSplitLoad)) break;  // P V of tile j - 2 has read V
       if (lane == 0) {
         words[0] = bad_k;
         words[4] = bad_v;
       }
-      rk.put(kv, kColPart, tid);
-      publish(bar_k + 8 * w, lane);
-      if (j >= 2 && !warp_wait(bar_o + 8 * w, prev, guard, kStSplitLoad)) break;  // P V of tile j - 2 has read V
       rv.put(kv + 3 * kColPart, kColPart, tid);
       publish(bar_v + 8 * w, lane);
     }
@@ -372,7 +378,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
     float o[64];
 #pragma unroll
     for (int i = 0; i < 64; ++i) o[i] = 0.f;
-    bool ok = true, repair = false, unfit_v = false;
+    bool ok = true, repair = false;
+    int n_v = 0;                               // unfit positions of V that this row sees; the first few of them:
+    int* seen_v = reinterpret_cast<int*>(gen + L::kSeen) + threadIdx.x;
     for (int j = w; j < n_tiles; j += 2) {
       const uint32_t par = (uint32_t)(j >> 1) & 1u;
       const int kb = (kt_lo + j) * kCols, kg0 = kb + g.k_off;
@@ -404,9 +412,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
       const float m_safe = (m_new == -CUDART_INF_F) ? 0.f : m_new;
       const float alpha = tc::ex2(m - m_safe);
       m = m_new;
-      const uint4* words = reinterpret_cast<const uint4*>(gen + L::kUnfit + 64 * w + 32 * par);
-      if ((words[1].x | words[1].y | words[1].z | words[1].w) != 0) unfit_v = true;
-      for_unfit(words[0], [&](int pos) { repair = repair || (qg < n && pos < ncols && M::mask(qg, kg0 + pos, n, g.margs)); });
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int q = 0; q < 4; ++q) {  // 16 positions: 8 columns of each part
@@ -428,6 +433,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
       if (lane == 0) tc::mbar_arrive(bar_p + 8 * w);
       if (!(ok = warp_wait(bar_o + 8 * w, par, guard, kStSplitCompute))) break;
       tc::tc_fence_after();
+      for_unfit(reinterpret_cast<const uint4*>(gen + L::kUnfit + 64 * w + 32 * par), [&](int pos, bool in_k, bool in_v) {
+        if (qg >= n || pos >= ncols || !M::mask(qg, kg0 + pos, n, g.margs)) return;
+        repair = repair || in_k;
+        if (in_v && n_v < L::kSeenV) seen_v[n_v * 256] = kb + pos;
+        n_v += in_v ? 1 : 0;
+      });
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         uint32_t t[32];
@@ -444,16 +455,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
     if (n_tiles > 1 && w == 1 && ok) {
 #pragma unroll
       for (int i = 0; i < 16; ++i) mo[i * kRows] = make_float4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
-      *ml = make_float4(m, l, repair ? 1.f : 0.f, unfit_v ? 1.f : 0.f);
+      *ml = make_float4(m, l, repair ? 1.f : 0.f, (float)n_v);
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(bar_merge);
     }
+    int n_v1 = 0;  // like n_v, of stream 1
     if (n_tiles > 1 && w == 0 && ok) {
       ok = warp_wait(bar_merge, 0, guard, kStSplitCompute);
       if (ok) {
         const float4 v = *ml;
         repair = repair || v.z != 0.f;
-        unfit_v = unfit_v || v.w != 0.f;
+        n_v1 = (int)v.w;
         const float m_all = fmaxf(m, v.x), m_safe = (m_all == -CUDART_INF_F) ? 0.f : m_all;
         const float a0 = tc::ex2(m - m_safe), a1 = tc::ex2(v.x - m_safe);
         m = m_all;
@@ -471,33 +483,30 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
     const int row = qb + r;
     if (w == 0 && ok && row < g.Lq) {
       const bool valid = qg < n;  // padded query rows: O = 0, LSE = 0
+      // Elements of V that went into the product as zeros: NaN and Inf are added to their channels, the others keep their bits.  A row
+      // that sees many such positions is left to the CUDA cores.
+      if (n_v > L::kSeenV || n_v1 > L::kSeenV) repair = true;
+#pragma unroll 1
+      for (int e = 0; e < n_v + n_v1 && !repair; ++e) {
+        const int pos = e < n_v ? seen_v[e * 256] : seen_v[(e - n_v) * 256 + 128];
+        const float* q = static_cast<const float*>(p.q.p) + b * p.q.sb + h * p.q.sh + (long long)row * p.q.sl;
+        const float* k = static_cast<const float*>(p.k.p) + b * p.k.sb + hk * p.k.sh + (long long)pos * p.k.sl;
+        const float* v = static_cast<const float*>(p.v.p) + b * p.v.sb + hk * p.v.sh + (long long)pos * p.v.sl;
+        float sc = 0.f;
+#pragma unroll 1
+        for (int i = 0; i < D; ++i) sc = fmaf(q[i], k[i], sc);
+        const float weight = tc::ex2(sc * (g.scale * kLog2e) - m);
+        if (weight == 0.f) continue;  // as if hidden, like simt.cuh
+#pragma unroll
+        for (int i = 0; i < 64; ++i) {
+          const float x = i < D ? v[i] : 0.f;
+          if (x - x != 0.f) o[i] += weight * x;
+          else if (fabsf(x) >= 3.39e38f) repair = true;  // finite, but too large for the parts
+        }
+      }
       const float inv = (valid && l != 0.f) ? 1.f / l : 0.f;
 #pragma unroll
       for (int i = 0; i < 64; ++i) o[i] = valid ? o[i] * inv : 0.f;
-      if (unfit_v && valid && !repair) {
-        // V went into the product without its non-finite elements: they are looked up again and added to their channels
-        const float* q = static_cast<const float*>(p.q.p) + b * p.q.sb + h * p.q.sh + (long long)row * p.q.sl;
-#pragma unroll 1
-        for (int pos = kt_lo * kCols; pos < imin(kt_hi * kCols, imin(n - g.k_off, g.Lk)); ++pos) {
-          if (!M::mask(qg, pos + g.k_off, n, g.margs)) continue;
-          const float* k = static_cast<const float*>(p.k.p) + b * p.k.sb + hk * p.k.sh + (long long)pos * p.k.sl;
-          const float* v = static_cast<const float*>(p.v.p) + b * p.v.sb + hk * p.v.sh + (long long)pos * p.v.sl;
-          bool any = false;
-#pragma unroll 1
-          for (int i = 0; i < D; ++i) any = any || unfit(v[i]);
-          if (!any) continue;
-          float sc = 0.f;
-#pragma unroll 1
-          for (int i = 0; i < D; ++i) sc = fmaf(q[i], k[i], sc);
-          const float weight = tc::ex2(sc * c - m);
-          if (weight == 0.f) continue;  // as if hidden, like simt.cuh
-#pragma unroll
-          for (int i = 0; i < 64; ++i) {
-            const float x = i < D ? v[i] : 0.f;
-            if (unfit(x)) o[i] += weight * inv * x;
-          }
-        }
-      }
       if (valid && (repair || l != l)) o[0] = __uint_as_float(kRepairMark);
       float* orow = static_cast<float*>(p.o.p) + b * p.o.sb + h * p.o.sh + row * p.o.sl;
       store_row_f32(orow, o, 16);
@@ -651,14 +660,15 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
       a.fetch(c1, b, hc, cb, rows, D, tid);
       d.fetch(c2, b, hc, cb, rows, D, tid);
       uint32_t* words = reinterpret_cast<uint32_t*>(gen + L::kUnfit + 32 * s) + (warp - 8);
-      const uint32_t bad1 = clean(a), bad2 = clean(d);
+      const uint32_t bad1 = clean(a);
       if (it >= 2 && !warp_wait(bar_acc + 8 * s, prev, guard, kStSplitLoad)) break;  // step it - 2 has read its tiles
+      a.put(st, kColPart, tid);
+      publish(bar_c1 + 8 * s, lane);
+      const uint32_t bad2 = clean(d);
       if (lane == 0) {
         words[0] = bad1;
         words[4] = bad2;
       }
-      a.put(st, kColPart, tid);
-      publish(bar_c1 + 8 * s, lane);
       d.put(st + 3 * kColPart, kColPart, tid);
       publish(bar_c2 + 8 * s, lane);
       if (++ct == ct_hi) {
@@ -747,12 +757,9 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
       const bool full = has_full && cg0 >= full_lo && cg0 + kCols <= full_hi && ncols >= kCols && rows_valid == kRows;
       if (!(ok = warp_wait(bar_s, par, guard, kStSplitCompute))) break;
       tc::tc_fence_after();
-      const uint4* words = reinterpret_cast<const uint4*>(gen + L::kUnfit + 32 * (it & 1));
       auto sees = [&](int cc) {
         return rg < n && cc < ncols && (kKeyRows ? M::mask(cg0 + cc, rg, n, g.margs) : M::mask(rg, cg0 + cc, n, g.margs));
       };
-#pragma unroll
-      for (int e = 0; e < 2; ++e) for_unfit(words[e], [&](int pos) { repair = repair || sees(pos); });
       float pe[32];
       load_scores16(tS + lane_sel + c0, pe);
       load_scores16(tS + lane_sel + c0 + 16, pe + 16);
@@ -789,6 +796,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
       if (kKeyRows) send(tS + lane_sel + c0, bar_p, pe);
       if (!(ok = warp_wait(bar_dp, par, guard, kStSplitCompute))) break;
       tc::tc_fence_after();
+      for_unfit(reinterpret_cast<const uint4*>(gen + L::kUnfit + 32 * (it & 1)), [&](int pos, bool, bool) { repair = repair || sees(pos); });
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         float d[16];
