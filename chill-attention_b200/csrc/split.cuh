@@ -1,8 +1,9 @@
 // fp32 attention in IEEE-like accuracy on the tensor cores (sm_100a): head dims 16, 32, 48 and 64, every operand as THREE bf16 parts.
 //
-// An fp32 number is exactly the sum of three bf16 numbers x = h + m + l (8 + 8 + 8 significand bits), and a product of two
-// bf16 numbers is exact in fp32.  Of the nine products of two such sums the kernels form six, hh, hm, mh, hl, mm and lh; the
-// others are below 2^-26 of |x y|.  So a GEMM costs six bf16 MMAs, which is still a multiple of the CUDA cores' fp32 rate.
+// An fp32 number of at least 2^-110 is exactly the sum of three bf16 numbers x = h + m + l (8 + 8 + 8 significand bits), and a
+// product of two bf16 numbers is exact in fp32.  Of the nine products of two such sums the kernels form six, hh, hm, mh, hl, mm and
+// lh; ml and lm are each at most 2^-25 of |x y| and ll 2^-34, together one rounding of fp32 at most.  So a GEMM costs six bf16 MMAs,
+// which is still a multiple of the CUDA cores' fp32 rate.
 //
 // What would cost accuracy is not the split but the tensor core's accumulator, which truncates: its error is one-sided and
 // grows with the number of additions.  It is kept below that of a chain of rounded fp32 FMAs (simt.cuh) by
@@ -10,9 +11,10 @@
 //     of one tile (64 channels or 64 positions: four MMA steps) is ever truncated at full magnitude, and
 //   * starting every tile's product from zero and adding the tiles up in registers, rounded.
 //
-// Numbers bf16 cannot hold (NaN, Inf, |x| > 3.39e38) would make 0 * NaN of what the mask hides.  In a streamed tile they enter
-// the parts as zeros, the tile says which of its positions have one, and a row that sees such a position is not stored but
-// marked (kRepairMark in its first channel); so is a row that ends with a NaN of its own.  The CUDA-core kernel is launched
+// What the parts cannot hold: NaN, Inf and |x| > 3.39e38 would make 0 * NaN of what the mask hides, and numbers below 2^-110 are no
+// sum of three bf16 numbers any more.  The first enter the parts of a streamed tile as zeros; the tile says which of its positions
+// have one, or eight channels that are all smaller than 2^-94, and a row that sees such a position is not stored but marked
+// (kRepairMark in its first channel); so is a row that has such channels itself or ends with a NaN.  The CUDA-core kernel is launched
 // behind these and replaces the marked rows, all others keep their bits.  A non-finite V only concerns its own channel of O: the
 // forward adds up to four of them per row and stream to their channels and marks nothing; rows that see more are marked.  Time
 // with NaN in every element, (2,8,1000), split and repair / CUDA cores alone, us: q 284 / 377, k and v 331 / 377, backward 1110 / 1200.
@@ -43,6 +45,11 @@ constexpr int kCols = 64;                       // streamed positions per step
 constexpr int kRowPart = kRows * 128;           // one bf16 part of a row operand: 128 rows of one 128-byte line
 constexpr int kColPart = kCols * 128;           // one part of a streamed tile
 constexpr int kLoaders = 128;                   // threads that load and split
+// Eight neighbouring channels of a position go into the parts as they are if the largest is 0 or in [kLeast, kMost): kMost is what
+// bf16 can hold; elements below 2^-110 lose the bits of their third part that lie under bf16's smallest subnormal, 2^-133, which is
+// less than 2^-39 of a neighbour of kLeast.
+constexpr float kLeast = 0x1p-94f, kMost = 3.39e38f;
+constexpr float kUp = 65536.f, kDown = 1.f / kUp;  // dS is split times 2^16: it may be tiny although V and dO are not
 
 enum : int { kStSplitLoad = 701, kStSplitMma = 702, kStSplitCompute = 703 };
 
@@ -68,6 +75,13 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& h, uint32_t& 
   l = tc::pack2<BF>(a - x, b - y);
 }
 
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {  // of the magnitudes; NaN if one is
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
+  return d;
+}
+__device__ __forceinline__ bool unfit(float x) { return !(fabsf(x) < kMost); }
+
 // ROWS x 64 fp32 elements of one (batch, head), eight channels of a row per thread and unit: from global memory into
 // registers, and from there as three parts into 128B-swizzled shared memory.  Rows beyond rows_in and channels beyond D are
 // zero and not read.
@@ -88,6 +102,11 @@ struct TileRegs {
       }
     }
   }
+  // magnitude of the largest element of unit i, NaN if one is
+  __device__ __forceinline__ float largest(int i) const {
+    const float4 &a = v[i][0], &b = v[i][1];
+    return max3_nan(max3_nan(a.x, a.y, a.z), max3_nan(a.w, b.x, b.y), max3_nan(b.z, b.w, 0.f));
+  }
   __device__ __forceinline__ void put(uint8_t* dst, int part_bytes, int tid) const {
 #pragma unroll
     for (int i = 0; i < kUnits; ++i) {
@@ -104,21 +123,15 @@ struct TileRegs {
     }
   }
 };
-// A streamed tile: elements that bf16 cannot hold are replaced by zeros.  Returns, to every lane, which of this warp's rows had
-// one: bit 4 i + e stands for row 16 i + 4 (warp) + e.
-__device__ __forceinline__ bool unfit(float x) { return !(fabsf(x) < 3.39e38f); }
-__device__ __forceinline__ float max3_nan(float a, float b, float c) {  // of the magnitudes; NaN if one is
-  float d;
-  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
-  return d;
-}
+// A streamed tile: elements that bf16 cannot hold are replaced by zeros.  Returns, to every lane, which of this warp's rows have
+// channels that are no part of a sum of parts (NaN, Inf, too large, too small): bit 4 i + e stands for row 16 i + 4 (warp) + e.
 __device__ __forceinline__ uint32_t clean(TileRegs<kCols>& t) {
   constexpr int N = TileRegs<kCols>::kUnits;
   bool bad[N], any = false;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
-    const float4 &a = t.v[i][0], &b = t.v[i][1];
-    bad[i] = unfit(max3_nan(max3_nan(a.x, a.y, a.z), max3_nan(a.w, b.x, b.y), max3_nan(b.z, b.w, 0.f)));
+    const float mx = t.largest(i);
+    bad[i] = unfit(mx) || (mx < kLeast && mx > 0.f);
     any = any || bad[i];
   }
   uint32_t rows = 0;
@@ -135,6 +148,23 @@ __device__ __forceinline__ uint32_t clean(TileRegs<kCols>& t) {
     }
   }
   return rows;
+}
+// Rows of half a resident tile with channels that are too small, like clean(); NaN, Inf and too large ones make the row's results
+// NaN by themselves.
+__device__ __forceinline__ uint32_t small_rows(const TileRegs<64>& t) {
+  uint32_t rows = 0;
+#pragma unroll
+  for (int i = 0; i < TileRegs<64>::kUnits; ++i) {
+    const float mx = t.largest(i);
+    const uint32_t who = __ballot_sync(0xffffffffu, mx < kLeast && mx > 0.f);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) rows |= ((who >> (8 * e)) & 0xffu) != 0 ? 1u << (4 * i + e) : 0u;
+  }
+  return rows;
+}
+// Whether row r of the resident tile is one of them; words: [half][loader warp].
+__device__ __forceinline__ bool is_small(const uint32_t* words, int r) {
+  return ((words[(r >> 6) * 4 + ((r >> 2) & 3)] >> (4 * ((r >> 4) & 3) + (r & 3))) & 1u) != 0;
 }
 // Positions that clean() has found in the two streamed tiles of a step; words: of the four loader warps, for the first tile and for
 // the second.  f(position, in the first, in the second) for each.
@@ -248,7 +278,8 @@ struct FwdSmem {
   static constexpr int kBars = kUnfit + 4 * 32;
   static constexpr int kMisc = kBars + 8 * 12;
   static constexpr int kSeenV = 4;               // positions a row remembers (softmax threads: 256)
-  static constexpr int kSeen = kMisc + 16;
+  static constexpr int kRowSmall = kMisc + 16;   // see is_small
+  static constexpr int kSeen = kRowSmall + 32;
   static constexpr int kDynamic = kSeen + kSeenV * 256 * 4 + 1024;
   static_assert(kRows * (64 + 4) * 4 <= kStream, "the merge uses the stream's tiles");
 };
@@ -286,6 +317,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
   const uint32_t bar_k = bars, bar_v = bars + 16, bar_s = bars + 32, bar_p = bars + 48, bar_o = bars + 64, bar_q = bars + 80, bar_merge = bars + 88;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::kMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::kMisc + 4);
+  uint32_t* row_small = reinterpret_cast<uint32_t*>(gen + L::kRowSmall);
   const Guard guard{pp.status, abort_flag};
   if (warp == 12) {
     if (lane == 0) {
@@ -339,6 +371,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
         r.fetch(p.q, b, h, qb + 64 * half, q_rows - 64 * half, D, tid);
+        const uint32_t small = small_rows(r);
+        if (lane == 0) row_small[4 * half + warp - 8] = small;
         r.put(gen + L::kQ + 64 * half * 128, kRowPart, tid);
       }
       publish(bar_q, lane);
@@ -485,7 +519,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
       const bool valid = qg < n;  // padded query rows: O = 0, LSE = 0
       // Elements of V that went into the product as zeros: NaN and Inf are added to their channels, the others keep their bits.  A row
       // that sees many such positions is left to the CUDA cores.
-      if (n_v > L::kSeenV || n_v1 > L::kSeenV) repair = true;
+      if (n_v > L::kSeenV || n_v1 > L::kSeenV || (n_tiles > 0 && is_small(row_small, r))) repair = true;
 #pragma unroll 1
       for (int e = 0; e < n_v + n_v1 && !repair; ++e) {
         const int pos = e < n_v ? seen_v[e * 256] : seen_v[(e - n_v) * 256 + 128];
@@ -498,10 +532,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) split_fwd_kernel(const __grid_
         const float weight = tc::ex2(sc * (g.scale * kLog2e) - m);
         if (weight == 0.f) continue;  // as if hidden, like simt.cuh
 #pragma unroll
-        for (int i = 0; i < 64; ++i) {
-          const float x = i < D ? v[i] : 0.f;
-          if (x - x != 0.f) o[i] += weight * x;
-          else if (fabsf(x) >= 3.39e38f) repair = true;  // finite, but too large for the parts
+        for (int i = 0; i < 64; i += 8) {
+          float mx = 0.f;  // of the finite ones
+#pragma unroll
+          for (int ii = i; ii < i + 8; ++ii) {
+            const float x = ii < D ? v[ii] : 0.f;
+            if (x - x != 0.f) o[ii] += weight * x;
+            else mx = fmaxf(mx, fabsf(x));
+          }
+          if (mx >= kMost || (mx < kLeast && mx > 0.f)) repair = true;
         }
       }
       const float inv = (valid && l != 0.f) ? 1.f / l : 0.f;
@@ -542,7 +581,8 @@ struct BwdSmem {
   static constexpr int kUnfit = kBad + kRows * 4;  // per stage: words of C1, words of C2 (four each)
   static constexpr int kBars = kUnfit + 2 * 32;
   static constexpr int kMisc = kBars + 8 * 14;
-  static constexpr int kDynamic = kMisc + 16 + 1024;
+  static constexpr int kRowSmall = kMisc + 16;       // see is_small
+  static constexpr int kDynamic = kRowSmall + 32 + 1024;
 };
 
 template <class M, bool kKeyRows>
@@ -585,6 +625,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
                  bar_c2 = bars + 64, bar_acc = bars + 80;
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gen + L::kMisc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + L::kMisc + 4);
+  uint32_t* row_small = reinterpret_cast<uint32_t*>(gen + L::kRowSmall);
   const Guard guard{pp.status, abort_flag};
   if (warp == 12) {
     if (lane == 0) {
@@ -645,8 +686,11 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
         r.fetch(r1, b, hr, rb + 64 * half, rows_valid - 64 * half, D, tid);
+        uint32_t small = small_rows(r);
         r.put(gen + L::kR1 + 64 * half * 128, kRowPart, tid);
         r.fetch(r2, b, hr, rb + 64 * half, rows_valid - 64 * half, D, tid);
+        small |= small_rows(r);
+        if (lane == 0) row_small[4 * half + warp - 8] = small;
         r.put(gen + L::kR2 + 64 * half * 128, kRowPart, tid);
       }
       publish(bar_r, lane);
@@ -686,11 +730,11 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
     const int rg = rg0 + r;
     const float c = g.scale * kLog2e;
     float* vec = reinterpret_cast<float*>(gen + L::kVec) + warp * 64;  // warp-private
-    float row_nl = 0.f, row_nd = 0.f;      // dQ part: -LSE and -delta of this row
+    float row_nl = 0.f, row_nd = 0.f;      // dQ part: -LSE and -delta (times 2^16) of this row
     if (!kKeyRows && rb + r < g.Lq) {
       const float v = p.lse[b * p.lse_sb + hr * p.lse_sh + (rb + r) * p.lse_sl];
       row_nl = v == -CUDART_INF_F ? 0.f : -v;
-      row_nd = -p.delta[((long long)b * g.H + hr) * g.Lq + rb + r];
+      row_nd = -p.delta[((long long)b * g.H + hr) * g.Lq + rb + r] * kUp;
     }
     float acc1[32], acc2[kKeyRows ? 32 : 1];
 #pragma unroll
@@ -749,7 +793,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
       if (kKeyRows) {
         __syncwarp();
         vec[lane] = nl_next == -CUDART_INF_F ? 0.f : -nl_next;
-        vec[32 + lane] = -nd_next;
+        vec[32 + lane] = -nd_next * kUp;
         __syncwarp();
         if (it + 1 < n_it) fetch_vec();
       }
@@ -805,10 +849,10 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
         for (int i = 0; i < 16; i += 4) {
           float4 nd = make_float4(row_nd, row_nd, row_nd, row_nd);
           if (kKeyRows) nd = *reinterpret_cast<const float4*>(vec + 32 + q * 16 + i);
-          pe[q * 16 + i] *= d[i] + nd.x;
-          pe[q * 16 + i + 1] *= d[i + 1] + nd.y;
-          pe[q * 16 + i + 2] *= d[i + 2] + nd.z;
-          pe[q * 16 + i + 3] *= d[i + 3] + nd.w;
+          pe[q * 16 + i] *= fmaf(d[i], kUp, nd.x);
+          pe[q * 16 + i + 1] *= fmaf(d[i + 1], kUp, nd.y);
+          pe[q * 16 + i + 2] *= fmaf(d[i + 2], kUp, nd.z);
+          pe[q * 16 + i + 3] *= fmaf(d[i + 3], kUp, nd.w);
         }
       }
       if (!full) {  // once more: delta of a hidden query may be NaN
@@ -821,7 +865,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
 
     // ---- rows: this thread has channels [c0, c0 + 32) of one row; the first warpgroup marks a row with a NaN in either half
     volatile int* bad = reinterpret_cast<volatile int*>(gen + L::kBad);
-    float nan = repair ? CUDART_NAN_F : 0.f;
+    float nan = repair || (n_it > 0 && is_small(row_small, r)) ? CUDART_NAN_F : 0.f;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       nan += acc1[i] - acc1[i];
@@ -839,7 +883,7 @@ __device__ __forceinline__ void bwd_body(const BwdParams& pp, uint8_t* smem_raw,
       const TRef& t1 = kKeyRows ? p.dk : p.dq;
       float* d1 = static_cast<float*>(t1.p) + b * t1.sb + hr * t1.sh + (long long)(rb + r) * t1.sl + c0;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) acc1[i] = valid ? acc1[i] * g.scale : 0.f;
+      for (int i = 0; i < 32; ++i) acc1[i] = valid ? acc1[i] * (g.scale * kDown) : 0.f;
       if (valid && wg == 0 && (nan != nan || bad[r] != 0)) acc1[0] = __uint_as_float(kRepairMark);
       store_row_f32(d1, acc1, 16);
       if (c0 + 16 < D) store_row_f32(d1 + 16, acc1 + 16, 16);
