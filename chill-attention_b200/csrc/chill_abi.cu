@@ -35,6 +35,14 @@ static int* device_status_ptr() {
   return p;
 }
 
+// The same for the split fp32 kernels, which the CUDA-core kernels can stand in for: without the word they are left out, and the
+// error that says so is not left behind for the launch that follows.
+static int* split_status_ptr() {
+  int* p = device_status_ptr();
+  if (p == nullptr) (void)cudaGetLastError();
+  return p;
+}
+
 // ------------------------------------------------------------------------- validation
 static size_t esize(int dtype) { return dtype == CHILL_F32 ? 4 : 2; }
 
@@ -257,10 +265,11 @@ static int fwd_generic(const chill_fwd_args& a, cudaStream_t st) {
   pp.vec = vec_bit(simt::kVecQ, a.q, a.q_strides, dt, D) | vec_bit(simt::kVecK, a.k, a.k_strides, dt, D) |
            vec_bit(simt::kVecV, a.v, a.v_strides, dt, D) | vec_bit(simt::kVecO, a.o, a.o_strides, dt, D);
   int e = 0;
-  if (pp.vec == (simt::kVecQ | simt::kVecK | simt::kVecV | simt::kVecO) && split_pays(a.s, 8192)) {
+  int* status = nullptr;
+  if (pp.vec == (simt::kVecQ | simt::kVecK | simt::kVecV | simt::kVecO) && split_pays(a.s, 8192) && (status = split_status_ptr()) != nullptr) {
     split::FwdParams sp;
     sp.f = p;
-    sp.status = device_status_ptr();
+    sp.status = status;
     CHILL_MASK_SWITCH(a.s.mask.id, (e = split_launch_fwd<MaskT>(sp, st)))
     if (e != 0) return cuda_fail((cudaError_t)e, "split_fwd launch");
     g_launches += 1;
@@ -446,10 +455,11 @@ static int bwd_generic(const chill_bwd_args& a, cudaStream_t st) {
            vec_bit(simt::kVecDq, a.dq, a.dq_strides, dt, D) | vec_bit(simt::kVecDk, a.dk, a.dk_strides, dt, D) |
            vec_bit(simt::kVecDv, a.dv, a.dv_strides, dt, D);
   int e = 0;
-  if (pp.vec == (255u & ~(uint32_t)simt::kVecO) && a.dk_part == nullptr && split_pays(a.s, 5120)) {
+  int* status = nullptr;
+  if (pp.vec == (255u & ~(uint32_t)simt::kVecO) && a.dk_part == nullptr && split_pays(a.s, 5120) && (status = split_status_ptr()) != nullptr) {
     split::BwdParams sp;
     sp.b = pp.b;
-    sp.status = device_status_ptr();
+    sp.status = status;
     CHILL_MASK_SWITCH(a.s.mask.id, (e = split_launch_bwd<MaskT>(sp, bwd_which(a.s.flags), st)))
     if (e != 0) return cuda_fail((cudaError_t)e, "split_bwd launch");
     g_launches += 1;
