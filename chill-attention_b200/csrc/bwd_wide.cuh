@@ -47,12 +47,10 @@ struct WideSmem {
   static constexpr int kBars = kVec + 8 * 2 * 32 * 4;
   static constexpr int kNumBars = 14;
   static constexpr int kMisc = kBars + 8 * kNumBars;
-  static constexpr int kTotal = kMisc + 16;
-  // 1 KB for aligning the base by hand, or what is left of it (dynamic shared memory starts aligned as a rule)
-  static constexpr int kDynamic = kTotal + 1024 <= 232448 ? kTotal + 1024 : 232448;
+  static constexpr int kDynamic = kMisc + 16;  // the array is declared with its alignment: there is no room to align it by hand
 };
 
-enum : int { kStWideProducer = 501, kStWideMma = 502, kStWideCompute = 503, kStWideEpilogue = 504, kStWideAlign = 505 };
+enum : int { kStWideProducer = 501, kStWideMma = 502, kStWideCompute = 503, kStWideEpilogue = 504 };
 
 // maps: R1, R2 = 128-row boxes of the row operands; C1, C2 = 64-row boxes of the streamed operands; OUT = 128-row
 // box of the gradient written.  kWideDV: R1 = K, (R2 unused), C1 = Q, C2 = dO, OUT = dV.  kWideDK: R1 = K, R2 = V,
@@ -111,13 +109,9 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
     return;
   }
 
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  uint8_t* gen_base = smem_raw + (base - smem_u32(smem_raw));
-  if (base + L::kTotal > smem_u32(smem_raw) + L::kDynamic) {  // the base was not aligned: nothing is computed
-    if (threadIdx.x == 0) atomicCAS(p.status, 0, kStWideAlign);
-    return;
-  }
+  extern __shared__ __align__(1024) uint8_t smem_wide[];  // the 128-byte swizzle repeats every 1 KB
+  uint8_t* gen_base = smem_wide;
+  const uint32_t base = smem_u32(smem_wide);
   const uint32_t sR1 = base + L::kR1, sR2 = base + L::kR2, sE = base + L::kE, sL = base + L::kL;
   const uint32_t bars = base + L::kBars;
   // "Early" tile: Q for dV, dO / V for dK / dQ, read by one score GEMM (e_done: that GEMM has finished).  "Late" tile: also, or
