@@ -36,13 +36,16 @@ ABI_VERSION = 5
 FLAG_BWD_DETERMINISTIC = 32
 FLAG_NARROW_HEAD = 64
 SELFTEST_STATUS = 901
+#: answers of chill_fwd_kernel
+FWD_CUDA_CORES, FWD_ONE_STREAM, FWD_TWO_STREAMS, FWD_TF32 = range(4)
 #: answers of chill_bwd_kernels
 BWD_CUDA_CORES, BWD_TWO_KERNELS, BWD_SINGLE, BWD_SINGLE_PAIR, BWD_WIDE, BWD_TF32 = range(6)
 
 EXPORTS = (
     "chill_fwd", "chill_bwd_delta", "chill_bwd", "chill_bwd_noalloc", "chill_bwd_scratch_bytes", "chill_bwd_dq_accum_bytes",
     "chill_fwd_uses_tensor_cores",
-    "chill_bwd_uses_tensor_cores", "chill_bwd_kernels", "chill_mask_tabulate", "chill_mask_tabulate_blocks", "chill_mask_traits",
+    "chill_bwd_uses_tensor_cores", "chill_fwd_kernel", "chill_bwd_kernels", "chill_mask_tabulate", "chill_mask_tabulate_blocks",
+    "chill_mask_traits",
     "chill_read_device_status", "chill_selftest_bounded_wait",
     "chill_launch_count", "chill_abi_version", "chill_status_string", "chill_last_cuda_error",
     "chill_host_workspace_bytes", "chill_fwd_bwd_host", "chill_host_chunk_schedule",
@@ -119,6 +122,7 @@ def load_library(path: str | None = None) -> C.CDLL:
         lib.chill_bwd_dq_accum_bytes.restype = C.c_size_t
         lib.chill_fwd_uses_tensor_cores.argtypes = [C.POINTER(FwdArgs)]
         lib.chill_bwd_uses_tensor_cores.argtypes = [C.POINTER(BwdArgs)]
+        lib.chill_fwd_kernel.argtypes = [C.POINTER(FwdArgs)]
         lib.chill_bwd_kernels.argtypes = [C.POINTER(BwdArgs)]
         lib.chill_mask_tabulate.argtypes = [C.POINTER(MaskDesc), C.c_int32, C.c_int32] + [C.c_void_p] * 6
         lib.chill_mask_tabulate_blocks.argtypes = [C.POINTER(MaskDesc), C.c_int32, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]
@@ -135,7 +139,7 @@ def load_library(path: str | None = None) -> C.CDLL:
         lib.chill_host_chunk_schedule.argtypes = [C.POINTER(HostArgs), C.POINTER(C.c_int32), C.c_int32]
         lib.chill_host_chunk_schedule.restype = C.c_int
         for name in ("chill_fwd", "chill_bwd_delta", "chill_bwd", "chill_bwd_noalloc", "chill_fwd_uses_tensor_cores",
-                     "chill_bwd_uses_tensor_cores", "chill_bwd_kernels", "chill_mask_tabulate", "chill_mask_tabulate_blocks",
+                     "chill_bwd_uses_tensor_cores", "chill_fwd_kernel", "chill_bwd_kernels", "chill_mask_tabulate", "chill_mask_tabulate_blocks",
                      "chill_mask_traits", "chill_selftest_bounded_wait",
                      "chill_read_device_status", "chill_abi_version"):
             getattr(lib, name).restype = C.c_int

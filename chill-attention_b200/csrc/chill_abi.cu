@@ -223,6 +223,15 @@ static bool fwd_tc_eligible(const chill_fwd_args& a) {
          tma_ok(a.v, a.v_strides, s.B, s.H_kv, s.Lk, es) && tma_ok(a.o, a.o_strides, s.B, s.H, s.Lq, es);
 }
 
+// CHILL_FWD_*: the kernel that serves a forward call (include/chill_b200.h).
+static int fwd_kernel(const chill_fwd_args& a) {
+  if (!fwd_tc_eligible(a)) return CHILL_FWD_CUDA_CORES;
+  if (a.s.dtype == CHILL_F32) return CHILL_FWD_TF32;
+  bool two = false;
+  CHILL_MASK_SWITCH(a.s.mask.id, (two = tc_fwd_two_streams<MaskT>(to_geo(a.s), a.s.D <= 64 ? 64 : a.s.D)))
+  return two ? CHILL_FWD_TWO_STREAMS : CHILL_FWD_ONE_STREAM;
+}
+
 static int check_fwd(const chill_fwd_args* a) {
   if (a == nullptr) return CHILL_E_INVALID;
   int st = check_shape(a->s);
@@ -713,6 +722,11 @@ int chill_bwd_uses_tensor_cores(const chill_bwd_args* a) {
   int st = check_bwd(a, true);
   if (st != CHILL_OK) return st;
   return (bwd_tc_eligible(*a) || bwd_wide_eligible(*a) || bwd_tf32_eligible(*a)) ? 1 : 0;
+}
+
+int chill_fwd_kernel(const chill_fwd_args* a) {
+  int st = check_fwd(a);
+  return st != CHILL_OK ? st : fwd_kernel(*a);
 }
 
 int chill_bwd_kernels(const chill_bwd_args* a) {

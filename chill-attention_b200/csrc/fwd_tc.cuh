@@ -571,9 +571,10 @@ fwd_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 // streams in us (bf16; graph replays):
 //   D = 128  (1,4,4096) full, 128 CTAs of 64 steps: 52.5 / 37.6   (1,8,1000), 16 steps: 16.8 / 16.2   (1,32,512), 8 steps: 11.2 / 12.3
 //            (1,16,2048), 256 CTAs: 35.4 / 45.1
-//   D = 64   (1,4,4096) full: 78.8 / 57.5   (1,16,2048), 256 CTAs: 46.8 / 39.7   (1,32,512): 13.5 / 12.3   window(256, 0), 6 steps:
-//            11.8 / 11.4   (2,8,300), 5 steps: 9.9 / 10.3   512 CTAs: full (2,16,2048) 66.9 / 72.7, causal (2,16,2048), 32 steps at
-//            most: 55.2 / 53.4, causal (2,4,8192): 161 / 121, causal (8,8,1024), 16 at most: 35.5 / 36.6
+//   D = 64   (1,4,4096) full: 78.8 / 57.5   (1,16,2048), 256 CTAs: 46.8 / 39.7   (1,32,512), 8 steps: 13.5 / 12.3   6 steps:
+//            chunkwise(128, 2) (1,8,4096), 256 CTAs 13.6 / 14.3, (8,12,384) full-width rows, 288 CTAs 13.8 / 14.6, few CTAs 11.5 / 11.0
+//            512 CTAs: full (2,16,2048) 66.9 / 72.7, causal (2,16,2048), 32 steps at most: 55.2 / 53.4, causal (2,4,8192): 161 / 121,
+//            causal (8,8,1024), 16 at most: 35.5 / 36.6
 template <class M>
 bool fwd_two_streams(const Geo& g, int D, int ctas) {
   const int sms = sm_count(), resident = sms * FwdShape<64, 2>::kCtasPerSm;
@@ -582,7 +583,7 @@ bool fwd_two_streams(const Geo& g, int D, int ctas) {
   int most;
   count_steps<M>(g, total, most);
   if (D == 128) return most >= 16;
-  return ctas <= resident ? most >= 6 : most >= 32 && 3 * total <= 2ll * most * ctas;
+  return ctas <= resident ? most >= 7 : most >= 32 && 3 * total <= 2ll * most * ctas;
 }
 
 }  // namespace tc

@@ -29,9 +29,15 @@ static int launch_fwd_one(const CUtensorMap* maps, const tc::FwdTcParams& p, dim
   return (int)cudaGetLastError();
 }
 
+template <>
+bool tc_fwd_two_streams<InstMask>(const Geo& g, int D) {
+  const long long ctas = (long long)((g.Lq + tc::kTile - 1) / tc::kTile) * g.H * g.B;
+  return D <= 128 && ctas <= 0x7fffffffll && tc::fwd_two_streams<InstMask>(g, D, (int)ctas);
+}
+
 template <typename T>
 static int launch_fwd_dim(int D, const CUtensorMap* maps, const tc::FwdTcParams& p, dim3 grid, cudaStream_t st) {
-  const bool two = D <= 128 && tc::fwd_two_streams<InstMask>(p.g, D, (int)grid.x);
+  const bool two = tc_fwd_two_streams<InstMask>(p.g, D);
   if (D == 128) return two ? launch_fwd_one<T, 128, 2>(maps, p, grid, st) : launch_fwd_one<T, 128, 1>(maps, p, grid, st);
   if (D == 64) return two ? launch_fwd_one<T, 64, 2>(maps, p, grid, st) : launch_fwd_one<T, 64, 1>(maps, p, grid, st);
   if (D == 256) return launch_fwd_one<T, 256, 1>(maps, p, grid, st);

@@ -91,6 +91,10 @@ int tc_launch_bwd(int dtype, int D, const CUtensorMap* maps, const tc::BwdTcPara
 template <class M>
 bool tc_bwd_short_loops(const Geo& g, int D);
 
+// Whether a 16-bit forward with D channels per tile takes the form with two streams of key tiles (fwd_two_streams, fwd_tc.cuh).
+template <class M>
+bool tc_fwd_two_streams(const Geo& g, int D);
+
 // 16-bit head dim 256 (bwd_wide.cuh, three launches); maps: Q, K, V, dO with 128-row boxes, the same four with 64-row
 // boxes, dQ, dK, dV.
 template <class M>

@@ -251,6 +251,14 @@ size_t chill_bwd_dq_accum_bytes(const chill_shape* s);
 int chill_fwd_uses_tensor_cores(const chill_fwd_args* a);
 int chill_bwd_uses_tensor_cores(const chill_bwd_args* a);
 
+/* Which kernel chill_fwd would launch for these arguments (host-only; pointers are looked at for their alignment), or a
+ * negative status if the arguments are invalid. */
+#define CHILL_FWD_CUDA_CORES 0   /* generic: simt.cuh, or split.cuh for large fp32 calls of head dim <= 64 */
+#define CHILL_FWD_ONE_STREAM 1   /* 16-bit: one chain of key tiles per tile of queries */
+#define CHILL_FWD_TWO_STREAMS 2  /* 16-bit: two chains, merged: few tiles of queries with many key tiles each */
+#define CHILL_FWD_TF32 3
+int chill_fwd_kernel(const chill_fwd_args* a);
+
 /* Which kernels chill_bwd would launch for these arguments (host-only; pointers are looked at for their alignment), or a
  * negative status if the arguments are invalid. */
 #define CHILL_BWD_CUDA_CORES 0   /* generic: simt.cuh, or split.cuh for large fp32 calls of head dim <= 64 */

@@ -41,6 +41,21 @@ def make_inputs(B, H, Hkv, L, D, dtype, seed=20):
     return q, k, v, do
 
 
+def fwd_kernel(lib, mask, B, H, Hkv, L, D, dtype, flags=0, pointer=4096):
+    """chill_fwd_kernel for contiguous tensors of this shape (host-only: the pointers are never followed)."""
+    import ctypes as C
+
+    from chill_attention import _cabi
+
+    q, k = (torch.empty(B, h, L, D, dtype=dtype, device="meta") for h in (H, Hkv))
+    a = _cabi.FwdArgs()
+    a.s = _cabi.make_shape(q, k, _cabi.BUILTIN_FUNCTOR_IDS[mask.cuda_functor], mask.constargs, None, D ** -0.5, flags=flags)
+    a.q = a.k = a.v = a.o = pointer
+    for t, name in ((q, "q"), (k, "k"), (k, "v"), (q, "o")):
+        setattr(a, name + "_strides", (C.c_int64 * 4)(*t.stride()))
+    return lib.chill_fwd_kernel(C.byref(a))
+
+
 def bwd_kernels(lib, mask, B, H, Hkv, L, D, dtype, flags=0, accum=True, functor=None, pointer=4096):
     """chill_bwd_kernels for contiguous tensors of this shape (host-only: the pointers are never followed)."""
     import ctypes as C

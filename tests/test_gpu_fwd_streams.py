@@ -1,9 +1,9 @@
 """Forward with two streams of key tiles per tile of queries (csrc/fwd_tc.cuh, chosen by fwd_two_streams: all CTAs resident at
-once, loops of 6 64-key steps at head dim 64 and 16 at 128), merged at the end; and key tiles that start between multiples of 64."""
+once, loops of 7 64-key steps at head dim 64 and 16 at 128), merged at the end; and key tiles that start between multiples of 64."""
 import pytest
 import torch
 
-from helpers import big_masks, check_forward, ensure_built, make_inputs, oracle_all
+from helpers import big_masks, check_forward, ensure_built, fwd_kernel, make_inputs, oracle_all
 
 pytestmark = pytest.mark.gpu
 
@@ -13,9 +13,19 @@ def _built():
     ensure_built()
 
 
-def check(mask, B, H, Hkv, L, D, dtype, lens=None):
+def most_steps(mask, L):
+    """Steps of 64 keys of the longest tile of 128 queries."""
+    lo, hi = (torch.as_tensor(x).expand(L) for x in type(mask).k_range_for_q(torch.arange(L), L, mask.constargs))
+    return max(int(hi[t:t + 128].max().clamp(max=L - 1) - lo[t:t + 128].min().clamp(min=0)) // 64 + 1 for t in range(0, L, 128))
+
+
+def check(mask, B, H, Hkv, L, D, dtype, lens=None, two=None):
     from chill_attention import _cabi, chill_attention
 
+    route = fwd_kernel(_cabi.load_library(), mask, B, H, Hkv, L, D, dtype, flags=_cabi.FLAG_NARROW_HEAD)
+    if two is None:  # tests of few tiles: the steps decide
+        two = D < 256 and most_steps(mask, L) >= (16 if D == 128 else 7)
+    assert route == (_cabi.FWD_TWO_STREAMS if two else _cabi.FWD_ONE_STREAM)
     q, k, v, do = make_inputs(B, H, Hkv, L, D, dtype, seed=L + D)
     o_ref, lse_ref, *_ = oracle_all(mask, q, k, v, do, lens)
     o, lse = chill_attention(q.cuda(), k.cuda(), v.cuda(), mask=mask, lens=None if lens is None else lens.cuda(), return_lse=True)
@@ -24,7 +34,7 @@ def check(mask, B, H, Hkv, L, D, dtype, lens=None):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=str)
-@pytest.mark.parametrize("D,L", [(32, 385), (64, 321), (64, 384), (64, 449), (64, 640), (128, 961), (128, 1024), (128, 1090)])
+@pytest.mark.parametrize("D,L", [(32, 385), (64, 321), (64, 384), (64, 385), (64, 448), (64, 449), (64, 640), (128, 961), (128, 1024), (128, 1090)])
 @pytest.mark.parametrize("mask_no", range(7))
 def test_two_streams(mask_no, D, L, dtype):
     """Even and odd numbers of steps; lens that leaves a tile of queries one step, or none, or a last step of one key."""
@@ -53,3 +63,12 @@ def test_key_tiles_start_anywhere(left, right, D):
 
     check(ca.SlidingWindowChillMask(left, right), 2, 4, 2, 333, D, torch.float16, torch.tensor([333, 200], dtype=torch.int32))
     check(ca.ChunkwiseChillMask(left + 7, 1), 1, 2, 2, 301, D, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16], ids=str)
+def test_more_tiles_than_fit_at_once(dtype):
+    """Causal, head dim 64, 320 tiles of queries: a few long loops outlast the rest; the full mask takes one stream there."""
+    import chill_attention as ca
+
+    check(ca.CausalChillMask(), 2, 10, 5, 2048, 64, dtype, two=True)
+    check(ca.FullChillMask(), 2, 10, 5, 2048, 64, dtype, torch.tensor([2048, 700], dtype=torch.int32), two=False)
