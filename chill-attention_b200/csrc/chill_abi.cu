@@ -248,17 +248,31 @@ static uint32_t vec_bit(uint32_t bit, const void* p, const int64_t* st, int dtyp
 
 // Whether an fp32 call of IEEE accuracy goes to the tensor cores with split operands (split.cuh): head dim <= 64, and enough
 // work, as steps of 128 queries x 64 keys times the channels the CUDA-core kernels would multiply, to make up for the longer
-// set-up; a single step per tile never does.  Forward, us, CUDA cores / split, full mask, head dim 64: (1,2,128) 8.6 / 14.3,
-// (1,8,256), 64 steps: 14.1 / 17.8, (8,8,128), 128 steps: 17.4 / 14.6, (1,1,2048), 512 steps: 90 / 72, (2,8,1000): 143 / 44,
-// (4,8,2048): 938 / 274; (8,16,64), one step each: 11.4 / 12.5; head dim 32 (2,4,1000): 62 / 41, with window(32, 0), 192 steps:
-// 13.5 / 16.3.  Backward: (1,4,257), 60 steps: 27 / 33, (1,8,256): 29.9 / 29.0, window(32, 0) (2,4,512), 96 steps: 30 / 26,
-// (2,8,1000): 442 / 135.
-static bool split_pays(const chill_shape& s, long long least) {
+// set-up; a single step per tile never does.  us, CUDA cores / split, head dim 64 unless stated.
+// Forward: full mask (1,2,128) 8.6 / 14.3, (1,8,256), 64 steps: 14.1 / 17.8, (8,8,128), 128 steps: 17.4 / 14.6, (1,1,2048), 512
+//   steps: 90 / 72, (2,8,1000): 143 / 44, (4,8,2048): 938 / 274; (8,16,64), one step each: 11.4 / 12.5.
+// Backward: (1,4,257), 60 steps: 27 / 33, (1,8,256): 29.9 / 29.0, window(32, 0) (2,4,512), 96 steps: 30 / 26, (2,8,1000): 442 / 130.
+// Narrow masks: tiles of 128 rows then take more steps per row than the CUDA cores' tiles of 64.  window(32, 0), forward: (1,8,1024),
+//   184 steps: 17.7 / 18.7, (1,8,2048): 24.6 / 19.5; head dim 32, where the steps weigh less: backward
+//   (2,8,4096) 145 / 152, but with eight heads per key head (1,8/1,4096) 121 / 111 (the forward, 57.0 / 58.7 at (1,32,2048), stays).
+// Few tiles: the CUDA cores then take tiles of 16 rows (simt_inst.cu), so that the longest chain of steps decides.  Backward (its dK / dV
+//   tiles walk all heads of the group): window(32, 0) (1,16/2,256) 78 / 115, chunkwise(64, 2) (1,8/1,512) 114 / 145, full
+//   (1,8/1,512), as many steps for 16 rows as for 128: 297 / 253; head dim 32: full (1,8/1,512) 190 / 221.  Forward, head dim 32, full:
+//   (1,2,1024) 32 / 38, (1,1,2048) 61 / 66, (1,2,2048), 256 tiles of 16 rows: 81 / 66, (1,8,512) with 8 steps 22.8 / 24.0.
+static bool split_pays(const chill_shape& s, bool backward) {
   if (s.dtype != CHILL_F32 || s.D > 64 || s.D % 16 != 0 || (s.flags & CHILL_FLAG_FORCE_GENERIC)) return false;
-  long long total = 0;
-  int most = 0;
-  CHILL_MASK_SWITCH_OR(s.mask.id, count_steps<MaskT>(to_geo(s), total, most), return false)
-  return most >= 2 && total * (s.D <= 32 ? 32 : 64) >= least;
+  const Geo g = to_geo(s);
+  long long total = 0, total64 = 0, unused = 0;
+  int most = 0, most64 = 0, most16 = 0;
+  CHILL_MASK_SWITCH_OR(s.mask.id, (count_steps<MaskT>(g, total, most), count_steps<MaskT, 64>(g, total64, most64), count_steps<MaskT, 16>(g, unused, most16)),
+                       return false)
+  const bool narrow = 10 * total > 7 * total64;
+  if (most < 2 || total * (s.D <= 32 ? 32 : 64) < (backward ? 5120 : (narrow ? 16384 : 8192))) return false;
+  if (backward && narrow && s.D == 32 && s.H == s.H_kv) return false;
+  long long tiles = (long long)((s.Lq + 63) / 64) * s.H * s.B;
+  if (backward) tiles += (long long)((s.Lk + 63) / 64) * s.H_kv * s.B;
+  if (2 * tiles >= sm_count()) return true;
+  return backward ? s.D > 32 && most <= most16 : s.D > 32 || (4 * tiles > sm_count() && most >= 16);
 }
 
 static int fwd_generic(const chill_fwd_args& a, cudaStream_t st) {
@@ -275,7 +289,7 @@ static int fwd_generic(const chill_fwd_args& a, cudaStream_t st) {
            vec_bit(simt::kVecV, a.v, a.v_strides, dt, D) | vec_bit(simt::kVecO, a.o, a.o_strides, dt, D);
   int e = 0;
   int* status = nullptr;
-  if (pp.vec == (simt::kVecQ | simt::kVecK | simt::kVecV | simt::kVecO) && split_pays(a.s, 8192) && (status = split_status_ptr()) != nullptr) {
+  if (pp.vec == (simt::kVecQ | simt::kVecK | simt::kVecV | simt::kVecO) && split_pays(a.s, false) && (status = split_status_ptr()) != nullptr) {
     split::FwdParams sp;
     sp.f = p;
     sp.status = status;
@@ -465,7 +479,7 @@ static int bwd_generic(const chill_bwd_args& a, cudaStream_t st) {
            vec_bit(simt::kVecDv, a.dv, a.dv_strides, dt, D);
   int e = 0;
   int* status = nullptr;
-  if (pp.vec == (255u & ~(uint32_t)simt::kVecO) && a.dk_part == nullptr && split_pays(a.s, 5120) && (status = split_status_ptr()) != nullptr) {
+  if (pp.vec == (255u & ~(uint32_t)simt::kVecO) && a.dk_part == nullptr && split_pays(a.s, true) && (status = split_status_ptr()) != nullptr) {
     split::BwdParams sp;
     sp.b = pp.b;
     sp.status = status;

@@ -87,11 +87,11 @@ __device__ __forceinline__ int valid_len(const Geo& g, int b) {
   return n;
 }
 
-// Steps of 128 queries x 64 keys of a call, over all heads: `total`, and the most a tile of queries has (for the rules that choose
+// Steps of ROWS queries x 64 keys of a call, over all heads: `total`, and the most a tile of queries has (for the rules that choose
 // between kernels).  At most 32 tiles are looked at (four where a tile's range takes a loop over its rows); lens is not known here.
-template <class M>
+template <class M, int ROWS = 128>
 void count_steps(const Geo& g, long long& total, int& most) {
-  constexpr int kRows = 128, kCols = 64, kLooks = M::kKLimsContinuous ? 32 : 4;
+  constexpr int kRows = ROWS, kCols = 64, kLooks = M::kKLimsContinuous ? 32 : 4;
   const int n_rt = (g.Lq + kRows - 1) / kRows, every = (n_rt + kLooks - 1) / kLooks;
   long long sum = 0, looks = 0;
   most = 0;

@@ -118,21 +118,21 @@ def test_nothing_but_the_rows_is_written(D, layout, mask_no):
     rows) keep their value.  Rows 4 channels apart, heads in between ([batch, position, head, channel]), packed."""
     from chill_attention import _cabi
 
-    mask, B, H, L, guard, fill = all_masks()[mask_no], 3, 24, 193, 256, 7.0
+    mask, B, H, L, guard, fill = all_masks()[mask_no], 6, 24, 193, 256, 7.0
     row = D + 4 if layout == "wide_rows" else D
-    strides = (L * H * row, row, H * row, 1) if layout == "blhd" else (H * L * row, L * row, row, 1)
 
-    def buffer():
-        return torch.full((B * H * L * row + 2 * guard,), fill, device="cuda")
+    def buffer(heads):
+        return torch.full((B * heads * L * row + 2 * guard,), fill, device="cuda"), heads
 
-    def view(buf):
-        return buf.as_strided((B, H, L, D), strides, guard)
+    def view(buf, heads):
+        strides = (L * heads * row, row, heads * row, 1) if layout == "blhd" else (heads * L * row, L * row, row, 1)
+        return buf.as_strided((B, heads, L, D), strides, guard)
 
-    q, k, v, do = make_inputs(B, H, H, L, D, torch.float32, seed=D)
+    q, k, v, do = make_inputs(B, H, H // 2, L, D, torch.float32, seed=D)
     o_ref, lse_ref, *g_ref = oracle_all(mask, q, k, v, do)
     q, k, v, do = (t.cuda() for t in (q, k, v, do))
-    buffers = [buffer() for _ in range(4)]
-    o, dq, dk, dv = (view(b) for b in buffers)
+    buffers = [buffer(heads) for heads in (H, H, H // 2, H // 2)]
+    o, dq, dk, dv = (view(*b) for b in buffers)
     lse, delta = (torch.empty(B, H, L, device="cuda") for _ in range(2))
     lib = _cabi.load_library()
     shape = _cabi.make_shape(q, k, _cabi.BUILTIN_FUNCTOR_IDS[mask.cuda_functor], mask.constargs, None, D ** -0.5)
@@ -142,8 +142,8 @@ def test_nothing_but_the_rows_is_written(D, layout, mask_no):
     assert lib.chill_launch_count() - before == 5  # the split kernels ran, forward and backward
     check_forward(o, lse, o_ref, lse_ref, None, torch.float32)
     check_grads((dq, dk, dv), g_ref, torch.float32)
-    for buf in buffers:
-        view(buf).fill_(fill)
+    for buf, heads in buffers:
+        view(buf, heads).fill_(fill)
         assert (buf == fill).all()
 
 
@@ -246,3 +246,29 @@ def test_mixed_scales_within_a_row():
         err = lambda x: (x.cpu().double() - exact[i]).norm(dim=2) / exact[i].norm(dim=2)  # noqa: E731, B023
         assert (err(mine[i]) <= 1.2 * err(fma[i]).clamp(min=2e-7)).all()
 
+
+
+@pytest.mark.parametrize("D,B,H,Hkv,L,window,split", [
+    (64, 1, 16, 2, 256, 32, (False, False)),   # 4 key tiles of 24 steps each; the CUDA cores' 16-row tiles have 16
+    (64, 1, 8, 1, 512, None, (True, True)),    # few tiles, but as many steps for 16 rows as for 128
+    (32, 1, 8, 1, 512, None, (False, False)),
+    (32, 1, 2, 1, 2048, None, (True, True)),   # forward: 256 tiles of 16 rows, 32 steps; backward: 96 tiles of 64 rows
+    (32, 1, 1, 1, 2048, None, (False, False)),
+    (64, 1, 8, 8, 1024, 32, (False, True)),    # narrow: 184 steps, 256 needed
+    (64, 1, 8, 8, 2048, 32, (True, True)),
+    (32, 2, 8, 8, 2048, 32, (True, False)),
+    (32, 1, 8, 1, 4096, 32, (True, True)),
+    (16, 2, 8, 8, 2048, 32, (True, True)),
+    (64, 1, 8, 8, 256, None, (False, False)),  # 64 steps
+])
+def test_route(D, B, H, Hkv, L, window, split):
+    """Both sides of each line of the dispatch rule, with results within each other's error."""
+    import chill_attention as ca
+
+    mask = ca.FullChillMask() if window is None else ca.SlidingWindowChillMask(window, 0)
+    inputs = make_inputs(B, H, Hkv, L, D, torch.float32, seed=L)
+    mine, routes = run(*inputs, mask)
+    ref, _ = run(*inputs, mask, split=False)
+    assert routes == split
+    for a, b in zip(mine, ref):
+        assert (a - b).norm() <= 3e-6 * b.norm()
