@@ -21,9 +21,9 @@
 //
 // Measured (causal bf16 (2,16,4096,256), dV / dK / dQ in us): 338 / 522 / 558 with one stage, one buffer of scores and four
 // elementwise warps (each step a chain of load, scores, elementwise, accumulate), 250 / 403 / 436 with two, 253 / 378 / 432 with
-// eight warps as well, which masked tiles need (chunkwise(100, 3) (2,8/4,2048): all three 580 -> 521 -> 323).  What bounds them now:
-// the streamed tiles leave the L2 at 5.6 (dK) to 8.5 TB/s (dV), and a score MMA with N = 64 reads 6 KB of shared memory in its 48
-// clocks.
+// eight warps as well, which masked tiles need (chunkwise(100, 3) (2,8/4,2048): all three 580 -> 521 -> 323).  What bounds them now is
+// the chain again: tensor pipe 42 to 46 %, shared-memory data pipe 45 to 54 % (a score MMA with N = 64 reads 6 KB in its 48 clocks),
+// L2 15 to 31 %, DRAM 8 to 10 % (counters: profiles/c2d256s_causal_bf16_bwd_wide_ncu.md).
 // Reference math: chill_attention/chill_bwd_dkdv.py:347-508, chill_bwd_dq.py:300-394.
 #pragma once
 #include "bwd_tc.cuh"
@@ -33,6 +33,8 @@ namespace tc {
 
 enum : int { kWideDV = 0, kWideDK = 1, kWideDQ = 2 };
 constexpr int kWideThreads = 384;  // warps 0-7 elementwise + epilogue, 8 TMA producer, 9 MMA issuer, 10-11 idle
+
+constexpr int kWideAlign = 128;  // of the dynamic shared memory, as declared
 
 template <int D, int MODE>
 struct WideSmem {
@@ -47,7 +49,10 @@ struct WideSmem {
   static constexpr int kBars = kVec + 8 * 2 * 32 * 4;
   static constexpr int kNumBars = 14;
   static constexpr int kMisc = kBars + 8 * kNumBars;
-  static constexpr int kDynamic = kMisc + 16;  // the array is declared with its alignment: there is no room to align it by hand
+  static constexpr int kTotal = kMisc + 16;
+  // What aligning the declared base to 1 KB by hand can take.  (Declared with 1 KB the kernels need none of it, but all three together
+  // take 10 % longer on causal (2,16,4096,256): 1087 -> 1200 us with delta.)
+  static constexpr int kDynamic = kTotal + 1024 - kWideAlign;
 };
 
 enum : int { kStWideProducer = 501, kStWideMma = 502, kStWideCompute = 503, kStWideEpilogue = 504 };
@@ -109,9 +114,9 @@ bwd_wide_kernel(const __grid_constant__ CUtensorMap tmR1, const __grid_constant_
     return;
   }
 
-  extern __shared__ __align__(1024) uint8_t smem_wide[];  // the 128-byte swizzle repeats every 1 KB
-  uint8_t* gen_base = smem_wide;
-  const uint32_t base = smem_u32(smem_wide);
+  extern __shared__ __align__(kWideAlign) uint8_t smem_wide[];
+  const uint32_t base = (smem_u32(smem_wide) + 1023u) & ~1023u;
+  uint8_t* gen_base = smem_wide + (base - smem_u32(smem_wide));
   const uint32_t sR1 = base + L::kR1, sR2 = base + L::kR2, sE = base + L::kE, sL = base + L::kL;
   const uint32_t bars = base + L::kBars;
   // "Early" tile: Q for dV, dO / V for dK / dQ, read by one score GEMM (e_done: that GEMM has finished).  "Late" tile: also, or
