@@ -22,8 +22,8 @@
 // Measured (causal bf16 (2,16,4096,256), dV / dK / dQ in us): 338 / 522 / 558 with one stage, one buffer of scores and four
 // elementwise warps (each step a chain of load, scores, elementwise, accumulate), 250 / 403 / 436 with two, 253 / 378 / 432 with
 // eight warps as well, which masked tiles need (chunkwise(100, 3) (2,8/4,2048): all three 580 -> 521 -> 323).  What bounds them now is
-// the chain again: tensor pipe 42 to 46 %, shared-memory data pipe 45 to 54 % (a score MMA with N = 64 reads 6 KB in its 48 clocks),
-// L2 15 to 31 %, DRAM 8 to 10 % (counters: profiles/c2d256s_causal_bf16_bwd_wide_ncu.md).
+// the chain again: tensor pipe 46 to 52 %, shared-memory data pipe 52 to 61 % (a score MMA with N = 64 reads 6 KB in its 48 clocks),
+// L2 17 to 34 %, DRAM 9 to 11 % (counters: profiles/c2d256s_causal_bf16_bwd_wide_ncu.md).
 // Reference math: chill_attention/chill_bwd_dkdv.py:347-508, chill_bwd_dq.py:300-394.
 #pragma once
 #include "bwd_tc.cuh"

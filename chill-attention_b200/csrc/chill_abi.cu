@@ -209,7 +209,7 @@ static bool shape_tf32_ok(const chill_shape& s) {
   return s.dtype == CHILL_F32 && (s.flags & CHILL_FLAG_ALLOW_TF32) && (s.D == 64 || s.D == 128) && s.sm_scale > 0.f;
 }
 
-// the forward also has a tensor-core kernel for 16-bit head dim 256 (one CTA per SM); the backward does not
+// 16-bit head dim 256: a forward with one CTA per SM and a backward of its own (bwd_wide.cuh)
 static bool shape_tc_fwd_only_ok(const chill_shape& s) {
   if (s.flags & CHILL_FLAG_FORCE_GENERIC) return false;
   return (s.dtype == CHILL_F16 || s.dtype == CHILL_BF16) && s.D == 256 && s.sm_scale > 0.f;

@@ -10,6 +10,9 @@
 //   * adding the large products (hh) into columns of their own, or last, after the small ones, so that only the contraction
 //     of one tile (64 channels or 64 positions: four MMA steps) is ever truncated at full magnitude, and
 //   * starting every tile's product from zero and adding the tiles up in registers, rounded.
+// What is left is one-sided all the same: O of V with a common component is low by up to 2.5e-7, and delta with it, which shows where
+// dP - delta cancels (V and dO from N(3, 1): dK off by 1.3e-5 at 129 keys, simt.cuh 1.1e-6; at 2048 keys 9e-6 and 3.5e-5).  Large and
+// small products of the scores in groups of their own change nothing there.
 //
 // What the parts cannot hold: NaN, Inf and |x| > 3.39e38 would make 0 * NaN of what the mask hides, and numbers below 2^-110 are no
 // sum of three bf16 numbers any more.  The first enter the parts of a streamed tile as zeros; the tile says which of its positions
@@ -21,9 +24,11 @@
 //
 // Measured against simt.cuh (full mask, head dim 64, us): (2,8,1000) forward 143 -> 44, backward 442 -> 130; (4,8,2048) forward
 // 938 -> 274, backward 2975 -> 825.  Distance from the 64-bit result (N(0, 1) inputs, 2-norm): O 5.9e-7 -> 2.0e-7, dQ, dK and dV
-// 0.3 to 0.95 of what it was at lengths from 129 to 2048, all masks.  What bounds them is the tensor pipe: 12 to 14 MMAs per score
-// product, 24 with N = 64 per accumulating one, which take 45 clocks each alone and 60 to 90 beside the elementwise warps' TMEM
-// and the loaders' shared-memory traffic.  MMA loops are rolled where their operands only differ by an addition.
+// 0.3 to 0.95 of what it was at lengths from 129 to 2048, all masks.  What bounds them is the chain of a step, not a resource: the
+// tensor pipe is busy for 35 to 38 % of the time (16 MMAs per score product, 6 up to 32 channels, and 24 with N = 64 per accumulating
+// one), shared memory for 30 %, the L2 for 10 % (profiles/split_fp32_kernels_ncu.md).  In the forward the loaders' part of it, loads,
+// split and stores of one tile after the other, is as long as what the streams do.  MMA loops are rolled where their operands only
+// differ by an addition.
 #pragma once
 #include <type_traits>
 

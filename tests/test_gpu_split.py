@@ -272,3 +272,18 @@ def test_route(D, B, H, Hkv, L, window, split):
     assert routes == split
     for a, b in zip(mine, ref):
         assert (a - b).norm() <= 3e-6 * b.norm()
+
+
+@pytest.mark.parametrize("mask_no", [0, 1, 4])
+@pytest.mark.parametrize("L", [129, 1000])
+def test_inputs_of_one_sign(L, mask_no):
+    """What the tensor core's truncation takes is one-sided, so it does not average out here.  Measured, distance from the 64-bit result
+    over the CUDA cores': O 0.65, dQ 1.0, dK 1.3 (2.8e-7 and 2.2e-7), dV 0.6; bound: 1.5."""
+    mask = big_masks()[mask_no]
+    inputs = [t.abs() for t in make_inputs(4, 16, 16, L, 64, torch.float32, seed=L)]
+    exact = oracle_all(mask, *inputs)
+    mine, routes = run(*inputs, mask)
+    fma, _ = run(*inputs, mask, split=False)
+    assert routes == (True, True)
+    for i in (0, 2, 3, 4):
+        assert (mine[i].cpu().double() - exact[i]).norm() <= 1.5 * (fma[i].cpu().double() - exact[i]).norm(), "o lse dq dk dv".split()[i]
