@@ -308,11 +308,11 @@ bwd_fused_tc_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const uint32_t stage_sh = base + L::kDrain + rg * (L::kDrainBufs * L::kDrainChunkBytes);
     int chunk_no = 0;
     bool ok = true;
+    float* first_rows = p.dq_accum + (size_t)(rg * 32 + q_row0) * D;  // from row 2^24 on the offset does not fit an int
     for (int it = 0; it < n_it; ++it) {
       const int h = hk * G + it / n_qt;
       const int qi = it % n_qt;
-      const int row = q_row0 + qi * kTile + rg * 32;  // from row 2^24 on its element offset does not fit an int
-      float* dst = p.dq_accum + ((size_t)b * g.H + h) * n_qt_total * (size_t)(kTile * D) + (size_t)row * D;
+      float* dst = first_rows + (((size_t)b * g.H + h) * n_qt_total + qi) * (size_t)(kTile * D);
       ok = mbar_wait(bar_dq_full, (uint32_t)it & 1u, guard, kStFusDrain);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
